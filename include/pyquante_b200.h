@@ -290,8 +290,8 @@ int pqb_oneint_noalloc(int n, const double *origin, const int *powers, const int
  * + dE_nuc, D = C_occ C_occ^T, W = C_occ diag(e_occ) C_occ^T.
  * pqb_set_shell_atoms: atom index of every uploaded shell (host array).
  * pqb_grad_2e: adds tr(D dG[D]) to grad[3*natoms] (device), derivative
- * integrals contracted with the density on the fly over the current plan;
- * mode PQB_MIXED runs the FP32-eligible list in FP32.
+ * integrals contracted with the density on the fly over the current plan
+ * (in FP64 in both modes).
  * pqb_grad_1e: adds 2 tr(D d(T+V)) - 2 tr(W dS) over a function table
  * (func_atom: device array, atom index per function; atoms on the host). */
 int pqb_set_shell_atoms(pqb_ctx *ctx, const int *shell_atom);

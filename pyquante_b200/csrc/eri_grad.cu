@@ -9,146 +9,348 @@
 // reference forms it as trace2(D, der2JmK(...)) over stored derivative
 // integrals (PyQuante/force.py:106-116,232-252,318-357).
 //
-// Derivative integrals come from the same Rys 2-D integrals with one more
-// unit of momentum on the bra and ket centres A, B, C:
+// Derivative integrals come from the Rys 2-D integrals with one more unit of
+// momentum on centres A and C,
 //   d/dA_x phi_a = 2 alpha_a phi_{a+1x} - a_x phi_{a-1x}
 // (the raising/lowering relation of PyQuante/AnalyticDerivatives.py, applied
-// to each primitive), and the fourth centre by translational invariance,
-// dD = -(dA + dB + dC).  One thread per work item (quartet, primitive
-// chunk); the component loops stay rolled (the derivative kernel favours
-// compact code over peak speed); nine gradient components accumulate in
-// registers and go to the four atoms with twelve atomics.
+// to each primitive), the raised B from the horizontal relation
+// (a,b+1) = (a+1,b) + AB (a,b), and the fourth centre by translational
+// invariance, dD = -(dA + dB + dC).
+//
+// The components are those of the shells' common contraction: D is the
+// pre-scaled density D'_kl = r_k r_l D_kl of the Fock-build kernels, so Gamma
+// carries the four component scales.  The gradient is summed per shell
+// (3 nshell accumulators spread the atomics that 3 natoms would serialise)
+// and gathered to the atoms at the end.
+//
+// Two splits (eri_grad_launch picks by the number of components):
+//  * up to 27 components: one thread per work item, everything in registers;
+//  * more: one warp per work item.  Lanes first share the (primitive quartet,
+//    root, axis) 2-D tables, which go to shared memory, then the (component,
+//    root) products.
+// A whole (H2O)4 / 6-31G* gradient takes 0.73 ms (60.6 ms with one thread per
+// item for every class, its tables and Gamma in local memory, and the classes
+// one after the other): 0.46 ms on the GPU, in which the items' serial chains
+// and the few high classes leave most of the chip idle.
 #include "eri_engine.cuh"
 #include "eri_launch.h"
 
 namespace pqb {
 
-template <int LA, int LB, int LC, int LD, typename R>
-__global__ void __launch_bounds__(128) eri_grad_kernel(const int4 *__restrict__ list, int nq,
-                                                       const PairInfo *__restrict__ pairs,
-                                                       const PrimPair *__restrict__ prims,
-                                                       const double *__restrict__ D, const double *__restrict__ fscale,
-                                                       const int *__restrict__ shell_atom, int n, double *grad)
+// Gamma of component (ia ib|ic id) without the weight, D' read at the
+// quartet's functions.
+__device__ __forceinline__ double gamma_of(const double *Db, int64_t nm, int i, int j, int k, int l)
+{
+    const double dij = __ldg(Db + i * nm + j), dkl = __ldg(Db + k * nm + l);
+    const double dik = __ldg(Db + i * nm + k), djl = __ldg(Db + j * nm + l);
+    const double dil = __ldg(Db + i * nm + l), djk = __ldg(Db + j * nm + k);
+    return 16.0 * dij * dkl - 4.0 * (dik * djl + dil * djk);
+}
+
+// ---------------------------------------------------------- thread mode --
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128) eri_grad_thread_kernel(const int4 *__restrict__ list, int nq,
+                                                              const PairInfo *__restrict__ pairs,
+                                                              const PrimPair *__restrict__ prims,
+                                                              const double *__restrict__ D, double *gshell)
 {
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    constexpr int NAB = NA * NB, NCD = NC * ND;
     constexpr int NR = (LA + LB + LC + LD + 1) / 2 + 1;
-    constexpr int EA = LA + 1, EB = LB + 1, EC = LC + 1, ED = LD;
-    constexpr int G2 = (EA + 1) * (EB + 1) * (EC + 1) * (ED + 1);
-    // component exponents packed per shell component: x | y << 4 | z << 8
-    auto pk3 = [](int L, int i) { return cart_lx(L, i) | (cart_ly(L, i) << 4) | (cart_lz(L, i) << 8); };
-    for (int qi = blockIdx.x * blockDim.x + threadIdx.x; qi < nq; qi += gridDim.x * blockDim.x) {
-        const int4 e = list[qi];
+    constexpr int sD = 1, sC = (LD + 1) * sD, sB = (LC + 2) * sC, sA = (LB + 1) * sB, G2 = (LA + 2) * sA;
+    const int lane = threadIdx.x & 31;
+    // whole warps step through the list; a lane past the end repeats the last
+    // item with no primitive quartets
+    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < nq; base += gridDim.x * blockDim.x) {
+        const int qi = base + lane;
+        const bool live = qi < nq;
+        const int4 e = list[live ? qi : nq - 1];
         const PairInfo &pb = pairs[e.x];
         const PairInfo &pk = pairs[e.y];
         const QCtx q = make_qctx(pb, pk, e.x, e.y);
-        // Gamma for every component of the quartet (0 for non-canonical ones)
-        double gam[NAB * NCD];
+        const bool bd = q.sa == q.sb, kd = q.sc == q.sd, qd = q.bra == q.ket, af = q.fa > q.fb;
+        const double *Db = D + q.bo;
+        double gam[NA * NB * NC * ND];
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int d = 0; d < ND; ++d)
+                        gam[((a * NB + b) * NC + c) * ND + d] =
+                            comp_weight(a, b, c, d, bd, kd, qd, af) *
+                            gamma_of(Db, q.nm, q.fa + a, q.fb + b, q.fc + c, q.fd + d);
+        double g9[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) g9[k] = 0.0;
+        const double AB[3] = {pb.AB[0], pb.AB[1], pb.AB[2]}, CD[3] = {pk.AB[0], pk.AB[1], pk.AB[2]};
+        const double A[3] = {pb.A[0], pb.A[1], pb.A[2]}, C[3] = {pk.A[0], pk.A[1], pk.A[2]};
+        // bra primitives fastest: the lanes of a warp mostly share the bra pair
+        const int npb = pb.nprim;
+        int ik = e.z / npb, ib = e.z - (e.z / npb) * npb;
+        const int count = live ? e.w : 0;
 #pragma unroll 1
-        for (int ab = 0; ab < NAB; ++ab) {
-            const int fi = q.fa + ab / NB, fj = q.fb + ab % NB;
-            const int64_t IJ = fpair(fi, fj);
-#pragma unroll 1
-            for (int cd = 0; cd < NCD; ++cd) {
-                const int fk = q.fc + cd / ND, fl = q.fd + cd % ND;
-                const int64_t KL = fpair(fk, fl);
-                double g = 0.0;
-                if (!((q.sa == q.sb && fi < fj) || (q.sc == q.sd && fk < fl) || (q.bra == q.ket && IJ < KL))) {
-                    const double s = 8.0 * (fi == fj ? 0.5 : 1.0) * (fk == fl ? 0.5 : 1.0) * (IJ == KL ? 0.5 : 1.0) *
-                                     fscale[fi] * fscale[fj] * fscale[fk] * fscale[fl];
-                    const double *Db = D + q.bo;
-                    const int nm = q.nm;
-                    const double dij = __ldg(Db + (int64_t)fi * nm + fj), dkl = __ldg(Db + (int64_t)fk * nm + fl);
-                    const double dik = __ldg(Db + (int64_t)fi * nm + fk), djl = __ldg(Db + (int64_t)fj * nm + fl);
-                    const double dil = __ldg(Db + (int64_t)fi * nm + fl), djk = __ldg(Db + (int64_t)fj * nm + fk);
-                    g = s * (2.0 * dij * dkl - 0.5 * (dik * djl + dil * djk));
-                }
-                gam[ab * NCD + cd] = g;
+        for (int t = 0; t < count; ++t) {
+            const PrimPair *pp = prims + pb.prim_off + ib, *pq = prims + pk.prim_off + ik;
+            const PrimJK P = load_prim_jk(pp), Q = load_prim_jk(pq);
+            const double a2 = 2.0 * __ldg(&pp->alpha_a), b2 = 2.0 * P.zeta - a2, c2 = 2.0 * __ldg(&pq->alpha_a);
+            if (++ib == npb) {
+                ib = 0;
+                ++ik;
             }
-        }
-        double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
-        const int npk = pk.nprim;
-        int ib = e.z / npk, ik = e.z - (e.z / npk) * npk;
-#pragma unroll 1
-        for (int t = 0; t < e.w; ++t) {
-            const PrimPair P = prims[pb.prim_off + ib];
-            const PrimPair Q = prims[pk.prim_off + ik];
-            if (++ik == npk) {
-                ik = 0;
-                ++ib;
-            }
-            const R aa2 = (R)(2.0 * P.alpha_a), ab2 = (R)(2.0 * (P.zeta - P.alpha_a)), ac2 = (R)(2.0 * Q.alpha_a);
-            const double zpe = P.zeta + Q.zeta;
             const double PQ[3] = {P.P[0] - Q.P[0], P.P[1] - Q.P[1], P.P[2] - Q.P[2]};
-            const double T = P.zeta * Q.zeta / zpe * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-            const double pre = P.K * Q.K * rsqrt(zpe);
+            const double rs = rsqrt_nr(P.zeta + Q.zeta), izpe = rs * rs;
+            const double T = P.zeta * Q.zeta * izpe * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+            const double pre = P.K * Q.K * rs;
             double uu[NR], ww[NR];
-            rys_roots<NR>(T, uu, ww);
-#pragma unroll 1
+            rys_roots_fast<NR>(T, uu, ww);
+#pragma unroll
             for (int r = 0; r < NR; ++r) {
-                R g[3][G2];
+                const RysCoef k = rys_coef(uu[r], P.zeta, Q.zeta, P.izeta, Q.izeta, izpe);
+                double g[3][G2];
 #pragma unroll
                 for (int x = 0; x < 3; ++x)
-                    rys2d<EA, EB, EC, ED, R>(uu[r], P.zeta, Q.zeta, P.P[x] - pb.A[x], Q.P[x] - pk.A[x], PQ[x], pb.AB[x],
-                                             pk.AB[x], x == 0 ? ww[r] * pre : 1.0, g[x]);
-#pragma unroll 1
-                for (int ab = 0; ab < NAB; ++ab) {
-                    const int pa = pk3(LA, ab / NB), pbb = pk3(LB, ab % NB);
-#pragma unroll 1
-                    for (int cd = 0; cd < NCD; ++cd) {
-                        const double gm = gam[ab * NCD + cd];
-                        if (gm == 0.0) continue;
-                        const int pc = pk3(LC, cd / ND), pd = pk3(LD, cd % ND);
-                        R I[3], dA[3], dB[3], dC[3];
+                    rys2d_c<LA + 1, LB, LC + 1, LD, double>(k, P.P[x] - A[x], Q.P[x] - C[x], PQ[x], AB[x], CD[x],
+                                                            x == 0 ? ww[r] * pre : 1.0, g[x]);
+#pragma unroll
+                for (int ab = 0; ab < NA * NB; ++ab)
+#pragma unroll
+                    for (int cd = 0; cd < NC * ND; ++cd) {
+                        const int ia = ab / NB, ib3 = ab % NB, ic = cd / ND, id = cd % ND;
+                        double I[3], dA[3], dB[3], dC[3];
 #pragma unroll
                         for (int x = 0; x < 3; ++x) {
-                            const int a = (pa >> (4 * x)) & 15, b = (pbb >> (4 * x)) & 15, c = (pc >> (4 * x)) & 15,
-                                      d = (pd >> (4 * x)) & 15;
-                            const R *gx = g[x];
-                            const int i0 = ((a * (EB + 1) + b) * (EC + 1) + c) * (ED + 1) + d;
-                            constexpr int sA = (EB + 1) * (EC + 1) * (ED + 1), sB = (EC + 1) * (ED + 1), sC = ED + 1;
-                            I[x] = gx[i0];
-                            dA[x] = aa2 * gx[i0 + sA] - (a > 0 ? (R)a * gx[i0 - sA] : (R)0);
-                            dB[x] = ab2 * gx[i0 + sB] - (b > 0 ? (R)b * gx[i0 - sB] : (R)0);
-                            dC[x] = ac2 * gx[i0 + sC] - (c > 0 ? (R)c * gx[i0 - sC] : (R)0);
+                            const int a = cart_l(LA, ia, x), b = cart_l(LB, ib3, x), c = cart_l(LC, ic, x),
+                                      d = cart_l(LD, id, x);
+                            const int o = a * sA + b * sB + c * sC + d * sD;
+                            const double up = g[x][o + sA];
+                            I[x] = g[x][o];
+                            dA[x] = a2 * up - (a > 0 ? a * g[x][o - (a > 0 ? sA : 0)] : 0.0);
+                            dB[x] = b2 * fma(AB[x], I[x], up) - (b > 0 ? b * g[x][o - (b > 0 ? sB : 0)] : 0.0);
+                            dC[x] = c2 * g[x][o + sC] - (c > 0 ? c * g[x][o - (c > 0 ? sC : 0)] : 0.0);
                         }
-                        gA[0] += gm * (double)(dA[0] * I[1] * I[2]);
-                        gA[1] += gm * (double)(I[0] * dA[1] * I[2]);
-                        gA[2] += gm * (double)(I[0] * I[1] * dA[2]);
-                        gB[0] += gm * (double)(dB[0] * I[1] * I[2]);
-                        gB[1] += gm * (double)(I[0] * dB[1] * I[2]);
-                        gB[2] += gm * (double)(I[0] * I[1] * dB[2]);
-                        gC[0] += gm * (double)(dC[0] * I[1] * I[2]);
-                        gC[1] += gm * (double)(I[0] * dC[1] * I[2]);
-                        gC[2] += gm * (double)(I[0] * I[1] * dC[2]);
+                        const double gm = gam[ab * NC * ND + cd];
+                        const double w0 = gm * I[1] * I[2], gx = gm * I[0], w1 = gx * I[2], w2 = gx * I[1];
+                        g9[0] = fma(w0, dA[0], g9[0]);
+                        g9[1] = fma(w1, dA[1], g9[1]);
+                        g9[2] = fma(w2, dA[2], g9[2]);
+                        g9[3] = fma(w0, dB[0], g9[3]);
+                        g9[4] = fma(w1, dB[1], g9[4]);
+                        g9[5] = fma(w2, dB[2], g9[5]);
+                        g9[6] = fma(w0, dC[0], g9[6]);
+                        g9[7] = fma(w1, dC[1], g9[7]);
+                        g9[8] = fma(w2, dC[2], g9[8]);
                     }
-                }
             }
         }
-        const int aA = shell_atom[q.sa], aB = shell_atom[q.sb], aC = shell_atom[q.sc], aD = shell_atom[q.sd];
+        // ket shells: one atomic per lane; bra shells: one per warp while the
+        // warp holds one bra pair (the item order is bra-major)
+        if (count > 0) {
 #pragma unroll
-        for (int x = 0; x < 3; ++x) {
-            atomicAdd(grad + 3 * aA + x, gA[x]);
-            atomicAdd(grad + 3 * aB + x, gB[x]);
-            atomicAdd(grad + 3 * aC + x, gC[x]);
-            atomicAdd(grad + 3 * aD + x, -(gA[x] + gB[x] + gC[x]));
+            for (int x = 0; x < 3; ++x) {
+                atomicAdd(gshell + 3 * q.sc + x, g9[6 + x]);
+                atomicAdd(gshell + 3 * q.sd + x, -(g9[x] + g9[3 + x] + g9[6 + x]));
+            }
+        }
+        const int bra0 = __shfl_sync(0xffffffffu, q.bra, 0);
+        const bool one_bra = __all_sync(0xffffffffu, bra0 == q.bra);
+        if (one_bra) {
+            int idx;
+            const double s = warp_sum_transposed<6>(g9, lane, idx);
+            if (idx < 6 && (lane & 3) == 0) atomicAdd(gshell + 3 * (idx < 3 ? q.sa : q.sb) + idx % 3, s);
+        } else if (count > 0) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                atomicAdd(gshell + 3 * q.sa + x, g9[x]);
+                atomicAdd(gshell + 3 * q.sb + x, g9[3 + x]);
+            }
         }
     }
 }
 
-template <typename R>
+// ------------------------------------------------------------ warp mode --
+template <int LA, int LB, int LC, int LD> struct GradWarpLayout {
+    static constexpr int NCOMP = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD);
+    static constexpr int NR = (LA + LB + LC + LD + 1) / 2 + 1;
+    static constexpr int sC = LD + 1, sB = (LC + 2) * sC, sA = (LB + 1) * sB, G2 = (LA + 2) * sA;
+    // an odd pitch spreads the (root, axis) tables over the banks
+    static constexpr int pitch = G2 | 1;
+    static constexpr size_t pq_bytes = sizeof(double) * 3 * NR * pitch;
+    // primitive quartets of one pass: their (root, axis) tables occupy the
+    // lanes, within 16 KB of tables a warp
+    static constexpr int fit = 32 / (3 * NR);
+    static constexpr int PB = fit > 1 && pq_bytes * fit <= 16384 ? fit : (fit > 2 && pq_bytes * 2 <= 16384 ? 2 : 1);
+    static constexpr size_t warp_bytes = PB * pq_bytes + sizeof(double) * NCOMP;
+    static constexpr int warps = 4 * warp_bytes + sizeof(uint2) * NCOMP <= 56 * 1024 ? 4 : 2;
+    static constexpr size_t bytes = warps * warp_bytes + sizeof(uint2) * NCOMP;
+};
+
+// One warp per item.  Bound by shared-memory wavefronts (18 loads per
+// component and root for about 36 FP64 operations; neighbouring lanes'
+// components share most of them).
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(GradWarpLayout<LA, LB, LC, LD>::warps * 32)
+eri_grad_warp_kernel(const int4 *__restrict__ list, int nq, const PairInfo *__restrict__ pairs,
+                     const PrimPair *__restrict__ prims, const double *__restrict__ D, double *gshell)
+{
+    using Lay = GradWarpLayout<LA, LB, LC, LD>;
+    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
+    constexpr int NR = Lay::NR, NCOMP = Lay::NCOMP, PB = Lay::PB, PITCH = Lay::pitch, W = Lay::warps;
+    constexpr int sA = Lay::sA, sB = Lay::sB, sC = Lay::sC;
+    extern __shared__ __align__(16) unsigned char gsm[];
+    __shared__ double expo[W][PB][3];   // 2 alpha_a, 2 alpha_b, 2 alpha_c of the pass
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *tab = reinterpret_cast<double *>(gsm) + (size_t)warp * (Lay::warp_bytes / sizeof(double));
+    double *gam = tab + PB * 3 * NR * PITCH;
+    // per component: offsets of its x, y, z factors and the lowered powers
+    uint2 *meta = reinterpret_cast<uint2 *>(gsm + W * Lay::warp_bytes);
+    for (int t = threadIdx.x; t < NCOMP; t += W * 32) {
+        const int ab = t / NCD, cd = t - ab * NCD;
+        unsigned off[3], pw = 0;
+        for (int x = 0; x < 3; ++x) {
+            const int a = cart_l(LA, ab / NB, x), b = cart_l(LB, ab % NB, x), c = cart_l(LC, cd / ND, x),
+                      d = cart_l(LD, cd % ND, x);
+            off[x] = a * sA + b * sB + c * sC + d;
+            pw |= (unsigned)(a | (b << 2) | (c << 4)) << (6 * x);
+        }
+        meta[t] = make_uint2(off[0] | (off[1] << 10) | (off[2] << 20), pw);
+    }
+    __syncthreads();
+    for (int qi = blockIdx.x * W + warp; qi < nq; qi += gridDim.x * W) {
+        const int4 e = list[qi];
+        const PairInfo &pb = pairs[e.x];
+        const PairInfo &pk = pairs[e.y];
+        const QCtx q = make_qctx(pb, pk, e.x, e.y);
+        const bool bd = q.sa == q.sb, kd = q.sc == q.sd, qd = q.bra == q.ket, af = q.fa > q.fb;
+        const double *Db = D + q.bo;
+        for (int t = lane; t < NCOMP; t += 32) {
+            const int ab = t / NCD, cd = t - ab * NCD, ia = ab / NB, ib = ab % NB, ic = cd / ND, id = cd % ND;
+            gam[t] = comp_weight(ia, ib, ic, id, bd, kd, qd, af) *
+                     gamma_of(Db, q.nm, q.fa + ia, q.fb + ib, q.fc + ic, q.fd + id);
+        }
+        double g9[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) g9[k] = 0.0;
+        const double AB[3] = {pb.AB[0], pb.AB[1], pb.AB[2]};
+        const int npb = pb.nprim;
+        for (int p0 = 0; p0 < e.w; p0 += PB) {
+            const int nb = e.w - p0 < PB ? e.w - p0 : PB;
+            __syncwarp();   // the tables of the pass before are read; gam is written
+            if (lane < nb * 3 * NR) {
+                const int b = lane / (3 * NR), rx = lane - b * (3 * NR), r = rx / 3, x = rx - r * 3;
+                const int g = e.z + p0 + b, ik = g / npb, ib = g - ik * npb;
+                const PrimPair *pp = prims + pb.prim_off + ib, *pq = prims + pk.prim_off + ik;
+                const PrimJK P = load_prim_jk(pp), Q = load_prim_jk(pq);
+                const double PQ[3] = {P.P[0] - Q.P[0], P.P[1] - Q.P[1], P.P[2] - Q.P[2]};
+                const double rs = rsqrt_nr(P.zeta + Q.zeta), izpe = rs * rs;
+                const double T = P.zeta * Q.zeta * izpe * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+                double u, w;
+                rys_root(NR, r, T, u, w);
+                const RysCoef k = rys_coef(u, P.zeta, Q.zeta, P.izeta, Q.izeta, izpe);
+                const double Px = x == 0 ? P.P[0] : (x == 1 ? P.P[1] : P.P[2]);
+                const double Qx = x == 0 ? Q.P[0] : (x == 1 ? Q.P[1] : Q.P[2]);
+                rys2d_c<LA + 1, LB, LC + 1, LD, double>(k, Px - pb.A[x], Qx - pk.A[x], Px - Qx, pb.AB[x], pk.AB[x],
+                                                        x == 0 ? w * P.K * Q.K * rs : 1.0, tab + lane * PITCH);
+                if (rx == 0) {
+                    const double a2 = 2.0 * __ldg(&pp->alpha_a);
+                    expo[warp][b][0] = a2;
+                    expo[warp][b][1] = 2.0 * P.zeta - a2;
+                    expo[warp][b][2] = 2.0 * __ldg(&pq->alpha_a);
+                }
+            }
+            __syncwarp();
+            for (int t = lane; t < nb * NR * NCOMP; t += 32) {
+                const int br = t / NCOMP, comp = t - br * NCOMP, b = br / NR;
+                const double gm = gam[comp];
+                if (gm == 0.0) continue;
+                const uint2 m = meta[comp];
+                const double a2 = expo[warp][b][0], b2 = expo[warp][b][1], c2 = expo[warp][b][2];
+                double I[3], dA[3], dB[3], dC[3];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    const double *g = tab + (br * 3 + x) * PITCH + ((m.x >> (10 * x)) & 1023u);
+                    const int pw = m.y >> (6 * x), a = pw & 3, b1 = (pw >> 2) & 3, c = (pw >> 4) & 3;
+                    const double up = g[sA];
+                    I[x] = g[0];
+                    // (a lowered power of zero multiplies the entry itself by zero)
+                    dA[x] = fma(a2, up, -(double)a * g[a ? -sA : 0]);
+                    dB[x] = fma(b2, fma(AB[x], I[x], up), LB > 0 ? -(double)b1 * g[b1 ? -sB : 0] : 0.0);
+                    dC[x] = fma(c2, g[sC], LC > 0 ? -(double)c * g[c ? -sC : 0] : 0.0);
+                }
+                const double w0 = gm * I[1] * I[2], gx = gm * I[0], w1 = gx * I[2], w2 = gx * I[1];
+                g9[0] = fma(w0, dA[0], g9[0]);
+                g9[1] = fma(w1, dA[1], g9[1]);
+                g9[2] = fma(w2, dA[2], g9[2]);
+                g9[3] = fma(w0, dB[0], g9[3]);
+                g9[4] = fma(w1, dB[1], g9[4]);
+                g9[5] = fma(w2, dB[2], g9[5]);
+                g9[6] = fma(w0, dC[0], g9[6]);
+                g9[7] = fma(w1, dC[1], g9[7]);
+                g9[8] = fma(w2, dC[2], g9[8]);
+            }
+        }
+        double g12[12];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) g12[k] = g9[k];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) g12[9 + x] = -(g9[x] + g9[3 + x] + g9[6 + x]);
+        int idx;
+        const double s = warp_sum_transposed<12>(g12, lane, idx);
+        if (idx < 12 && (lane & 1) == 0) {
+            const int sh = idx < 3 ? q.sa : (idx < 6 ? q.sb : (idx < 9 ? q.sc : q.sd));
+            atomicAdd(gshell + 3 * sh + idx % 3, s);
+        }
+        __syncwarp();   // gam is rewritten for the next item
+    }
+}
+
+// grad[3 atom] += the atom's shells
+__global__ void grad_gather_kernel(int nshell, const int *__restrict__ shell_atom, const double *__restrict__ gshell,
+                                   double *grad)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * nshell) return;
+    atomicAdd(grad + 3 * shell_atom[t / 3] + t % 3, gshell[t]);
+}
+
+cudaError_t launch_grad_gather(int nshell, const int *shell_atom, const double *gshell, double *grad, cudaStream_t st)
+{
+    if (nshell > 0)
+        grad_gather_kernel<<<(3 * nshell + 127) / 128, 128, 0, st>>>(nshell, shell_atom, gshell, grad);
+    return cudaGetLastError();
+}
+
+// More than 27 components' Gamma and tables leave the registers in thread
+// mode; below, a warp's lanes would share too few products.
+template <int LA, int LB, int LC, int LD>
+static cudaError_t eri_grad_launch(const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
+                                   const double *D, double *gshell, cudaStream_t st, int nsm)
+{
+    if constexpr (ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) <= 27) {
+        int grid = (nq + 127) / 128;
+        if (grid > nsm * 32) grid = nsm * 32;
+        eri_grad_thread_kernel<LA, LB, LC, LD><<<grid, 128, 0, st>>>(list, nq, pairs, prims, D, gshell);
+    } else {
+        using Lay = GradWarpLayout<LA, LB, LC, LD>;
+        auto kern = eri_grad_warp_kernel<LA, LB, LC, LD>;
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
+        if (e != cudaSuccess) return e;
+        int grid = (nq + Lay::warps - 1) / Lay::warps;
+        if (grid > nsm * 16) grid = nsm * 16;
+        kern<<<grid, Lay::warps * 32, Lay::bytes, st>>>(list, nq, pairs, prims, D, gshell);
+    }
+    return cudaGetLastError();
+}
+
 cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                        const double *D, const double *fscale, const int *shell_atom, int n, double *grad,
-                        cudaStream_t st, int nsm)
+                        const double *Dscaled, double *gshell, cudaStream_t st, int nsm)
 {
     if (nq <= 0) return cudaSuccess;
-    int grid = (nq + 127) / 128;
-    if (grid > nsm * 32) grid = nsm * 32;
 #define PQB_GCASE(CB, CK)                                                                                      \
     case CB *(CB + 1) / 2 + CK:                                                                               \
-        eri_grad_kernel<pc_la(CB), pc_lb(CB), pc_la(CK), pc_lb(CK), R>                                         \
-            <<<grid, 128, 0, st>>>(list, nq, pairs, prims, D, fscale, shell_atom, n, grad);                   \
-        break;
+        return eri_grad_launch<pc_la(CB), pc_lb(CB), pc_la(CK), pc_lb(CK)>(list, nq, pairs, prims, Dscaled, gshell, \
+                                                                           st, nsm);
     switch (qc) {
         PQB_GCASE(0, 0)
         PQB_GCASE(1, 0) PQB_GCASE(1, 1)
@@ -160,21 +362,6 @@ cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs,
         return cudaErrorInvalidValue;
     }
 #undef PQB_GCASE
-    return cudaGetLastError();
-}
-
-cudaError_t launch_grad_f64(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                            const double *D, const double *fscale, const int *shell_atom, int n, double *grad,
-                            cudaStream_t st, int nsm)
-{
-    return launch_grad<double>(qc, list, nq, pairs, prims, D, fscale, shell_atom, n, grad, st, nsm);
-}
-
-cudaError_t launch_grad_f32(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                            const double *D, const double *fscale, const int *shell_atom, int n, double *grad,
-                            cudaStream_t st, int nsm)
-{
-    return launch_grad<float>(qc, list, nq, pairs, prims, D, fscale, shell_atom, n, grad, st, nsm);
 }
 
 }  // namespace pqb

@@ -39,10 +39,9 @@ cudaError_t launch_jk2_f32(int qc, const int4 *list, int nq, const PairInfo *pai
                            double *const Kacc[2], cudaStream_t st, int nsm, const ItemScreen &scr = ItemScreen{});
 cudaError_t launch_schwarz_f64(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
                                unsigned long long *Q2bits, const double *fscale, cudaStream_t st, int nsm);
-cudaError_t launch_grad_f64(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                            const double *D, const double *fscale, const int *shell_atom, int n, double *grad,
-                            cudaStream_t st, int nsm);
-cudaError_t launch_grad_f32(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                            const double *D, const double *fscale, const int *shell_atom, int n, double *grad,
-                            cudaStream_t st, int nsm);
+// Adds dE2 per shell (gshell[3 nshell]) from the pre-scaled density; the
+// gather adds the shells to their atoms.
+cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
+                        const double *Dscaled, double *gshell, cudaStream_t st, int nsm);
+cudaError_t launch_grad_gather(int nshell, const int *shell_atom, const double *gshell, double *grad, cudaStream_t st);
 }  // namespace pqb

@@ -68,6 +68,7 @@ struct pqb_ctx {
     int64_t plan_prims[2][kNumQuartetClass] = {{0}};
     std::vector<int4> plan_h;        // host copy of the plan (for sharding)
     int *d_shell_atom = nullptr;     // atom index of every shell (gradients)
+    double *d_gshell = nullptr;      // per-shell sums of the two-electron gradient (allocated with it)
     int2 *d_pk_tiles = nullptr;      // (i, j0) tiles of the stored-integral J/K kernel
     int pk_tiles_n = 0, pk_tiles_nbf = -1;
     bool packed_simple = false;      // force the one-block-per-row stored J/K kernel (tests)
@@ -1040,6 +1041,8 @@ static void release_basis(pqb_ctx *ctx)
     free_dev(ctx->d_diag);
     free_dev(ctx->d_plan);
     free_dev(ctx->d_shell_atom);
+    free_dev(ctx->d_gshell);
+    ctx->d_gshell = nullptr;
     free_dev(ctx->d_mol_off);
     free_dev(ctx->d_mol_n);
     ctx->d_shell_atom = nullptr;
@@ -2134,6 +2137,9 @@ static int set_shell_atoms_impl(pqb_ctx *ctx, const int *shell_atom)
     if (!ctx || !shell_atom) return fail(ctx, PQB_E_ARG, "pqb_set_shell_atoms: bad arguments");
     if (!ctx->d_pairs) return fail(ctx, PQB_E_STATE, "pqb_set_shell_atoms: no basis uploaded");
     PQB_CK(ctx, cudaSetDevice(ctx->device));
+    // what pqb_grad_2e needs, so that it allocates nothing itself
+    if (!ctx->d_gshell) PQB_CK(ctx, cudaMalloc(&ctx->d_gshell, sizeof(double) * 3 * ctx->nshell));
+    PQB_CK(ctx, ensure_streams(ctx));
     if (!ctx->d_shell_atom) PQB_CK(ctx, cudaMalloc(&ctx->d_shell_atom, sizeof(int) * ctx->nshell));
     PQB_CK(ctx, cudaMemcpy(ctx->d_shell_atom, shell_atom, sizeof(int) * ctx->nshell, cudaMemcpyHostToDevice));
     return PQB_OK;
@@ -2157,18 +2163,24 @@ static int grad_2e_impl(pqb_ctx *ctx, const double *D, double *grad, int mode, v
     if (!ctx->d_shell_atom) return fail(ctx, PQB_E_STATE, "pqb_grad_2e: call pqb_set_shell_atoms first");
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
-    for (int part = 0; part < 2; ++part)
-        for (int c = 0; c < kNumQuartetClass; ++c) {
-            const int nq = (int)ctx->plan_cnt[part][c];
-            if (nq == 0) continue;
-            const int4 *list = ctx->d_plan + ctx->plan_off[part][c];
-            if (part == 1 && mode == PQB_MIXED)
-                PQB_CK(ctx, launch_grad_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, D, ctx->d_fscale,
-                                            ctx->d_shell_atom, ctx->nbf, grad, st, ctx->nsm));
-            else
-                PQB_CK(ctx, launch_grad_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, D, ctx->d_fscale,
-                                            ctx->d_shell_atom, ctx->nbf, grad, st, ctx->nsm));
-        }
+    (void)mode;   // both lists in FP64: one launch per class over the class-major plan
+    scale_elements_kernel<<<ctx->nsm * 4, 256, 0, st>>>(D, ctx->d_escale, ctx->d_Dscaled, ctx->d_Dscaled_f,
+                                                         ctx->dense_len);
+    PQB_CK(ctx, cudaMemsetAsync(ctx->d_gshell, 0, sizeof(double) * 3 * ctx->nshell, st));
+    // highest angular momentum first: its items run longest
+    PQB_CK(ctx, cudaEventRecord(ctx->ev_fork, st));
+    for (int k = 0; k < pqb_ctx::kStreams; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
+    for (int c = kNumQuartetClass - 1, k = 0; c >= 0; --c) {
+        const int nq = (int)(ctx->plan_cnt[0][c] + ctx->plan_cnt[1][c]);
+        if (nq == 0) continue;
+        PQB_CK(ctx, launch_grad(c, ctx->d_plan + ctx->plan_off[0][c], nq, ctx->d_pairs, ctx->d_prims, ctx->d_Dscaled,
+                                ctx->d_gshell, ctx->streams[k++ % pqb_ctx::kStreams], ctx->nsm));
+    }
+    for (int k = 0; k < pqb_ctx::kStreams; ++k) {
+        PQB_CK(ctx, cudaEventRecord(ctx->ev_join[k], ctx->streams[k]));
+        PQB_CK(ctx, cudaStreamWaitEvent(st, ctx->ev_join[k], 0));
+    }
+    PQB_CK(ctx, launch_grad_gather(ctx->nshell, ctx->d_shell_atom, ctx->d_gshell, grad, st));
     return PQB_OK;
 }
 
