@@ -209,6 +209,9 @@ int pqb_jk_direct_class(pqb_ctx *ctx, const double *D, double *Jacc, double *Kac
  *   P = nbf(nbf+1)/2): out holds nrows * nbf * nbf doubles.
  * pqb_mo_unpack_pairs: out[(mu*nbf + nu)*ncol + c] = Y[pair(mu,nu)*ncol + c]
  *   (rows stored per packed AO pair, unpacked to both orders).
+ * pqb_mo_contract_pairs: out[((a*nbf + nu)*nb + b)*nj + j] =
+ *   sum_mu C[mu*na + a] Y[(b*P + pair(mu,nu))*nj + j], without the unpacked
+ *   rows (nb * nj at most 4,194,240).
  * pqb_mo_pack: moints[ijkl2intindex(a,i,b,j)] = Z[((a*nmo + i)*nocc + b)*nmo + j]
  *   for a, b < nocc, i, j < nmo (len = Q(Q+1)/2, Q = nmo(nmo+1)/2: the
  *   packed MO array TransformIntsMP2 returns; other slots are left as is).
@@ -216,6 +219,7 @@ int pqb_jk_direct_class(pqb_ctx *ctx, const double *D, double *Jacc, double *Kac
  *   (e_a + e_b - e_r - e_s) from V[((a*nvirt + r)*nocc + b)*nvirt + s]. */
 int pqb_mo_unpack_rows(const double *ints, int64_t len, int nbf, int64_t row0, int nrows, double *out, void *stream);
 int pqb_mo_unpack_pairs(const double *Y, int nbf, int64_t ncol, double *out, void *stream);
+int pqb_mo_contract_pairs(const double *Y, int nbf, int nb, int nj, const double *C, int na, double *out, void *stream);
 int pqb_mo_pack(const double *Z, int nocc, int nmo, double *moints, int64_t len, void *stream);
 int pqb_mp2_pairs(const double *V, int nocc, int nvirt, const double *e_occ, const double *e_virt, double *Epair,
                   void *stream);

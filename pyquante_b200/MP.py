@@ -6,15 +6,18 @@
 ``Ints`` is the packed AO array of ``Ints.getints`` (a PackedInts, a torch
 tensor or an array).  The reference transforms one index at a time in
 Python loops, O(N^5) calls of ``dot``; here the four quarter transformations
-are FP64 GEMMs on the GPU (cuBLAS DGEMM through torch), fed by the engine's
-own gather kernels (pqb_mo_unpack_rows, pqb_mo_unpack_pairs) that turn the
-8-fold packed order into dense rows, and the pair energies are one kernel
-(pqb_mp2_pairs).  Everything is FP64: no reduced-precision tensor-core path.
+are FP64 matrix products on the GPU: three cuBLAS DGEMMs through torch and the
+engine's own contraction over one index of the packed AO pair
+(pqb_mo_contract_pairs), with the gather of the 8-fold packed order into
+dense rows (pqb_mo_unpack_rows) before and the pair energies
+(pqb_mp2_pairs) after them.  Everything is FP64: no reduced-precision
+tensor-core path.
 
     1. (mu nu|sigma eta) -> (mu nu|b j): per batch of packed AO pairs mu >= nu,
-       unpack the rows and contract eta with C[:, j] and sigma with C[:, b];
-    2. (mu nu|b j) -> (a i|b j): unpack the pair index to (mu, nu) and
-       contract nu with C[:, i] and mu with C[:, a].
+       unpack the rows and contract sigma with C[:, b], then eta with C[:, j]
+       (occupied b first: 2 P N^2 nocc operations instead of 2 P N^2 nvirt);
+    2. (mu nu|b j) -> (a i|b j): contract mu with C[:, a] on the packed pair
+       rows, then nu with C[:, i].
 MP2 takes i, j over the virtual orbitals only; TransformIntsMP2 over all MOs,
 as the reference does, and stores (ai|bj) at ijkl2intindex(a, i, b, j) of a
 packed MO array (zeros elsewhere).
@@ -44,34 +47,38 @@ def _check(rc, what):
 
 
 def _half_transform(ints, nbf, Cb, Cj, stream=None):
-    """Y[P, nb, nj] = (mu nu|b j) = sum_{sigma eta} Cb[sigma, b] Cj[eta, j]
-    (mu nu|sigma eta) for every packed AO pair mu >= nu."""
+    """Y[nb, P, nj] = (mu nu|b j) = sum_{sigma eta} Cb[sigma, b] Cj[eta, j]
+    (mu nu|sigma eta) for every packed AO pair mu >= nu.  The occupied index
+    goes first: it is the smaller one, and both steps are then plain GEMMs of
+    tall matrices."""
     lib = _lib.load()
     P = nbf * (nbf + 1) // 2
     nb, nj = Cb.shape[1], Cj.shape[1]
-    Y = torch.empty((P, nb, nj), dtype=torch.float64, device=ints.device)
+    Y = torch.empty((nb, P, nj), dtype=torch.float64, device=ints.device)
     batch = max(1, min(P, _ROW_BATCH_BYTES // (8 * nbf * nbf)))
     X = torch.empty((batch, nbf, nbf), dtype=torch.float64, device=ints.device)
+    T = torch.empty(nb * batch * nbf, dtype=torch.float64, device=ints.device)
     CbT = Cb.T.contiguous()
+    Cjb = Cj.expand(nb, nbf, nj)
     for r0 in range(0, P, batch):
         nr = min(batch, P - r0)
         Xb = X[:nr]
         _check(lib.pqb_mo_unpack_rows(ptr(ints), ints.numel(), nbf, r0, nr, ptr(Xb), stream_ptr(stream)),
                "pqb_mo_unpack_rows")
-        T1 = torch.matmul(Xb.view(nr * nbf, nbf), Cj).view(nr, nbf, nj)     # eta -> j
-        torch.matmul(CbT, T1, out=Y[r0:r0 + nr])                          # sigma -> b
+        T1 = T[:nb * nr * nbf]
+        torch.matmul(CbT, Xb.view(nr * nbf, nbf).T, out=T1.view(nb, nr * nbf))        # sigma -> b
+        torch.bmm(T1.view(nb, nr, nbf), Cjb, out=Y[:, r0:r0 + nr])                    # eta -> j
     return Y
 
 
 def _second_half(Y, nbf, Ca, Ci, stream=None):
-    """Z[a, i, c] = sum_{mu nu} Ca[mu, a] Ci[nu, i] Y[pair(mu, nu), c]."""
+    """Z[a, i, b, j] = sum_{mu nu} Ca[mu, a] Ci[nu, i] Y[b, pair(mu, nu), j]."""
     lib = _lib.load()
-    P, ncol = Y.shape[0], Y.shape[1] * Y.shape[2]
-    Yf = torch.empty((nbf, nbf, ncol), dtype=torch.float64, device=Y.device)
-    _check(lib.pqb_mo_unpack_pairs(ptr(Y), nbf, ncol, ptr(Yf), stream_ptr(stream)), "pqb_mo_unpack_pairs")
-    T = torch.matmul(Ca.T.contiguous(), Yf.view(nbf, nbf * ncol)).view(Ca.shape[1], nbf, ncol)   # mu -> a
-    del Yf
-    return torch.matmul(Ci.T.contiguous(), T)                                                 # nu -> i
+    nb, nj, na = Y.shape[0], Y.shape[2], Ca.shape[1]
+    T = torch.empty((na, nbf, nb * nj), dtype=torch.float64, device=Y.device)
+    _check(lib.pqb_mo_contract_pairs(ptr(Y), nbf, nb, nj, ptr(Ca), na, ptr(T), stream_ptr(stream)),
+           "pqb_mo_contract_pairs")                                              # mu -> a
+    return torch.matmul(Ci.T.contiguous(), T)                                       # nu -> i
 
 
 class MOInts:

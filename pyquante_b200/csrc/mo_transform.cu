@@ -8,8 +8,11 @@
 //   * mo_unpack_rows_kernel: a batch of packed bra rows (ij| into dense
 //     N x N matrices (ij|kl), for every kl (the gather of the 8-fold packed
 //     order, Src/cints.c:413-425, in 64 bits);
-//   * mo_unpack_pairs_kernel: half-transformed integrals stored per packed
-//     AO pair back into dense (mu, nu) rows, symmetric;
+//   * mo_contract_pairs_kernel: the contraction over one index of the packed
+//     AO pair of the half-transformed integrals, as FP64 tensor-core tiles
+//     that gather the pair rows;
+//   * mo_unpack_pairs_kernel: rows stored per packed AO pair into dense
+//     (mu, nu) rows, symmetric;
 //   * mo_pack_kernel: (ai|bj) into the reference's packed MO array at
 //     ijkl2intindex(a, i, b, j);
 //   * mp2_pairs_kernel: the pair energies
@@ -19,6 +22,9 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pyquante_b200.h"
+#include "dmma.cuh"
+
+using namespace pqb;
 
 namespace {
 
@@ -32,17 +38,48 @@ __device__ __forceinline__ int64_t packed_of(int64_t ij, int64_t kl)
     return ij >= kl ? ij * (ij + 1) / 2 + kl : kl * (kl + 1) / 2 + ij;
 }
 
-// out[r][k][l] = (IJ_r|kl), IJ_r = row0 + r.  One thread per output element
-// (writes coalesced; the reads are the packed rows, contiguous for kl <= IJ
-// and strided by kl beyond).
-__global__ void mo_unpack_rows_kernel(const double *__restrict__ ints, int nbf, int64_t row0, int nrows,
-                                      double *__restrict__ out)
+// out[r][k][l] = (IJ_r|kl), IJ_r = row0 + r.  A block takes a 32 x 32 tile
+// k >= l of four consecutive bra rows: each packed element is read once, along
+// l where the row holds it (kl <= IJ) and four neighbours IJ at a time, one
+// 32-byte sector, where a later row does, and goes out twice, the transposed
+// half through shared memory.  Bound by the 8 N^2 bytes a row that it writes:
+// all 11,325 rows at N = 150 (2.04 GB out) take 0.95 ms, 1.65 ms
+// with one thread per output element (64-bit divisions, strided reads of every
+// element twice).
+constexpr int kUnpackRows = 4;
+
+__global__ void __launch_bounds__(256) mo_unpack_rows_kernel(const double *__restrict__ ints, int nbf, int64_t row0,
+                                                             int nrows, int ntile2, double *__restrict__ out)
 {
-    const int64_t nn = (int64_t)nbf * nbf, total = nn * nrows;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / nn, kl = t - r * nn;
-        const int64_t k = kl / nbf, l = kl - k * nbf;
-        out[t] = __ldg(ints + packed_of(row0 + r, pair_of(k, l)));
+    __shared__ double s[kUnpackRows][32][33];
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int tile = blockIdx.x % ntile2, r0 = (int)(blockIdx.x / ntile2) * kUnpackRows;
+    int kt = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
+    while (kt * (kt + 1) / 2 > tile) --kt;
+    while ((kt + 1) * (kt + 2) / 2 <= tile) ++kt;
+    const int lt = tile - kt * (kt + 1) / 2;
+    const int64_t IJ0 = row0 + r0;
+    const int rows = nrows - r0 < kUnpackRows ? nrows - r0 : kUnpackRows;
+    for (int kk = ty; kk < 32; kk += 8) {
+        const int k = kt * 32 + kk, l = lt * 32 + lane;
+        if (k < nbf && l <= k) {
+            const int64_t KL = (int64_t)k * (k + 1) / 2 + l, col = KL * (KL + 1) / 2 + IJ0;
+#pragma unroll
+            for (int r = 0; r < kUnpackRows; ++r) {
+                const int64_t IJ = IJ0 + r;
+                if (r < rows) s[r][kk][lane] = __ldg(ints + (KL <= IJ ? IJ * (IJ + 1) / 2 + KL : col + r));
+            }
+        }
+    }
+    __syncthreads();
+    for (int r = 0; r < rows; ++r) {
+        double *o = out + (int64_t)(r0 + r) * nbf * nbf;
+        for (int kk = ty; kk < 32; kk += 8) {
+            const int k = kt * 32 + kk, l = lt * 32 + lane;
+            if (k < nbf && l < nbf) o[(int64_t)k * nbf + l] = lt < kt || lane <= kk ? s[r][kk][lane] : s[r][lane][kk];
+            const int kT = lt * 32 + kk, lT = kt * 32 + lane;
+            if (lt < kt && lT < nbf) o[(int64_t)kT * nbf + lT] = s[r][lane][kk];
+        }
     }
 }
 
@@ -55,6 +92,109 @@ __global__ void mo_unpack_pairs_kernel(const double *__restrict__ Y, int nbf, in
         const int64_t mu = row / nbf, nu = row - mu * nbf;
         out[t] = __ldg(Y + pair_of(mu, nu) * ncol + c);
     }
+}
+
+// out[((a * nbf + nu) * nb + b) * nj + j] =
+//     sum_mu C[mu * na + a] Y[(b * P + pair(mu, nu)) * nj + j],
+// the contraction over one index of a symmetric pair (mu, nu) stored once, as
+// FP64 tensor-core tiles: a block takes one nu, MT = 8 MF of the na columns of
+// C and 64 of the nb * nj columns (b, j), and gathers the rows pair(mu, nu) of
+// Y as its K dimension, so the pair index is never unpacked to nbf^2 rows.
+// nu runs fastest over the grid: the P rows of a 64-column strip (5.8 MB at
+// N = 150) stay in L2 for both orders of every pair.  N = 150, 30 columns of
+// C, 3,600 of Y: 0.29 ms (16.5 TFLOP/s); the unpacked copy alone took 0.37 ms.
+constexpr int kPairK = 16, kPairCols = 64, kPairStages = 3, kPairPitchB = kPairCols + 4;
+
+template <int MF> struct PairLayout {
+    static constexpr int MT = 8 * MF;
+    static constexpr int pitchA = (MT + 15) / 16 * 16 + 4;   // 4 mod 16 doubles: fragment reads hit distinct banks
+    static constexpr int stage = kPairK * (pitchA + kPairPitchB);
+    static constexpr size_t bytes = sizeof(double) * kPairStages * stage;
+};
+
+template <int MF>
+__global__ void __launch_bounds__(128) mo_contract_pairs_kernel(const double *__restrict__ Y, int nbf, int nb, int nj,
+                                                                const double *__restrict__ C, int na,
+                                                                double *__restrict__ out)
+{
+    using Lay = PairLayout<MF>;
+    extern __shared__ double sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nu = blockIdx.x, a0 = blockIdx.z * Lay::MT;
+    const int64_t P = (int64_t)nbf * (nbf + 1) / 2, ncol = (int64_t)nb * nj, c0 = (int64_t)blockIdx.y * kPairCols;
+    // this thread's column of the B tile
+    const int64_t cc = c0 + (tid & 63), cs = cc < ncol ? cc : 0;
+    const double *Yc = Y + (cs / nj) * P * nj + cs % nj;
+    auto load = [&](int k0, int slot) {
+        double *As = sm + slot * Lay::stage, *Bs = As + kPairK * Lay::pitchA;
+        for (int e = tid; e < kPairK * Lay::MT; e += 128) {
+            const int k = e / Lay::MT, a = e - k * Lay::MT;
+            const bool ok = k0 + k < nbf && a0 + a < na;
+            cp_async8(As + k * Lay::pitchA + a, ok ? C + (int64_t)(k0 + k) * na + a0 + a : C, ok);
+        }
+#pragma unroll
+        for (int k = tid >> 6; k < kPairK; k += 2) {
+            const bool ok = k0 + k < nbf && cc < ncol;
+            cp_async8(Bs + k * kPairPitchB + (tid & 63), ok ? Yc + pair_of(k0 + k, nu) * nj : Y, ok);
+        }
+    };
+    double acc[MF][2][2];
+#pragma unroll
+    for (int m = 0; m < MF; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
+    const int nk = (nbf + kPairK - 1) / kPairK;
+#pragma unroll
+    for (int s = 0; s < kPairStages - 1; ++s) {
+        if (s < nk) load(s * kPairK, s);
+        cp_async_commit();
+    }
+    for (int t = 0; t < nk; ++t) {
+        cp_async_wait<kPairStages - 2>();
+        __syncthreads();   // stage t has landed; stage t - 1's readers are done
+        if (t + kPairStages - 1 < nk) load((t + kPairStages - 1) * kPairK, (t + kPairStages - 1) % kPairStages);
+        cp_async_commit();
+        const double *As = sm + (t % kPairStages) * Lay::stage + (lane & 3) * Lay::pitchA + (lane >> 2);
+        const double *Bs = sm + (t % kPairStages) * Lay::stage + kPairK * Lay::pitchA + (lane & 3) * kPairPitchB +
+                           warp * 16 + (lane >> 2);
+#pragma unroll
+        for (int k = 0; k < kPairK; k += 4) {
+            double b[2], a[MF];
+#pragma unroll
+            for (int n = 0; n < 2; ++n) b[n] = Bs[k * kPairPitchB + 8 * n];
+#pragma unroll
+            for (int m = 0; m < MF; ++m) a[m] = As[k * Lay::pitchA + 8 * m];
+#pragma unroll
+            for (int m = 0; m < MF; ++m)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) dmma(acc[m][n], a[m], b[n]);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MF; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const int a = a0 + 8 * m + (lane >> 2);
+            const int64_t c = c0 + warp * 16 + 8 * n + 2 * (lane & 3);
+            double *o = out + ((int64_t)a * nbf + nu) * ncol + c;
+            if (a < na && c < ncol) o[0] = acc[m][n][0];
+            if (a < na && c + 1 < ncol) o[1] = acc[m][n][1];
+        }
+}
+
+template <int MF>
+cudaError_t launch_contract_pairs(const double *Y, int nbf, int nb, int nj, const double *C, int na, double *out, int nz,
+                                  cudaStream_t st)
+{
+    using Lay = PairLayout<MF>;
+    const cudaError_t e = cudaFuncSetAttribute(mo_contract_pairs_kernel<MF>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
+    if (e != cudaSuccess) return e;
+    const int64_t strips = ((int64_t)nb * nj + kPairCols - 1) / kPairCols;
+    // (the grid's y dimension holds 65535 strips a launch: 4.2 M columns, more than Y's rows fit in memory for)
+    if (strips > 65535) return cudaErrorInvalidValue;
+    mo_contract_pairs_kernel<MF><<<dim3(nbf, (unsigned)strips, nz), 128, Lay::bytes, st>>>(Y, nbf, nb, nj, C, na, out);
+    return cudaGetLastError();
 }
 
 // moints[ijkl2intindex(a, i, b, j)] = Z[((a * nmo + i) * nocc + b) * nmo + j]
@@ -117,8 +257,15 @@ int pqb_mo_unpack_rows(const double *ints, int64_t len, int nbf, int64_t row0, i
     if (!ints || !out || nbf <= 0 || nrows <= 0 || row0 < 0) return PQB_E_ARG;
     const int64_t P = (int64_t)nbf * (nbf + 1) / 2;
     if (len != P * (P + 1) / 2 || row0 + nrows > P) return PQB_E_SHAPE;
-    const int64_t total = (int64_t)nbf * nbf * nrows;
-    mo_unpack_rows_kernel<<<grid_for(total), 256, 0, (cudaStream_t)stream>>>(ints, nbf, row0, nrows, out);
+    const int nt = (nbf + 31) / 32, nt2 = nt * (nt + 1) / 2;
+    // (at most 2^31 - 1 blocks a launch)
+    const int64_t groups = ((int64_t)nrows + kUnpackRows - 1) / kUnpackRows, most = 0x7fffffff / nt2;
+    for (int64_t g = 0; g < groups; g += most) {
+        const int64_t r = g * kUnpackRows, ng = groups - g < most ? groups - g : most;
+        const int64_t left = nrows - r < ng * kUnpackRows ? nrows - r : ng * kUnpackRows;
+        mo_unpack_rows_kernel<<<(unsigned)(ng * nt2), 256, 0, (cudaStream_t)stream>>>(ints, nbf, row0 + r, (int)left, nt2,
+                                                                                      out + r * nbf * nbf);
+    }
     return cudaGetLastError() == cudaSuccess ? PQB_OK : PQB_E_CUDA;
 }
 
@@ -128,6 +275,26 @@ int pqb_mo_unpack_pairs(const double *Y, int nbf, int64_t ncol, double *out, voi
     const int64_t total = (int64_t)nbf * nbf * ncol;
     mo_unpack_pairs_kernel<<<grid_for(total), 256, 0, (cudaStream_t)stream>>>(Y, nbf, ncol, out);
     return cudaGetLastError() == cudaSuccess ? PQB_OK : PQB_E_CUDA;
+}
+
+int pqb_mo_contract_pairs(const double *Y, int nbf, int nb, int nj, const double *C, int na, double *out, void *stream)
+{
+    if (!Y || !C || !out || nbf <= 0 || nb <= 0 || nj <= 0 || na <= 0) return PQB_E_ARG;
+    // rows of C a block: all of them up to 64, else equal parts
+    const int nz = (na + 63) / 64, mf = ((na + nz - 1) / nz + 7) / 8;
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (mf) {
+    case 1: e = launch_contract_pairs<1>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 2: e = launch_contract_pairs<2>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 3: e = launch_contract_pairs<3>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 4: e = launch_contract_pairs<4>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 5: e = launch_contract_pairs<5>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 6: e = launch_contract_pairs<6>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 7: e = launch_contract_pairs<7>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    case 8: e = launch_contract_pairs<8>(Y, nbf, nb, nj, C, na, out, nz, st); break;
+    }
+    return e == cudaSuccess ? PQB_OK : PQB_E_CUDA;
 }
 
 int pqb_mo_pack(const double *Z, int nocc, int nmo, double *moints, int64_t len, void *stream)

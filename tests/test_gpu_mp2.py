@@ -13,7 +13,7 @@ import pyq_oracle as O
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from pyquante_b200 import MP, Ints, geometries  # noqa: E402
+from pyquante_b200 import MP, Ints, _lib, geometries  # noqa: E402
 from pyquante_b200.Basis.basis import BasisSet  # noqa: E402
 from pyquante_b200.hartree_fock import rhf  # noqa: E402
 from pyquante_b200.Molecule import Molecule  # noqa: E402
@@ -104,3 +104,38 @@ def test_mp2_h2o8_properties():
         MP._ROW_BATCH_BYTES = saved
     print("(H2O)8 RHF %.10f MP2 correction %.10f" % (e, e1))
     assert e1 < 0.0 and abs(e1 - e2) < 1e-11
+
+
+@pytest.mark.parametrize("n,row0,nrows", [(1, 0, 1), (31, 0, 496), (32, 5, 6), (33, 557, 4), (65, 7, 13)])
+def test_unpack_rows_at_tile_edges(n, row0, nrows):
+    """Copies: equal to the packed array's own elements."""
+    P = n * (n + 1) // 2
+    ints = torch.arange(P * (P + 1) // 2, dtype=torch.float64, device="cuda")
+    out = torch.full((nrows, n, n), -1.0, dtype=torch.float64, device="cuda")
+    assert _lib.load().pqb_mo_unpack_rows(_lib.ptr(ints), ints.numel(), n, row0, nrows, _lib.ptr(out),
+                                          _lib.stream_ptr()) == _lib.PQB_OK
+    k, l = np.indices((n, n))
+    KL = np.maximum(k, l) * (np.maximum(k, l) + 1) // 2 + np.minimum(k, l)
+    for r in range(nrows):
+        hi, lo = np.maximum(KL, row0 + r), np.minimum(KL, row0 + r)
+        assert np.array_equal(out[r].cpu().numpy(), hi * (hi + 1) // 2 + lo)
+
+
+@pytest.mark.parametrize("n,nb,nj,na", [(1, 1, 1, 1), (16, 1, 64, 8), (17, 3, 43, 9), (33, 2, 31, 64), (47, 5, 26, 65),
+                                        (30, 7, 11, 130)])
+def test_contract_pairs_at_tile_edges(n, nb, nj, na):
+    """Against the dense FP64 product: sums of n terms of order one (1e-13
+    leaves a hundred roundings)."""
+    g = torch.Generator().manual_seed(n)
+    P = n * (n + 1) // 2
+    Y = torch.randn(nb, P, nj, generator=g, dtype=torch.float64).cuda()
+    C = torch.randn(n, na, generator=g, dtype=torch.float64).cuda()
+    out = torch.empty(na, n, nb, nj, dtype=torch.float64, device="cuda")
+    assert _lib.load().pqb_mo_contract_pairs(_lib.ptr(Y), n, nb, nj, _lib.ptr(C), na, _lib.ptr(out),
+                                             _lib.stream_ptr()) == _lib.PQB_OK
+    i, j = torch.tril_indices(n, n, device="cuda")
+    full = torch.empty(nb, n, n, nj, dtype=torch.float64, device="cuda")
+    full[:, i, j] = Y
+    full[:, j, i] = Y
+    want = torch.einsum("ma,bmnj->anbj", C, full)
+    assert float((out - want).abs().max()) < 1e-13 * n * float(want.abs().max().clamp(min=1.0))
