@@ -235,8 +235,12 @@ int pqb_mp2_pairs(const double *V, int nocc, int nvirt, const double *e_occ, con
  *   adjustment a_jk (mu' = mu + a_jk (1 - mu^2)).
  * pqb_grid_amps: B[g*n + i] = amplitude of basis function i (the function
  *   table of pqb_oneint) at point g of pts[npts][4].
- * pqb_grid_rowdot: out[g] = sum_i A[g*n + i] B[g*n + i] (the density from
- *   B D and B).
+ * pqb_grid_rowdot: out[g] = sum_i A[g*n + i] B[g*n + i].
+ * pqb_grid_density: rho[g*stride + c] = sum_ij B[g*n + i] D[i*n + j] B[g*n + j]
+ *   for c < copies (copies <= stride).
+ * pqb_grid_fock: F[i*n + j] = sum_g B[g*n + i] v[g] B[g*n + j].
+ *   Both use work, 16-byte aligned device memory of pqb_grid_work(npts, n)
+ *   doubles.
  * pqb_xc_svwn: per point, Slater exchange plus VWN correlation of the spin
  *   densities rhoa, rhob, times the weight w: wf = w f_xc, wva = w v_a,
  *   wvb = w v_b. */
@@ -245,6 +249,10 @@ int pqb_becke_weights(int npts, const double *pts, const int *owner, int natoms,
 int pqb_grid_amps(int n, const double *origin, const int *powers, const int *prim_off, const double *exps,
                   const double *cn, const double *norms, int npts, const double *pts, double *B, void *stream);
 int pqb_grid_rowdot(int npts, int n, const double *A, const double *B, double *out, void *stream);
+int64_t pqb_grid_work(int npts, int n);
+int pqb_grid_density(int npts, int n, const double *B, const double *D, double *rho, int stride, int copies,
+                     double *work, void *stream);
+int pqb_grid_fock(int npts, int n, const double *B, const double *v, double *F, double *work, void *stream);
 int pqb_xc_svwn(int npts, const double *rhoa, const double *rhob, const double *w, double *wf, double *wva,
                 double *wvb, void *stream);
 

@@ -12,7 +12,8 @@ pyquante_b200.Lebedev).  Becke's cell weights (J. Chem. Phys. 88, 2547
 (1988), with the heteronuclear size adjustment of its appendix;
 PyQuante/MolecularGrid.py:228-263) come from pqb_becke_weights, the basis
 amplitudes on the points from pqb_grid_amps, the density from
-pqb_grid_rowdot -- all on the device.
+pqb_grid_density and a potential's matrix from pqb_grid_fock -- all on the
+device.
 """
 import numpy as np
 import torch
@@ -113,21 +114,39 @@ class MolecularGrid:
 
     set_bf_amps = add_basis
 
+    def _work(self):
+        return torch.empty(_lib.load().pqb_grid_work(self.ng, self.nbf), dtype=torch.float64, device=self.device)
+
     def set_density(self, D, Db=None):
         """density[:, 0] = sum_ij B_gi D_ij B_gj; density[:, 1] the same for
         Db (or a copy of the first column)."""
-        lib = _lib.load()
+        lib, n = _lib.load(), self.nbf
+        if self.bfgrid is None or tuple(self.bfgrid.shape) != (self.ng, n):
+            raise RuntimeError("set_density: no basis amplitudes on this grid (add_basis first)")
+        B, work = self.bfgrid.contiguous(), self._work()
         for col, M in ((0, D), (1, Db)):
             if M is None:
-                self.density[:, 1] = self.density[:, 0]
                 continue
             Mt = torch.as_tensor(np.asarray(M) if not isinstance(M, torch.Tensor) else M, dtype=torch.float64,
-                                 device=self.device)
-            BD = torch.matmul(self.bfgrid, Mt)
-            out = torch.empty(self.ng, dtype=torch.float64, device=self.device)
-            _check(lib.pqb_grid_rowdot(self.ng, self.nbf, ptr(BD), ptr(self.bfgrid), ptr(out), stream_ptr()),
-                   "pqb_grid_rowdot")
-            self.density[:, col] = out
+                                 device=self.device).contiguous()
+            if tuple(Mt.shape) != (n, n):
+                raise RuntimeError("set_density: the density is %s, the basis has %d functions" % (tuple(Mt.shape), n))
+            _check(lib.pqb_grid_density(self.ng, n, ptr(B), ptr(Mt), ptr(self.density[:, col:]), 2,
+                                        2 if col == 0 and Db is None else 1, ptr(work), stream_ptr()),
+                   "pqb_grid_density")
+
+    def fock(self, v):
+        """F_ij = sum_g B_gi v_g B_gj for a vector v over the points."""
+        B, v = self.bfgrid.contiguous(), v.contiguous()
+        n = self.nbf
+        if tuple(B.shape) != (self.ng, n) or tuple(v.shape) != (self.ng,):
+            raise RuntimeError("fock: amplitudes %s and values %s do not match the grid's %d points"
+                               % (tuple(B.shape), tuple(v.shape), self.ng))
+        F = torch.empty((n, n), dtype=torch.float64, device=self.device)
+        work = self._work()
+        _check(_lib.load().pqb_grid_fock(self.ng, n, ptr(B), ptr(v), ptr(F), ptr(work), stream_ptr()),
+               "pqb_grid_fock")
+        return F
 
     def setdens(self, D):
         self.set_density(D)

@@ -23,6 +23,15 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool o
                  : "memory");
 }
 
+// Up to two doubles, both addresses 16-byte aligned: the first `count` (0, 1
+// or 2) from src, zeros for the rest.
+__device__ __forceinline__ void cp_async16(double *dst, const double *src, int count)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(8 * count)
+                 : "memory");
+}
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 template <int N> __device__ __forceinline__ void cp_async_wait()

@@ -7,8 +7,8 @@ E = 2 tr(D h) + 2 tr(D J) + Exc + E_nuc with the spin-averaged density
 D = C_occ C_occ^T (+ half the open shells).
 
 The grid work runs on the GPU: basis amplitudes (pqb_grid_amps), the
-density (one DGEMM B D and pqb_grid_rowdot), the functional
-(pqb_xc_svwn) and Fxc = B^T diag(w v) B (one DGEMM).
+density (pqb_grid_density), the functional (pqb_xc_svwn) and
+Fxc = B^T diag(w v) B (pqb_grid_fock).
 """
 import logging
 
@@ -36,13 +36,16 @@ def getXC(gr, nel, **kwargs):
     if need_gradients.get(functional, True):
         raise NotImplementedError("gradient-corrected functionals are not built")
     gr.floor_density()
-    gr.renormalize(nel)
     w = gr.weights()
+    # (renormalize() with its factor kept on the GPU: the host waits once, for Exc)
+    total = torch.dot(w, gr.density.sum(1))
+    gr.density *= nel / total
     fxc, va, vb, _, _, _ = XC(gr.density.T, None, functional=functional)
-    exc = float(torch.dot(w, fxc))
-    wva = w * va
-    B = gr.bfgrid
-    Fxc = torch.matmul(B.T, B * wva[:, None])
+    exc = torch.dot(w, fxc)
+    Fxc = gr.fock(w * va)
+    exc, total = torch.stack([exc, total]).tolist()
+    if total == 0.0:
+        raise ZeroDivisionError("the density on the grid is zero")
     return exc, Fxc
 
 

@@ -13,7 +13,7 @@ import pyq_oracle as O
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from pyquante_b200 import Ints, geometries  # noqa: E402
+from pyquante_b200 import Ints, _lib, geometries  # noqa: E402
 from pyquante_b200.Basis.basis import BasisSet  # noqa: E402
 from pyquante_b200.DFunctionals import XC  # noqa: E402
 from pyquante_b200.dft import dft  # noqa: E402
@@ -97,3 +97,30 @@ def test_dft_water_dimer_vs_oracle():
     e_orc, _, _ = O.dft(at, S, h, O.orc_get2ints(obfs), obfs, 10)
     e_gpu, _, _ = dft(mol, bfs=bs, ConvCriteria=1e-10, MaxIter=80, direct=True)
     assert abs(e_gpu - e_orc) < 1e-8
+
+
+@pytest.mark.parametrize("skew", [0, 1])
+@pytest.mark.parametrize("npts,n", [(1, 1), (127, 7), (128, 32), (300, 33), (1000, 40), (257, 41), (515, 96), (131, 121),
+                                    (40000, 25), (3000, 310), (2049, 225), (900, 401)])
+def test_density_and_fock_tiles_at_their_edges(npts, n, skew):
+    """pqb_grid_density (an unsymmetric D among them) and pqb_grid_fock against
+    dense FP64 products: sums of n^2 and npts terms of order one, 1e-13 of
+    their sums of magnitudes leaving a hundred roundings.  skew: amplitudes that
+    start 8 bytes past a 16-byte boundary."""
+    g = torch.Generator().manual_seed(npts + n)
+    B = torch.randn(npts * n + skew, generator=g, dtype=torch.float64).cuda()[skew:].view(npts, n)
+    D = torch.randn(n, n, generator=g, dtype=torch.float64).cuda()
+    v = torch.randn(npts, generator=g, dtype=torch.float64).cuda()
+    lib, P, st = _lib.load(), _lib.ptr, _lib.stream_ptr()
+    work = torch.empty(lib.pqb_grid_work(npts, n), dtype=torch.float64, device="cuda")
+    rho = torch.full((npts, 3), -7.0, dtype=torch.float64, device="cuda")
+    assert lib.pqb_grid_density(npts, n, P(B), P(D), P(rho), 3, 2, P(work), st) == _lib.PQB_OK
+    want = ((B @ D) * B).sum(1)
+    tol = 1e-13 * float((B.abs() @ D.abs() * B.abs()).sum(1).max())
+    assert float((rho[:, 0] - want).abs().max()) <= tol and torch.equal(rho[:, 0], rho[:, 1])
+    assert bool((rho[:, 2] == -7.0).all())
+    F = torch.empty(n, n, dtype=torch.float64, device="cuda")
+    assert lib.pqb_grid_fock(npts, n, P(B), P(v), P(F), P(work), st) == _lib.PQB_OK
+    want = B.T @ (v[:, None] * B)
+    assert float((F - want).abs().max()) <= 1e-13 * float((B.abs().T @ (v.abs()[:, None] * B.abs())).max())
+    assert torch.equal(F, F.T)
