@@ -126,7 +126,8 @@ int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *c
 
 /* Tuning knobs (used by pyquante_b200.autotune): PQB_PARAM_CHUNK = the
  * largest number of primitive quartets in one J/K work item, for class
- * qclass (0..20, or -1 for all; effective at the next pqb_plan);
+ * qclass (0..20, or -1 for all; effective at the next pqb_plan, which cuts
+ * small bases' items shorter still);
  * PQB_PARAM_STREAMS = streams the class launches are spread over (1..16);
  * PQB_PARAM_ORDER = class launch order (0 by estimated cost, 1 highest
  * angular momentum first, the default); PQB_PARAM_PACKED_KERNEL = the

@@ -81,7 +81,8 @@ struct pqb_ctx {
     long long *d_mol_off = nullptr;
     int *d_mol_n = nullptr;
     int chunk[kNumQuartetClass];     // primitive-quartet chunk per class
-    int nstreams = 8;
+    int nstreams = 16;
+    bool small_plan = false;         // the current plan is one of a few molecules' latency (see plan_chunks)
     int order = 1;                   // class launch order: 0 by cost, 1 high angular momentum first
     // fork/join streams for concurrent class launches
     static constexpr int kStreams = 16;
@@ -1350,6 +1351,44 @@ int pqb_schwarz(pqb_ctx *ctx, double *Q_host, void *stream)
     }
 }
 
+// The chunk of each class for a plan of this basis.  The tuned chunks (32
+// primitive quartets an item) suit builds that fill the GPU; below that an
+// item's serial chain is the build's length (a (11|11) primitive quartet takes
+// 1.5 us), so the items are cut until a class gives about 4096 of them, to a
+// least length that grows with the basis's primitive quartets (each cut item
+// digests again).  Measured, FP64 build, 32 -> this rule: water / 6-31G** (0.06 M
+// primitive quartets) 84 -> 52 us, (H2O)3 / STO-3G (0.6 M) 71 -> 38, C2H6 / 6-31G*
+// (1.2 M) 92 -> 78, (H2O)3 / 6-31G** (4.3 M) 117 -> 104; C4H10 / 6-31G* (13 M) 212
+// -> 224 if it were cut to 4, so it is not.  Returns whether the mixed mode's
+// FP32-eligible lists are better merged into the FP64 launches too (below 9 M:
+// water dimer / 6-31G* 77 -> 58 us; (H2O)5 / 6-31G*, 23 M, 184 apart, 198 merged).
+static bool plan_chunks(const pqb_ctx *ctx, int *chunk)
+{
+    double u[kNumQuartetClass] = {0.0}, total = 0.0;
+    const auto &pairs = ctx->pairs;
+    for (size_t p0 = 0; p0 < pairs.size();) {
+        // one molecule's pairs
+        double s1[kNumPairClass] = {0.0}, s2[kNumPairClass] = {0.0};
+        size_t p = p0;
+        for (; p < pairs.size() && ctx->pair_first[p] == ctx->pair_first[p0]; ++p) {
+            const double n = pairs[p].nprim;
+            s1[pairs[p].cls] += n;
+            s2[pairs[p].cls] += n * n;
+        }
+        for (int cb = 0; cb < kNumPairClass; ++cb)
+            for (int ck = 0; ck <= cb; ++ck) {
+                const double x = cb == ck ? 0.5 * (s1[cb] * s1[cb] + s2[cb]) : s1[cb] * s1[ck];
+                u[quartet_class(cb, ck)] += x;
+                total += x;
+            }
+        p0 = p;
+    }
+    const int lo = (int)std::min(64.0, std::max(4.0, total / 0.75e6));
+    for (int c = 0; c < kNumQuartetClass; ++c)
+        chunk[c] = std::min(ctx->chunk[c], std::max(lo, (int)std::min(1024.0, u[c] / 4096.0)));
+    return total < 9e6;
+}
+
 int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *counts)
 {
     if (!ctx) return PQB_E_ARG;
@@ -1377,6 +1416,8 @@ int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *c
     };
     drop_graphs(ctx);
     ctx->have_plan = false;
+    int chunk[kNumQuartetClass];
+    ctx->small_plan = plan_chunks(ctx, chunk);
     std::vector<Range> rg;
     try {
         rg.resize(T);
@@ -1397,7 +1438,7 @@ int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *c
                 int4 e = oriented_quartet(pairs, p, q, qc);
                 const int part = b < fp32_thresh ? 1 : 0;
                 auto &dst = r.items[part][qc];
-                const int ch = ctx->chunk[qc];
+                const int ch = chunk[qc];
                 for (int s0 = 0; s0 < e.w; s0 += ch) dst.push_back(make_int4(e.x, e.y, s0, std::min(ch, e.w - s0)));
                 r.prims[part][qc] += e.w;
             }
@@ -1679,8 +1720,9 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
     }
     std::sort(order, order + 2 * kNumQuartetClass, [&](int x, int y) { return cost[x] > cost[y]; });
     // in an FP64 build both parts of a class are one list (the plan is
-    // class-major): one launch per class, over more items
-    const bool merged = mode != PQB_MIXED;
+    // class-major): one launch per class, over more items.  A small mixed build
+    // runs the same way: it is bound by launches and chains, not by arithmetic
+    const bool merged = mode != PQB_MIXED || ctx->small_plan;
     for (int i = 0, k = 0; i < 2 * kNumQuartetClass; ++i) {
         const int part = order[i] / kNumQuartetClass, c = order[i] % kNumQuartetClass;
         if (merged && part == 1) continue;
@@ -1688,7 +1730,7 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
         if (nq == 0) continue;
         cudaStream_t sk = ctx->streams[k++ % ctx->nstreams];
         const int4 *list = ctx->d_plan + ctx->plan_off[part][c];
-        const bool f32 = part == 1 && mode == PQB_MIXED;
+        const bool f32 = part == 1;
         if (jonly) {
             if (f32)
                 PQB_CK(ctx, launch_j_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Dsf[0], Jacc[0], sk, ctx->nsm,
