@@ -17,14 +17,14 @@
 //  * thread mode (NAB*NCD <= 81, which is every class with L <= 4): one
 //    thread per work item; the recurrence intermediates and all contracted
 //    components live in registers.
-//  * block mode (larger classes): a 256-thread block holds NSQ = 256/NAB
-//    quartets; per primitive quartet the roots (NSQ*NR tasks) and the 2-D
-//    integrals (NSQ*NR*3 tasks) go to shared memory, then every thread
-//    accumulates the NCD ket components of one bra component pair in
-//    registers.
+//  * warp mode (larger classes, FP64 in both precision modes): a warp holds
+//    32/NCD quartets, a lane per ket component pair; per primitive quartet the
+//    lanes share the roots and the 2-D integrals, which go to shared memory,
+//    then every lane accumulates the NAB bra components of its ket component
+//    pair in registers.
 //
-// The epilogue functor consumes the contracted integrals of one bra
-// component pair (ia, ib) for all ket components, so the same engine
+// The epilogue functor consumes a quartet's contracted integrals (thread
+// mode) or those of one ket component pair (warp mode), so the same engine
 // writes packed integrals, digests into J/K, or forms Schwarz bounds.
 #pragma once
 #include <atomic>
@@ -57,14 +57,9 @@ __device__ __forceinline__ int64_t fpair(int i, int j)
 //   thread_quartet<LA,LB,LC,LD>(q, acc[NAB*NCD], lane, live)
 //                                                  whole quartet, thread mode (all lanes
 //                                                  of the warp call it; live = a real item)
-//   kTile                                          false: block mode calls
-//     block_ab<LA,LB,LC,LD>(q, ia, ib, acc[NCD])     per bra component pair;
-//                                                  true: block mode stores the
-//     tile_store<LA,LB,LC,LD>(q, ia, ib, acc, V)     quartet's weighted integrals
-//     tile_reduce<LA,LB,LC,LD>(q, V, t, nt)          in a shared tile V and reduces
-//                                                    them after a block barrier
-
-__device__ __forceinline__ bool skip_bra(const QCtx &q, int fi, int fj) { return q.sa == q.sb && fi < fj; }
+//   lane_quartet<LA,LB,LC,LD>(q, ic, id, lane, live, acc[NAB], buf)
+//                                                  one ket component pair of a quartet,
+//                                                  warp mode (all lanes of the warp call it)
 
 // 1 if (x0, y0) > (x1, y1) lexicographically, 1/2 if equal, 0 if less.
 __host__ __device__ constexpr double lex_weight(int x0, int y0, int x1, int y1)
@@ -91,44 +86,125 @@ __device__ __forceinline__ double comp_weight(int ia, int ib, int ic, int id, bo
 }
 
 // Packed canonical integrals at ijkl2intindex (Src/cints.c:413-425), 64-bit.
+// Bound by the L2's rate of partial-sector writes (about 105 G sectors/s;
+// a row's neighbouring elements come from other classes' quartets, so a thread
+// owns only the run of consecutive elements that one shell gives): runs go out
+// 16 bytes at a time.  Which index runs is decided per quartet by the shells'
+// order, so the component loops hold no comparisons.  (H2O)6 / 6-31G** (N = 150,
+// 513 MB): 1.36 -> 1.01 ms a call, 107 -> 86 M sectors; the kernels one after the
+// other 2.20 -> 1.37 ms, of which the sharing of long items (kCoopLanes) took
+// (00|00), with items of 1,296 primitive quartets, from 0.34 to 0.08.
 struct EpiPacked {
     double *out;
     const double *fscale;
-    static constexpr bool kTile = false;
+    static constexpr bool kCoop = true;
     __device__ __forceinline__ bool screened(const PairInfo &, const PairInfo &, int, int) const { return false; }
-    template <int LC, int LD, typename R>
-    __device__ __forceinline__ void ab(const QCtx &q, int ia, int ib, const R *acc) const
+
+    // p[n] = x[n S] f[n] s, n < N, f the component scales of functions f0 ..
+    template <int N, int S, typename R>
+    __device__ __forceinline__ void run(double *p, const R *x, int f0, double s) const
     {
-        constexpr int NC = ncart(LC), ND = ncart(LD);
-        const int fi = q.fa + ia, fj = q.fb + ib;
-        if (skip_bra(q, fi, fj)) return;
-        const int64_t IJ = fpair(fi, fj);
-        const double sij = fscale[fi] * fscale[fj];
+        double v[N];
 #pragma unroll
-        for (int ic = 0; ic < NC; ++ic)
+        for (int n = 0; n < N; ++n) v[n] = (double)x[n * S] * (s * __ldg(fscale + f0 + n));
+        if constexpr (N == 1) {
+            p[0] = v[0];
+        } else if (reinterpret_cast<uintptr_t>(p) & 8) {
+            p[0] = v[0];
 #pragma unroll
-            for (int id = 0; id < ND; ++id) {
-                const int fk = q.fc + ic, fl = q.fd + id;
-                if (q.sc == q.sd && fk < fl) continue;
-                const int64_t KL = fpair(fk, fl);
-                if (q.bra == q.ket && IJ < KL) continue;
-                const int64_t hi = IJ > KL ? IJ : KL, lo = IJ > KL ? KL : IJ;
-                out[hi * (hi + 1) / 2 + lo] = (double)acc[ic * ND + id] * sij * fscale[fk] * fscale[fl];
-            }
+            for (int n = 1; n + 1 < N; n += 2) *reinterpret_cast<double2 *>(p + n) = make_double2(v[n], v[n + 1]);
+            if (N % 2 == 0) p[N - 1] = v[N - 1];
+        } else {
+#pragma unroll
+            for (int n = 0; n + 1 < N; n += 2) *reinterpret_cast<double2 *>(p + n) = make_double2(v[n], v[n + 1]);
+            if (N % 2 == 1) p[N - 1] = v[N - 1];
+        }
+    }
+    // the row of the packed array that starts at (IJ|0)
+    __device__ __forceinline__ double *row(int64_t IJ) const { return out + IJ * (IJ + 1) / 2; }
+    // bra and ket each of two shells, and no shell the highest of both: every
+    // component's canonical order is that of the shells
+    __device__ __forceinline__ static bool plain(const QCtx &q)
+    {
+        return q.sa != q.sb && q.sc != q.sd && max(q.fa, q.fb) != max(q.fc, q.fd);
+    }
+    // one component of any quartet, if canonical
+    __device__ __forceinline__ void one(const QCtx &q, int fi, int fj, int fk, int fl, double v) const
+    {
+        if ((q.sa == q.sb && fi < fj) || (q.sc == q.sd && fk < fl)) return;
+        const int64_t IJ = fpair(fi, fj), KL = fpair(fk, fl);
+        if (q.bra == q.ket && IJ < KL) return;
+        const double w = v * fscale[fi] * fscale[fj] * fscale[fk] * fscale[fl];
+        *(IJ > KL ? row(IJ) + KL : row(KL) + IJ) = w;
     }
     template <int LA, int LB, int LC, int LD, typename R>
-    __device__ __forceinline__ void thread_quartet(const QCtx &q, const R *acc, int lane, bool live) const
+    __device__ __forceinline__ void thread_quartet(const QCtx &q, const R *acc, int, bool live) const
     {
-        constexpr int NB = ncart(LB), NCD = ncart(LC) * ncart(LD);
-        (void)lane;
+        constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
         if (!live) return;
+        if (!plain(q)) {
 #pragma unroll
-        for (int ab = 0; ab < ncart(LA) * NB; ++ab) this->ab<LC, LD, R>(q, ab / NB, ab % NB, acc + ab * NCD);
+            for (int t = 0; t < NA * NB * NCD; ++t)
+                one(q, q.fa + t / NCD / NB, q.fb + t / NCD % NB, q.fc + t % NCD / ND, q.fd + t % ND, (double)acc[t]);
+        } else if (max(q.fa, q.fb) > max(q.fc, q.fd)) {
+#pragma unroll
+            for (int ab = 0; ab < NA * NB; ++ab) {
+                const int fi = q.fa + ab / NB, fj = q.fb + ab % NB;
+                double *r = row(fpair(fi, fj));
+                const double s = __ldg(fscale + fi) * __ldg(fscale + fj);
+                if (q.fc > q.fd) {
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        run<ND, 1>(r + fpair(q.fc + c, q.fd), acc + ab * NCD + c * ND, q.fd, s * __ldg(fscale + q.fc + c));
+                } else {
+#pragma unroll
+                    for (int d = 0; d < ND; ++d)
+                        run<NC, ND>(r + fpair(q.fd + d, q.fc), acc + ab * NCD + d, q.fc, s * __ldg(fscale + q.fd + d));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int cd = 0; cd < NCD; ++cd)
+                ket_row<NA, NB, NCD>(q, q.fc + cd / ND, q.fd + cd % ND, acc + cd);
+        }
     }
-    template <int LA, int LB, int LC, int LD, typename R>
-    __device__ __forceinline__ void block_ab(const QCtx &q, int ia, int ib, const R *acc) const
+    // row (fk, fl) of a plain quartet whose ket is the higher pair; x[ab * S]
+    template <int NA, int NB, int S, typename R>
+    __device__ __forceinline__ void ket_row(const QCtx &q, int fk, int fl, const R *x) const
     {
-        ab<LC, LD, R>(q, ia, ib, acc);
+        double *r = row(fpair(fk, fl));
+        const double s = __ldg(fscale + fk) * __ldg(fscale + fl);
+        if (q.fa > q.fb) {
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+                run<NB, S>(r + fpair(q.fa + a, q.fb), x + a * NB * S, q.fb, s * __ldg(fscale + q.fa + a));
+        } else {
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+                run<NA, NB * S>(r + fpair(q.fb + b, q.fa), x + b * S, q.fa, s * __ldg(fscale + q.fb + b));
+        }
+    }
+    template <int LA, int LB, int LC, int LD, int NCW>
+    __device__ __forceinline__ void lane_quartet(const QCtx &q, int ic, int id, int, bool live, double *acc, double *) const
+    {
+        constexpr int NA = ncart(LA), NB = ncart(LB);
+        const int fk = q.fc + ic, fl = q.fd + id;
+        if (!live) return;
+        if (!plain(q)) {
+#pragma unroll
+            for (int ab = 0; ab < NA * NB; ++ab) one(q, q.fa + ab / NB, q.fb + ab % NB, fk, fl, acc[ab]);
+        } else if (max(q.fa, q.fb) > max(q.fc, q.fd)) {
+            // neighbouring lanes hold neighbouring elements
+            const int64_t KL = fpair(fk, fl);
+            const double skl = __ldg(fscale + fk) * __ldg(fscale + fl);
+#pragma unroll
+            for (int ab = 0; ab < NA * NB; ++ab) {
+                const int fi = q.fa + ab / NB, fj = q.fb + ab % NB;
+                row(fpair(fi, fj))[KL] = acc[ab] * (skl * __ldg(fscale + fi) * __ldg(fscale + fj));
+            }
+        } else {
+            ket_row<NA, NB, 1>(q, fk, fl, acc);
+        }
     }
 };
 
@@ -139,30 +215,29 @@ struct EpiPacked {
 // of the warp must take part.
 struct WarpRuns {
     unsigned f;   // bit s: lane - 2^s lies in this lane's run
+    int steps;    // scan steps that reach the longest run of the warp
     bool last;    // last lane of its run
-    __device__ __forceinline__ WarpRuns(long long key, int lane)
+    __device__ __forceinline__ WarpRuns(int key_hi, int key_lo, int lane)
     {
         // a run is a maximal block of consecutive lanes with one key (the
-        // same key may come back later in the warp as another run): first
-        // the lane where this lane's run starts (max-scan of run heads)
-        const long long kp = __shfl_up_sync(0xffffffffu, key, 1);
-        int start = (lane == 0 || kp != key) ? lane : 0;
-#pragma unroll
-        for (int s = 0; s < 5; ++s) {
-            const int o = __shfl_up_sync(0xffffffffu, start, 1 << s);
-            if (lane >= (1 << s) && o > start) start = o;
-        }
+        // same key may come back later in the warp as another run): the run
+        // heads of the warp as one ballot
+        const int ph = __shfl_up_sync(0xffffffffu, key_hi, 1), pl = __shfl_up_sync(0xffffffffu, key_lo, 1);
+        const bool head = lane == 0 || ph != key_hi || pl != key_lo;
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        const int back = __clz((heads << (31 - lane)));   // lanes since this lane's head
         f = 0;
 #pragma unroll
         for (int s = 0; s < 5; ++s)
-            if (lane - (1 << s) >= start) f |= 1u << s;
-        const long long kn = __shfl_down_sync(0xffffffffu, key, 1);
-        last = lane == 31 || kn != key;
+            if (back >= (1 << s)) f |= 1u << s;
+        steps = 32 - __clz((int)__reduce_max_sync(0xffffffffu, (unsigned)back));
+        last = lane == 31 || ((heads >> ((lane + 1) & 31)) & 1u);
     }
     template <typename V> __device__ __forceinline__ V sum(V x) const
     {
 #pragma unroll
         for (int s = 0; s < 5; ++s) {
+            if (s >= steps) break;   // uniform over the warp
             const V y = __shfl_up_sync(0xffffffffu, x, 1 << s);
             if ((f >> s) & 1u) x += y;
         }
@@ -215,9 +290,8 @@ __device__ __forceinline__ V warp_sum_transposed(const V *v, int lane, int &idx)
 //
 // Thread mode: the quartet's six D blocks are loaded once, the six J/K
 // blocks (ab, cd, ac, ad, bc, bd) are summed in registers, and each block
-// element goes to global memory with one atomic.  Block mode: the weighted
-// integrals go to a shared tile; each output element is then one thread's
-// reduction over the tile (no shared-memory atomics).  With NDEN = 2 both
+// element goes to global memory with one atomic.  Warp mode: see
+// lane_quartet.  With NDEN = 2 both
 // densities are digested from the same integrals (UHF); WITHK = false keeps
 // the Coulomb terms alone.
 template <int NDEN, bool WITHK = true>
@@ -226,7 +300,7 @@ struct EpiJKn {
     double *Jacc[NDEN], *Kacc[NDEN];
     const float *Df[NDEN];        // their single-precision copies (FP32 lists of the mixed mode), or null
     ItemScreen scr;               // items skipped by molecule mask or density bound (all fields optional)
-    static constexpr bool kTile = true;
+    static constexpr bool kCoop = false;   // (its items are cut short by the plan instead)
     __device__ __forceinline__ bool screened(const PairInfo &pb, const PairInfo &pk, int bra, int ket) const
     {
         if (scr.molmask && __ldg(scr.molmask + pb.mol) == 0) return true;
@@ -244,15 +318,32 @@ struct EpiJKn {
     // list's precision R (FP32 lists read the single-precision density); the
     // accumulation into Jacc/Kacc is FP64.
     template <int LA, int LB, int LC, int LD, typename R>
-    __device__ __forceinline__ void thread_quartet(const QCtx &q, const R *acc, int lane, bool) const
+    __device__ __forceinline__ void thread_quartet(const QCtx &q, R *acc, int lane, bool) const
     {
         using T = R;
         constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
-        const bool bd = q.sa == q.sb, kd = q.sc == q.sd, qd = q.bra == q.ket, af = q.fa > q.fb;
+        // degeneracy weights, applied once; shells of unlike angular momentum, or
+        // bra and ket of unlike classes, are never the same, and most warps hold no
+        // such quartet at all
+        if constexpr (LA == LB || LC == LD || (LA == LC && LB == LD)) {
+            const bool bd = LA == LB && q.sa == q.sb, kd = LC == LD && q.sc == q.sd,
+                       qd = LA == LC && LB == LD && q.bra == q.ket, af = q.fa > q.fb;
+            if (bd || kd || qd) {
+#pragma unroll
+                for (int a = 0; a < NA; ++a)
+#pragma unroll
+                    for (int b = 0; b < NB; ++b)
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+#pragma unroll
+                            for (int d = 0; d < ND; ++d)
+                                acc[(a * NB + b) * NCD + c * ND + d] *= (T)comp_weight(a, b, c, d, bd, kd, qd, af);
+            }
+        }
         // Jacc[a,b] is shared by lanes with the same bra pair; Kacc[a,c] and
         // Kacc[b,c] by lanes that also share the ket's first shell (the bra
         // runs are scanned only for warps of more than one bra pair)
-        const WarpRuns rbc(((long long)q.bra << 32) | (unsigned)q.sc, lane);
+        const WarpRuns rbc(q.bra, q.sc, lane);
         // (the shuffle is taken by every lane, outside any condition)
         const int bra0 = __shfl_sync(0xffffffffu, q.bra, 0);
         const bool one_bra = __all_sync(0xffffffffu, bra0 == q.bra);
@@ -265,8 +356,11 @@ struct EpiJKn {
         else
             Db = D[s] + q.bo;
         double *Jb = Jacc[s] + q.bo, *Kb = Kacc[s] + q.bo;
-        const int64_t nm = q.nm;
-        const T *Da = Db + q.fa * nm, *Dbr = Db + q.fb * nm, *Dc = Db + q.fc * nm;
+        // row bases in 64 bits, offsets within the few rows of a shell in 32
+        const int nm = q.nm;
+        const int64_t oa = (int64_t)q.fa * nm, ob = (int64_t)q.fb * nm, oc = (int64_t)q.fc * nm;
+        const T *Da = Db + oa, *Dbr = Db + ob, *Dc = Db + oc;
+        double *Ja = Jb + oa, *Jc = Jb + oc, *Ka = Kb + oa, *Kbr = Kb + ob;
         // Coulomb: Jacc[a,b] and Jacc[c,d]
         {
             T dab[NA][NB], dcd[NC][ND], jcd[NC][ND];
@@ -291,8 +385,7 @@ struct EpiJKn {
                     for (int c = 0; c < NC; ++c)
 #pragma unroll
                         for (int d = 0; d < ND; ++d) {
-                            const T v = (T)acc[(a * NB + b) * NCD + c * ND + d] *
-                                        (T)comp_weight(a, b, c, d, bd, kd, qd, af);
+                            const T v = acc[(a * NB + b) * NCD + c * ND + d];
                             jab = fma(v, dcd[c][d], jab);
                             jcd[c][d] = fma(v, dab[a][b], jcd[c][d]);
                         }
@@ -304,20 +397,20 @@ struct EpiJKn {
                 const double js = (double)warp_sum_transposed<(NA * NB <= 32 ? NA * NB : 1)>(jabv, lane, idx);
                 constexpr int KP = NA * NB <= 1 ? 1 : NA * NB <= 2 ? 2 : NA * NB <= 4 ? 4 : NA * NB <= 8 ? 8 : NA * NB <= 16 ? 16 : 32;
                 if (idx < NA * NB && (lane & (32 / KP - 1)) == 0 && js != 0.0)
-                    atomicAdd(Jb + (q.fa + idx / NB) * nm + q.fb + idx % NB, 2.0 * js);
+                    atomicAdd(Ja + idx / NB * nm + q.fb + idx % NB, 2.0 * js);
             } else {
-                const WarpRuns rb((long long)q.bra, lane);
+                const WarpRuns rb(q.bra, 0, lane);
 #pragma unroll
                 for (int ab = 0; ab < NA * NB; ++ab) {
                     const double js = (double)rb.sum(jabv[ab]);
-                    if (rb.last && js != 0.0) atomicAdd(Jb + (q.fa + ab / NB) * nm + q.fb + ab % NB, 2.0 * js);
+                    if (rb.last && js != 0.0) atomicAdd(Ja + ab / NB * nm + q.fb + ab % NB, 2.0 * js);
                 }
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c)
 #pragma unroll
                 for (int d = 0; d < ND; ++d)
-                    if (jcd[c][d] != (T)0) atomicAdd(Jb + (q.fc + c) * nm + q.fd + d, 2.0 * (double)jcd[c][d]);
+                    if (jcd[c][d] != (T)0) atomicAdd(Jc + c * nm + q.fd + d, 2.0 * (double)jcd[c][d]);
         }
         if constexpr (!WITHK) continue;   // Coulomb only
         // exchange rows of the bra's first shell: Kacc[a,c] += v D_bd, Kacc[a,d] += v D_bc
@@ -343,19 +436,18 @@ struct EpiJKn {
                     for (int c = 0; c < NC; ++c)
 #pragma unroll
                         for (int d = 0; d < ND; ++d) {
-                            const T v = (T)acc[(a * NB + b) * NCD + c * ND + d] *
-                                        (T)comp_weight(a, b, c, d, bd, kd, qd, af);
+                            const T v = acc[(a * NB + b) * NCD + c * ND + d];
                             kac[c] = fma(v, dbd[b][d], kac[c]);
                             kad[d] = fma(v, dbc[b][c], kad[d]);
                         }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const double ks = (double)rbc.sum(kac[c]);
-                    if (rbc.last && ks != 0.0) atomicAdd(Kb + (q.fa + a) * nm + q.fc + c, ks);
+                    if (rbc.last && ks != 0.0) atomicAdd(Ka + a * nm + q.fc + c, ks);
                 }
 #pragma unroll
                 for (int d = 0; d < ND; ++d)
-                    if (kad[d] != (T)0) atomicAdd(Kb + (q.fa + a) * nm + q.fd + d, (double)kad[d]);
+                    if (kad[d] != (T)0) atomicAdd(Ka + a * nm + q.fd + d, (double)kad[d]);
             }
         }
         // exchange rows of the bra's second shell: Kacc[b,c] += v D_ad, Kacc[b,d] += v D_ac
@@ -381,112 +473,133 @@ struct EpiJKn {
                     for (int c = 0; c < NC; ++c)
 #pragma unroll
                         for (int d = 0; d < ND; ++d) {
-                            const T v = (T)acc[(a * NB + b) * NCD + c * ND + d] *
-                                        (T)comp_weight(a, b, c, d, bd, kd, qd, af);
+                            const T v = acc[(a * NB + b) * NCD + c * ND + d];
                             kbc[c] = fma(v, dad[a][d], kbc[c]);
                             kbd[d] = fma(v, dac[a][c], kbd[d]);
                         }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const double ks = (double)rbc.sum(kbc[c]);
-                    if (rbc.last && ks != 0.0) atomicAdd(Kb + (q.fb + b) * nm + q.fc + c, ks);
+                    if (rbc.last && ks != 0.0) atomicAdd(Kbr + b * nm + q.fc + c, ks);
                 }
 #pragma unroll
                 for (int d = 0; d < ND; ++d)
-                    if (kbd[d] != (T)0) atomicAdd(Kb + (q.fb + b) * nm + q.fd + d, (double)kbd[d]);
+                    if (kbd[d] != (T)0) atomicAdd(Kbr + b * nm + q.fd + d, (double)kbd[d]);
             }
         }
         }
     }
 
-    // block mode: the tile row of bra component (ia, ib) holds its NCD
-    // weighted integrals (row stride NCD + 1 spreads the rows over the banks)
-    template <int LA, int LB, int LC, int LD>
-    static constexpr int kTileStride = ncart(LC) * ncart(LD) + 1;
-
-    template <int LA, int LB, int LC, int LD, typename R>
-    __device__ __forceinline__ void tile_store(const QCtx &q, int ia, int ib, const R *acc, double *V) const
+    // Warp mode: a lane holds the NAB integrals of one ket component pair
+    // (c, d); a slot's lanes are consecutive, d fastest.  Every output's part is
+    // summed in the lane first, then over the slot's d or its NCW c lanes by
+    // shuffles (Kacc), or over all of them through buf (Jacc[a,b]; NAB x 33
+    // doubles of the warp's shared memory).  Lanes without a live quartet carry
+    // zeros.
+    template <int N> static __device__ __forceinline__ double strided_sum(double x, int stride)
     {
-        constexpr int NC = ncart(LC), ND = ncart(LD), NB = ncart(LB);
-        constexpr int ST = kTileStride<LA, LB, LC, LD>;
-        const bool bd = q.sa == q.sb, kd = q.sc == q.sd, qd = q.bra == q.ket, af = q.fa > q.fb;
-        const int64_t nm = q.nm;
-        // runtime bra indices: the bra and quartet factors of comp_weight in closed form
-        const double wb = bd ? (ia > ib ? 1.0 : (ia == ib ? 0.5 : 0.0)) : 1.0;
-        const int x0 = (bd || af) ? ia : ib, y0 = (bd || af) ? ib : ia;
-        double jab[NDEN];
-#pragma unroll
-        for (int s = 0; s < NDEN; ++s) jab[s] = 0.0;
-        double *row = V + (ia * NB + ib) * ST;
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-#pragma unroll
-            for (int d = 0; d < ND; ++d) {
-                const double wk = kd ? (c > d ? 1.0 : (c == d ? 0.5 : 0.0)) : 1.0;
-                const int x1 = (bd || af) ? c : d, y1 = (bd || af) ? d : c;
-                const double wq = qd ? (x0 != x1 ? (x0 > x1 ? 1.0 : 0.0) : (y0 != y1 ? (y0 > y1 ? 1.0 : 0.0) : 0.5))
-                                     : 1.0;
-                const double v = (double)acc[c * ND + d] * (wb * wk * wq);
-#pragma unroll
-                for (int s = 0; s < NDEN; ++s) jab[s] = fma(v, __ldg(D[s] + q.bo + (q.fc + c) * nm + q.fd + d), jab[s]);
-                row[c * ND + d] = v;
-            }
-#pragma unroll
-        for (int s = 0; s < NDEN; ++s)
-            if (jab[s] != 0.0) atomicAdd(Jacc[s] + q.bo + (q.fa + ia) * nm + q.fb + ib, 2.0 * jab[s]);
+        // the sum over N lanes (N = 1, 3 or 6) at the given stride, valid in the first
+        static_assert(N == 1 || N == 3 || N == 6, "cartesian components of s, p, d");
+        if constexpr (N == 6) x += __shfl_down_sync(0xffffffffu, x, 3 * stride);
+        if constexpr (N > 1) {
+            const double y = __shfl_down_sync(0xffffffffu, x, stride), z = __shfl_down_sync(0xffffffffu, x, 2 * stride);
+            x += y + z;
+        }
+        return x;
     }
 
-    // outputs of one quartet: Jacc[c,d] (NCD), Kacc[a,c], Kacc[a,d],
-    // Kacc[b,c], Kacc[b,d]; threads t, t + nt, ... of the quartet's slot
-    template <int LA, int LB, int LC, int LD>
-    __device__ __forceinline__ void tile_reduce(const QCtx &q, const double *V, int t, int nt) const
+    template <int LA, int LB, int LC, int LD, int NCW>
+    __device__ __forceinline__ void lane_quartet(const QCtx &q, int c, int d, int lane, bool live, double *acc,
+                                                 double *buf) const
     {
-        constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
-        constexpr int ST = kTileStride<LA, LB, LC, LD>;
-        constexpr int O1 = NCD, O2 = O1 + NA * NC, O3 = O2 + NA * ND, O4 = O3 + NB * NC,
-                      O5 = WITHK ? O4 + NB * ND : O1;
-        const int64_t nm = q.nm;
+        constexpr int NA = ncart(LA), NB = ncart(LB), ND = ncart(LD), NAB = NA * NB, W = NCW * ND;
+        const bool c_first = c % NCW == 0;
+        if constexpr (LA == LB || LC == LD || (LA == LC && LB == LD)) {
+            const bool bd = LA == LB && q.sa == q.sb, kd = LC == LD && q.sc == q.sd,
+                       qd = LA == LC && LB == LD && q.bra == q.ket, af = q.fa > q.fb;
+            if (bd || kd || qd) {
 #pragma unroll
-        for (int sd = 0; sd < NDEN; ++sd) {
-        const double *Db = D[sd] + q.bo;
-        double *Jo = Jacc[sd], *Ko = Kacc[sd];
-        for (int o = t; o < O5; o += nt) {
-            double s = 0.0;
-            double *dst;
-            if (o < O1) {                     // Jacc[c,d] = 2 sum_ab v D_ab
-                const int c = o / ND, d = o - (o / ND) * ND;
-                for (int a = 0; a < NA; ++a)
-                    for (int b = 0; b < NB; ++b)
-                        s = fma(V[(a * NB + b) * ST + c * ND + d], __ldg(Db + (q.fa + a) * nm + q.fb + b), s);
-                s *= 2.0;
-                dst = Jo + q.bo + (q.fc + c) * nm + q.fd + d;
-            } else if (o < O2) {              // Kacc[a,c] = sum_bd v D_bd
-                const int a = (o - O1) / NC, c = (o - O1) - ((o - O1) / NC) * NC;
-                for (int b = 0; b < NB; ++b)
-                    for (int d = 0; d < ND; ++d)
-                        s = fma(V[(a * NB + b) * ST + c * ND + d], __ldg(Db + (q.fb + b) * nm + q.fd + d), s);
-                dst = Ko + q.bo + (q.fa + a) * nm + q.fc + c;
-            } else if (o < O3) {              // Kacc[a,d] = sum_bc v D_bc
-                const int a = (o - O2) / ND, d = (o - O2) - ((o - O2) / ND) * ND;
-                for (int b = 0; b < NB; ++b)
-                    for (int c = 0; c < NC; ++c)
-                        s = fma(V[(a * NB + b) * ST + c * ND + d], __ldg(Db + (q.fb + b) * nm + q.fc + c), s);
-                dst = Ko + q.bo + (q.fa + a) * nm + q.fd + d;
-            } else if (o < O4) {              // Kacc[b,c] = sum_ad v D_ad
-                const int b = (o - O3) / NC, c = (o - O3) - ((o - O3) / NC) * NC;
-                for (int a = 0; a < NA; ++a)
-                    for (int d = 0; d < ND; ++d)
-                        s = fma(V[(a * NB + b) * ST + c * ND + d], __ldg(Db + (q.fa + a) * nm + q.fd + d), s);
-                dst = Ko + q.bo + (q.fb + b) * nm + q.fc + c;
-            } else {                          // Kacc[b,d] = sum_ac v D_ac
-                const int b = (o - O4) / ND, d = (o - O4) - ((o - O4) / ND) * ND;
-                for (int a = 0; a < NA; ++a)
-                    for (int c = 0; c < NC; ++c)
-                        s = fma(V[(a * NB + b) * ST + c * ND + d], __ldg(Db + (q.fa + a) * nm + q.fc + c), s);
-                dst = Ko + q.bo + (q.fb + b) * nm + q.fd + d;
+                for (int ab = 0; ab < NAB; ++ab) acc[ab] *= comp_weight(ab / NB, ab % NB, c, d, bd, kd, qd, af);
             }
-            if (s != 0.0) atomicAdd(dst, s);
         }
+        if (!live) {
+#pragma unroll
+            for (int ab = 0; ab < NAB; ++ab) acc[ab] = 0.0;
+        }
+        const int nm = q.nm;
+        const int64_t oa = (int64_t)q.fa * nm, ob = (int64_t)q.fb * nm, oc = (int64_t)(q.fc + c) * nm;
+#pragma unroll
+        for (int s = 0; s < NDEN; ++s) {
+            const double *Db = D[s] + q.bo;
+            const double *Da = Db + oa, *Dbr = Db + ob;
+            double *Jb = Jacc[s] + q.bo;
+            // Jacc[c,d] in the lane, Jacc[a,b] over the slot
+            {
+                const double dcd = __ldg(Db + oc + q.fd + d);
+                double jcd = 0.0;
+#pragma unroll
+                for (int ab = 0; ab < NAB; ++ab) {
+                    jcd = fma(acc[ab], __ldg(Da + ab / NB * nm + q.fb + ab % NB), jcd);
+                    buf[ab * 33 + lane] = acc[ab] * dcd;
+                }
+                if (live && jcd != 0.0) atomicAdd(Jb + oc + q.fd + d, 2.0 * jcd);
+                __syncwarp();
+                // the slot's lanes step through its NAB sums
+                if (live) {
+                    const int l0 = lane / W * W;
+                    for (int ab = lane - l0; ab < NAB; ab += W) {
+                        double x = 0.0;
+#pragma unroll
+                        for (int k = 0; k < W; ++k) x += buf[ab * 33 + l0 + k];
+                        if (x != 0.0) atomicAdd(Jb + oa + ab / NB * nm + q.fb + ab % NB, 2.0 * x);
+                    }
+                }
+                __syncwarp();
+            }
+            if constexpr (!WITHK) continue;   // Coulomb only
+            double *Ka = Kacc[s] + q.bo + oa, *Kbr = Kacc[s] + q.bo + ob;
+            {
+                double dbd[NB], dbc[NB];
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    dbd[b] = __ldg(Dbr + b * nm + q.fd + d);
+                    dbc[b] = __ldg(Dbr + b * nm + q.fc + c);
+                }
+#pragma unroll
+                for (int a = 0; a < NA; ++a) {
+                    double kac = 0.0, kad = 0.0;
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        kac = fma(acc[a * NB + b], dbd[b], kac);
+                        kad = fma(acc[a * NB + b], dbc[b], kad);
+                    }
+                    kac = strided_sum<ND>(kac, 1);
+                    kad = strided_sum<NCW>(kad, ND);
+                    if (live && d == 0 && kac != 0.0) atomicAdd(Ka + a * nm + q.fc + c, kac);
+                    if (live && c_first && kad != 0.0) atomicAdd(Ka + a * nm + q.fd + d, kad);
+                }
+            }
+            {
+                double dad[NA], dac[NA];
+#pragma unroll
+                for (int a = 0; a < NA; ++a) {
+                    dad[a] = __ldg(Da + a * nm + q.fd + d);
+                    dac[a] = __ldg(Da + a * nm + q.fc + c);
+                }
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    double kbc = 0.0, kbd = 0.0;
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) {
+                        kbc = fma(acc[a * NB + b], dad[a], kbc);
+                        kbd = fma(acc[a * NB + b], dac[a], kbd);
+                    }
+                    kbc = strided_sum<ND>(kbc, 1);
+                    kbd = strided_sum<NCW>(kbd, ND);
+                    if (live && d == 0 && kbc != 0.0) atomicAdd(Kbr + b * nm + q.fc + c, kbc);
+                    if (live && c_first && kbd != 0.0) atomicAdd(Kbr + b * nm + q.fd + d, kbd);
+                }
+            }
         }
     }
 };
@@ -504,7 +617,7 @@ using EpiJ = EpiJKn<1, false>;
 struct EpiSchwarz {
     unsigned long long *Q2bits;   // bit patterns of non-negative doubles
     const double *fscale;
-    static constexpr bool kTile = false;
+    static constexpr bool kCoop = true;
     __device__ __forceinline__ bool screened(const PairInfo &, const PairInfo &, int, int) const { return false; }
     template <int LC, int LD, typename R>
     __device__ __forceinline__ void ab(const QCtx &q, int ia, int ib, const R *acc) const
@@ -528,10 +641,19 @@ struct EpiSchwarz {
 #pragma unroll
         for (int ab = 0; ab < ncart(LA) * NB; ++ab) this->ab<LC, LD, R>(q, ab / NB, ab % NB, acc + ab * NCD);
     }
-    template <int LA, int LB, int LC, int LD, typename R>
-    __device__ __forceinline__ void block_ab(const QCtx &q, int ia, int ib, const R *acc) const
+    template <int LA, int LB, int LC, int LD, int NCW>
+    __device__ __forceinline__ void lane_quartet(const QCtx &q, int ic, int id, int, bool live, double *acc, double *) const
     {
-        ab<LC, LD, R>(q, ia, ib, acc);
+        // (ia, ib) == (ic, id) on a diagonal quartet
+        constexpr int ND = ncart(LD);
+        if (!live) return;
+        double v = 0.0;
+#pragma unroll
+        for (int ab = 0; ab < ncart(LA) * ncart(LB); ++ab)
+            if (ab == ic * ND + id) v = acc[ab];
+        const double s = fscale[q.fc + ic] * fscale[q.fd + id];
+        v = fabs(v) * s * s;
+        atomicMax(Q2bits + q.bra, (unsigned long long)__double_as_longlong(v));
     }
 };
 
@@ -570,55 +692,11 @@ __host__ __device__ constexpr int thread_min_blocks(int nabcd)
     return nabcd == 1 ? 8 : (nabcd <= 3 ? 6 : (nabcd <= 9 ? 5 : (nabcd == 27 ? 3 : 2)));
 }
 
-// Single-precision counterpart of add_prim_quartet for the FP32 lists of
-// the mixed mode: geometry, roots (rys_roots_f32), 2-D tables and assembly
-// all in FP32; only large-T root forms are evaluated in FP64.
 struct QuartetGeomF {
     float A[3], C[3], AB[3], CD[3];
 };
 
-template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void add_prim_quartet_f32(const QuartetGeomF &g, const float *P, const float *Q, float *acc)
-{
-    constexpr int NB = ncart(LB), ND = ncart(LD);
-    constexpr int NAB = ncart(LA) * NB, NCD = ncart(LC) * ND;
-    constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
-    constexpr int G2D = (LA + 1) * (LB + 1) * (LC + 1) * (LD + 1);
-    // P, Q: zeta, 1/zeta, P[3], K
-    const float zeta = P[0], eta = Q[0];
-    const float PQ[3] = {P[2] - Q[2], P[3] - Q[3], P[4] - Q[4]};
-    const float rs = rsqrtf(zeta + eta), izpe = rs * rs;
-    const float T = zeta * eta * izpe * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-    const float pre = P[5] * Q[5] * rs;
-    float uu[NR], ww[NR];
-    rys_roots_f32<NR>(T, uu, ww);
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        const float ue = uu[r] * izpe, ce = eta * ue, cz = zeta * ue;
-        const float b00 = 0.5f * ue, b10 = 0.5f * P[1] * (1.0f - ce), b01 = 0.5f * Q[1] * (1.0f - cz);
-        float gx[G2D], gy[G2D], gz[G2D];
-        float *gt[3] = {gx, gy, gz};
-#pragma unroll
-        for (int x = 0; x < 3; ++x)
-            rys2d_f<LA, LB, LC, LD>(b00, b10, b01, fmaf(-ce, PQ[x], P[2 + x] - g.A[x]), fmaf(cz, PQ[x], Q[2 + x] - g.C[x]),
-                                    g.AB[x], g.CD[x], x == 0 ? ww[r] * pre : 1.0f, gt[x]);
-#pragma unroll
-        for (int ab = 0; ab < NAB; ++ab)
-#pragma unroll
-            for (int cd = 0; cd < NCD; ++cd) {
-                const int ia = ab / NB, ib = ab % NB, ic = cd / ND, id = cd % ND;
-                const int ox = ((cart_lx(LA, ia) * (LB + 1) + cart_lx(LB, ib)) * (LC + 1) + cart_lx(LC, ic)) * (LD + 1) +
-                               cart_lx(LD, id);
-                const int oy = ((cart_ly(LA, ia) * (LB + 1) + cart_ly(LB, ib)) * (LC + 1) + cart_ly(LC, ic)) * (LD + 1) +
-                               cart_ly(LD, id);
-                const int oz = ((cart_lz(LA, ia) * (LB + 1) + cart_lz(LB, ib)) * (LC + 1) + cart_lz(LC, ic)) * (LD + 1) +
-                               cart_lz(LD, id);
-                acc[ab * NCD + cd] = fmaf(gx[ox] * gy[oy], gz[oz], acc[ab * NCD + cd]);
-            }
-    }
-}
-
-// The same for the Obara--Saika classes: F_m(T) and the vertical
+// FP32 lists of the mixed mode: geometry, F_m(T) and the vertical
 // recurrence in single precision, accumulated into the contracted [e0|f0].
 template <int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void os_prim_quartet_f32(const QuartetGeomF &g, const float *P, const float *Q, float *v)
@@ -650,7 +728,10 @@ __device__ __forceinline__ void os_prim_quartet_f32(const QuartetGeomF &g, const
     OsClass<LA, LB, LC, LD>::template vrr<float>(o, F, v);
 }
 
-template <int LA, int LB, int LC, int LD, typename R, class Epi>
+// G lanes share an item (1, or kCoopLanes for the long items of whole
+// quartets), each every G-th primitive quartet; the contracted [e0|f0] are
+// added over them, and the first lane has the item's epilogue.
+template <int LA, int LB, int LC, int LD, typename R, class Epi, int G = 1>
 __global__ void __launch_bounds__(128, thread_min_blocks(ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)))
 eri_thread_kernel(const int4 *__restrict__ list, int nq,
                                                          const PairInfo *__restrict__ pairs,
@@ -658,14 +739,14 @@ eri_thread_kernel(const int4 *__restrict__ list, int nq,
 {
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     constexpr int NAB = NA * NB, NCD = NC * ND;
-    constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
-    constexpr int G2D = (LA + 1) * (LB + 1) * (LC + 1) * (LD + 1);
+    using OS = OsClass<LA, LB, LC, LD>;
+    static_assert(OS::kOn, "thread mode has the Obara--Saika classes only");
     // whole warps step through the list together (the J/K epilogue reduces
     // over the lanes); a lane past the end repeats the last item with no
     // primitive quartets
     const int lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < nq; base += gridDim.x * blockDim.x) {
-        const int qi = base + lane;
+    for (int base = (blockIdx.x * blockDim.x + threadIdx.x - lane) / G; base < nq; base += gridDim.x * blockDim.x / G) {
+        const int qi = base + lane / G;
         const bool live = qi < nq;
         int4 e = list[live ? qi : nq - 1];   // bra pair, ket pair, first primitive quartet, count
         if (!live) e.w = 0;
@@ -704,7 +785,6 @@ eri_thread_kernel(const int4 *__restrict__ list, int nq,
             float Pn[8], Q[8];
             ld8f(pbp[ib].f, Pn);
             ld8f(pkp[ik].f, Q);
-            using OS = OsClass<LA, LB, LC, LD>;
             float v[OS::NV];
 #pragma unroll
             for (int c = 0; c < OS::NV; ++c) v[c] = 0.0f;
@@ -720,10 +800,7 @@ eri_thread_kernel(const int4 *__restrict__ list, int nq,
                 if (t + 1 < e.w) ld8f(pbp[ib2].f, Pn);
                 float Qn[8];
                 if (ik2 != ik && t + 1 < e.w) ld8f(pkp[ik2].f, Qn);
-                if constexpr (OS::kOn)
-                    os_prim_quartet_f32<LA, LB, LC, LD>(gf, P, Q, v);
-                else
-                    add_prim_quartet_f32<LA, LB, LC, LD>(gf, P, Q, reinterpret_cast<float *>(acc));
+                os_prim_quartet_f32<LA, LB, LC, LD>(gf, P, Q, v);
                 if (ik2 != ik && t + 1 < e.w) {
 #pragma unroll
                     for (int c = 0; c < 8; ++c) Q[c] = Qn[c];
@@ -731,21 +808,63 @@ eri_thread_kernel(const int4 *__restrict__ list, int nq,
                 ib = ib2;
                 ik = ik2;
             }
-            if constexpr (OS::kOn) OS::template hrr<float>(gf.AB, gf.CD, v, reinterpret_cast<float *>(acc));
+            OS::template hrr<float>(gf.AB, gf.CD, v, reinterpret_cast<float *>(acc));
             const QCtx q = make_qctx(pb, pk, e.x, e.y);
             epi.template thread_quartet<LA, LB, LC, LD, R>(q, acc, lane, live);
             continue;
         }
-        PrimJK Pn = load_prim_jk(pbp + ib);
-        PrimJK Q = load_prim_jk(pkp + ik);
-        if constexpr (OsClass<LA, LB, LC, LD>::kOn) {
-            // Obara--Saika per primitive quartet, Head-Gordon--Pople transfer
-            // once per item on the contracted [e0|f0]
-            using OS = OsClass<LA, LB, LC, LD>;
-            constexpr int LT = LA + LB + LC + LD;
-            R v[OS::NV];
+        // Obara--Saika per primitive quartet, Head-Gordon--Pople transfer
+        // once per item on the contracted [e0|f0]
+        constexpr int LT = LA + LB + LC + LD;
+        R v[OS::NV];
 #pragma unroll
-            for (int c = 0; c < OS::NV; ++c) v[c] = (R)0;
+        for (int c = 0; c < OS::NV; ++c) v[c] = (R)0;
+        const auto add = [&](const PrimJK &P, const PrimJK &Q) {
+            const double zeta = P.zeta, eta = Q.zeta;
+            const double PQx = P.P[0] - Q.P[0], PQy = P.P[1] - Q.P[1], PQz = P.P[2] - Q.P[2];
+            const double rs = rsqrt_nr_unchecked(zeta + eta);   // exponent sums: 1e-36 < x < 1e36
+            const double izpe = rs * rs;
+            const double T = zeta * eta * izpe * (PQx * PQx + PQy * PQy + PQz * PQz);
+            const double pre = P.K * Q.K * rs;
+            double F[LT + 1];
+            boys_os<LT>(T, F);
+            R Fs[LT + 1];
+#pragma unroll
+            for (int m = 0; m <= LT; ++m) Fs[m] = (R)(F[m] * pre);
+            OsGeom<R> g;
+            const double rz = eta * izpe, re = zeta * izpe;
+            g.PA[0] = P.P[0] - Ax;
+            g.PA[1] = P.P[1] - Ay;
+            g.PA[2] = P.P[2] - Az;
+            g.QC[0] = Q.P[0] - Cx;
+            g.QC[1] = Q.P[1] - Cy;
+            g.QC[2] = Q.P[2] - Cz;
+            g.WP[0] = -rz * PQx;
+            g.WP[1] = -rz * PQy;
+            g.WP[2] = -rz * PQz;
+            g.WQ[0] = re * PQx;
+            g.WQ[1] = re * PQy;
+            g.WQ[2] = re * PQz;
+            g.rz = rz;
+            g.re = re;
+            g.oo2z = 0.5 * P.izeta;
+            g.oo2e = 0.5 * Q.izeta;
+            g.oo2ze = 0.5 * izpe;
+            OS::template vrr<R>(g, Fs, v);
+        };
+        if constexpr (G > 1) {
+            for (int t = lane % G; t < e.w; t += G) {
+                const int kq = (e.z + t) / npb, kb = e.z + t - kq * npb;
+                add(load_prim_jk(pbp + kb), load_prim_jk(pkp + kq));
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < OS::NV; ++c)
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+        } else {
+            PrimJK Pn = load_prim_jk(pbp + ib);
+            PrimJK Q = load_prim_jk(pkp + ik);
             for (int t = 0; t < e.w; ++t) {
                 const PrimJK P = Pn;
                 int ib2 = ib + 1, ik2 = ik;
@@ -757,288 +876,195 @@ eri_thread_kernel(const int4 *__restrict__ list, int nq,
                 // the next ket primitive pair, fetched a step ahead
                 PrimJK Qn = Q;
                 if (ik2 != ik && t + 1 < e.w) Qn = load_prim_jk(pkp + ik2);
-                const double zeta = P.zeta, eta = Q.zeta;
-                const double PQx = P.P[0] - Q.P[0], PQy = P.P[1] - Q.P[1], PQz = P.P[2] - Q.P[2];
-                const double rs = rsqrt_nr_unchecked(zeta + eta);   // exponent sums: 1e-36 < x < 1e36
-                const double izpe = rs * rs;
-                const double T = zeta * eta * izpe * (PQx * PQx + PQy * PQy + PQz * PQz);
-                const double pre = P.K * Q.K * rs;
-                double F[LT + 1];
-                boys_os<LT>(T, F);
-                R Fs[LT + 1];
-#pragma unroll
-                for (int m = 0; m <= LT; ++m) Fs[m] = (R)(F[m] * pre);
-                OsGeom<R> g;
-                const double rz = eta * izpe, re = zeta * izpe;
-                g.PA[0] = P.P[0] - Ax;
-                g.PA[1] = P.P[1] - Ay;
-                g.PA[2] = P.P[2] - Az;
-                g.QC[0] = Q.P[0] - Cx;
-                g.QC[1] = Q.P[1] - Cy;
-                g.QC[2] = Q.P[2] - Cz;
-                g.WP[0] = -rz * PQx;
-                g.WP[1] = -rz * PQy;
-                g.WP[2] = -rz * PQz;
-                g.WQ[0] = re * PQx;
-                g.WQ[1] = re * PQy;
-                g.WQ[2] = re * PQz;
-                g.rz = rz;
-                g.re = re;
-                g.oo2z = 0.5 * P.izeta;
-                g.oo2e = 0.5 * Q.izeta;
-                g.oo2ze = 0.5 * izpe;
-                OS::template vrr<R>(g, Fs, v);
+                add(P, Q);
                 Q = Qn;
                 ib = ib2;
                 ik = ik2;
             }
-            const R AB[3] = {(R)ABx, (R)ABy, (R)ABz}, CD[3] = {(R)CDx, (R)CDy, (R)CDz};
-            OS::template hrr<R>(AB, CD, v, acc);
-            const QCtx q = make_qctx(pb, pk, e.x, e.y);
-            epi.template thread_quartet<LA, LB, LC, LD, R>(q, acc, lane, live);
-            continue;
         }
-        for (int t = 0; t < e.w; ++t) {
-            const PrimJK P = Pn;
-            // the next bra primitive pair is fetched while this one computes
-            int ib2 = ib + 1, ik2 = ik;
-            if (ib2 == npb) {
-                ib2 = 0;
-                ++ik2;
-            }
-            if (t + 1 < e.w) Pn = load_prim_jk(pbp + ib2);
-            const double zeta = P.zeta, eta = Q.zeta;
-            const double PQx = P.P[0] - Q.P[0], PQy = P.P[1] - Q.P[1], PQz = P.P[2] - Q.P[2];
-            const double rs = rsqrt_nr(zeta + eta);
-            const double izpe = rs * rs;
-            const double T = zeta * eta * izpe * (PQx * PQx + PQy * PQy + PQz * PQz);
-            const double pre = P.K * Q.K * rs;
-            double uu[NR], ww[NR];
-            rys_roots_fast<NR>(T, uu, ww);
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const RysCoef k = rys_coef(uu[r], zeta, eta, P.izeta, Q.izeta, izpe);
-                R gx[G2D], gy[G2D], gz[G2D];
-                rys2d_c<LA, LB, LC, LD, R>(k, P.P[0] - Ax, Q.P[0] - Cx, PQx, ABx, CDx, ww[r] * pre, gx);
-                rys2d_c<LA, LB, LC, LD, R>(k, P.P[1] - Ay, Q.P[1] - Cy, PQy, ABy, CDy, 1.0, gy);
-                rys2d_c<LA, LB, LC, LD, R>(k, P.P[2] - Az, Q.P[2] - Cz, PQz, ABz, CDz, 1.0, gz);
-#pragma unroll
-                for (int ab = 0; ab < NAB; ++ab)
-#pragma unroll
-                    for (int cd = 0; cd < NCD; ++cd) {
-                        const int ia = ab / NB, ib3 = ab % NB, ic = cd / ND, id = cd % ND;
-                        const int ox = ((cart_lx(LA, ia) * (LB + 1) + cart_lx(LB, ib3)) * (LC + 1) + cart_lx(LC, ic)) *
-                                           (LD + 1) + cart_lx(LD, id);
-                        const int oy = ((cart_ly(LA, ia) * (LB + 1) + cart_ly(LB, ib3)) * (LC + 1) + cart_ly(LC, ic)) *
-                                           (LD + 1) + cart_ly(LD, id);
-                        const int oz = ((cart_lz(LA, ia) * (LB + 1) + cart_lz(LB, ib3)) * (LC + 1) + cart_lz(LC, ic)) *
-                                           (LD + 1) + cart_lz(LD, id);
-                        acc[ab * NCD + cd] += gx[ox] * gy[oy] * gz[oz];
-                    }
-            }
-            if (ik2 != ik && t + 1 < e.w) Q = load_prim_jk(pkp + ik2);
-            ib = ib2;
-            ik = ik2;
-        }
+        const R AB[3] = {(R)ABx, (R)ABy, (R)ABz}, CD[3] = {(R)CDx, (R)CDy, (R)CDz};
+        OS::template hrr<R>(AB, CD, v, acc);
         const QCtx q = make_qctx(pb, pk, e.x, e.y);
-        epi.template thread_quartet<LA, LB, LC, LD, R>(q, acc, lane, live);
+        epi.template thread_quartet<LA, LB, LC, LD, R>(q, acc, lane, live && lane % G == 0);
     }
 }
 
-// ----------------------------------------------------------- block mode --
-constexpr int kBlockThreads = 256;
+// ------------------------------------------------------------ warp mode --
+// The larger classes, by Rys quadrature.  A warp holds S = 32/NCD quartets
+// (two halves of (22|22)'s ket components take turns); a pass takes up to PB
+// primitive quartets of each through three steps with a warp barrier between
+// them: roots and recurrence coefficients (a lane per primitive quartet,
+// quartet and root), 2-D integrals into shared memory (times three axes), and
+// assembly, where a lane adds up the NAB bra components of its ket component
+// pair in registers (its 2-D entries are at compile-time offsets from one
+// address per axis).
+// Bound by shared-memory wavefronts (70-77 % of the L1 data pipe before the
+// pitches were odd) and FP64 issue (28 % of its peak; 10-19 % before).  C8H18 /
+// 6-31G** (N = 210), the eight classes one after the other, launches included:
+// 794 us, of which (21|11) 185; with 256-thread blocks whose eight warps met at
+// two block barriers a pass, and a digestion through a shared tile, 1077 and 329.
+// The whole build: 2.38 -> 2.13 ms; (H2O)8 / 6-31G** 0.372 -> 0.324 ms.  16 KB of
+// tables a warp (longer passes, fewer blocks) measured the same.
+constexpr int kWarpsPerBlock = 4;
 
-// Shared-memory budget of the 2-D integrals of one pass of a block: PB
-// primitive quartets per slot go through the roots, 2-D and assembly phases
-// together (two barriers per pass), as many as fit in the budget (at most 4).
-constexpr size_t kBlockPassBytes = 64 * 1024;
-
-template <int LA, int LB, int LC, int LD, typename R, class Epi>
-struct BlockLayout {
-    static constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    static constexpr int NAB = NA * NB, NCD = NC * ND;
+template <int LA, int LB, int LC, int LD>
+struct WarpLayout {
+    static constexpr int NAB = ncart(LA) * ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
     static constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
-    static constexpr int G2D = (LA + 1) * (LB + 1) * (LC + 1) * (LD + 1);
-    static constexpr int NSQ = kBlockThreads / NAB;
-    static constexpr size_t pq_bytes = (size_t)NSQ * 3 * NR * G2D * sizeof(R);   // one primitive quartet per slot
-    static constexpr int PB = pq_bytes * 4 <= kBlockPassBytes ? 4
-                              : pq_bytes * 3 <= kBlockPassBytes ? 3
-                              : pq_bytes * 2 <= kBlockPassBytes ? 2 : 1;
-    static constexpr size_t g_bytes = (PB * pq_bytes + 15) / 16 * 16;
-    // the integral tile of a tiled epilogue reuses the 2-D integral buffer
-    static constexpr size_t tile_bytes = Epi::kTile ? (size_t)NSQ * NAB * (NCD + 1) * sizeof(double) : 0;
-    static constexpr size_t bytes = g_bytes > tile_bytes ? g_bytes : tile_bytes;
+    static constexpr int HALVES = NCD > 32 ? 2 : 1, NCW = NC / HALVES, W = NCW * ND, S = 32 / W;
+    // odd pitches: the lanes' tables (2-D step) and the slots' (assembly) spread over the banks
+    static constexpr int G2D = ((LA + 1) * (LB + 1) * (LC + 1) * (LD + 1)) | 1, slot_words = 3 * NR * G2D | 1;
+    // primitive quartets of a pass: their roots occupy the lanes, within 12 KB of tables
+    static constexpr int fit = 32 / (S * NR), by_mem = 12288 / (8 * S * slot_words);
+    static constexpr int PB0 = fit < by_mem ? fit : by_mem, PB = PB0 < 1 ? 1 : (PB0 > 4 ? 4 : PB0);
+    static constexpr int tab_words = PB * S * slot_words;
+    // the Jacc[a,b] sums reuse the tables
+    static constexpr int words = tab_words > NAB * 33 ? tab_words : NAB * 33;
+    static constexpr size_t bytes = sizeof(double) * kWarpsPerBlock * words;
 };
 
+template <int NR> struct RysRoots {
+    double w[NR], b00[NR], b10[NR], b01[NR], ce[NR], cz[NR];
+    double PA[3], QC[3], PQ[3];
+};
 struct SlotData {
     QCtx q;
-    int npk, pp0, npp, pb_off, pk_off;
+    int npb, pp0, npp, pb_off, pk_off;
+    bool live;         // a work item that is not screened
     double A[3], AB[3], C[3], CD[3];
 };
-struct SlotPrim {
-    double zeta, eta, PA[3], QC[3], PQ[3];
-};
 
-// (the classes with at most six ket components fit three blocks per SM)
-template <int LA, int LB, int LC, int LD, typename R, class Epi>
-__global__ void __launch_bounds__(kBlockThreads, ncart(LC) * ncart(LD) <= 6 ? 3 : 0) eri_block_kernel(const int4 *__restrict__ list, int nq,
-                                                                  const PairInfo *__restrict__ pairs,
-                                                                  const PrimPair *__restrict__ prims, Epi epi)
+template <int LA, int LB, int LC, int LD, class Epi>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, WarpLayout<LA, LB, LC, LD>::NAB > 18 ? 3 : 4) eri_warp_kernel(const int4 *__restrict__ list, int nq,
+                                                                          const PairInfo *__restrict__ pairs,
+                                                                          const PrimPair *__restrict__ prims, Epi epi)
 {
-    using Lay = BlockLayout<LA, LB, LC, LD, R, Epi>;
-    constexpr int NB = Lay::NB, NC = Lay::NC, ND = Lay::ND, NAB = Lay::NAB, NCD = Lay::NCD;
-    constexpr int NR = Lay::NR, G2D = Lay::G2D, NSQ = Lay::NSQ, PB = Lay::PB;
+    using Lay = WarpLayout<LA, LB, LC, LD>;
+    constexpr int NB = ncart(LB), ND = Lay::ND, NAB = Lay::NAB, NR = Lay::NR, G2D = Lay::G2D, S = Lay::S, W = Lay::W,
+                  PB = Lay::PB, SW = Lay::slot_words;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R *sg = reinterpret_cast<R *>(smem_raw);
-    __shared__ SlotData sd[NSQ];
-    __shared__ SlotPrim sp[PB][NSQ];
-    __shared__ double su[PB][NSQ][NR], sw[PB][NSQ][NR];
-    __shared__ int s_maxpp;
-
-    const int tid = threadIdx.x;
-    const int slot = tid / NAB, ab = tid - slot * NAB;
-    const bool active = slot < NSQ;
-    const int ia = active ? ab / NB : 0, ib = active ? ab % NB : 0;
-    // offsets of this thread's bra component pair inside one (slot, axis, root) 2-D block
-    const int ox = (cart_l(LA, ia, 0) * (LB + 1) + cart_l(LB, ib, 0)) * (LC + 1) * (LD + 1);
-    const int oy = (cart_l(LA, ia, 1) * (LB + 1) + cart_l(LB, ib, 1)) * (LC + 1) * (LD + 1);
-    const int oz = (cart_l(LA, ia, 2) * (LB + 1) + cart_l(LB, ib, 2)) * (LC + 1) * (LD + 1);
-
-    for (int base = blockIdx.x * NSQ; base < nq; base += gridDim.x * NSQ) {
-        if (tid == 0) s_maxpp = 0;
-        __syncthreads();
-        if (tid < NSQ) {
-            SlotData &s = sd[tid];
-            const int qi = base + tid;
-            bool take = qi < nq;
-            if (take) {
-                const int4 t = list[qi];
-                take = !epi.screened(pairs[t.x], pairs[t.y], t.x, t.y);
-            }
-            if (take) {
-                const int4 e = list[qi];
-                const PairInfo &pb = pairs[e.x];
-                const PairInfo &pk = pairs[e.y];
-                s.q = make_qctx(pb, pk, e.x, e.y);
-                s.npk = pk.nprim;
-                s.pp0 = e.z;
-                s.npp = e.w;
-                s.pb_off = pb.prim_off;
-                s.pk_off = pk.prim_off;
-                for (int x = 0; x < 3; ++x) {
-                    s.A[x] = pb.A[x];
-                    s.AB[x] = pb.AB[x];
-                    s.C[x] = pk.A[x];
-                    s.CD[x] = pk.AB[x];
-                }
-                atomicMax(&s_maxpp, s.npp);
-            } else {
-                s.q.bra = -1;
-                s.npk = 1;
-                s.pp0 = s.npp = 0;
-                s.pb_off = s.pk_off = 0;
-                for (int x = 0; x < 3; ++x) s.A[x] = s.AB[x] = s.C[x] = s.CD[x] = 0.0;
+    __shared__ SlotData sd[kWarpsPerBlock][S];
+    __shared__ RysRoots<NR> sr[kWarpsPerBlock][PB * S];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *tab = reinterpret_cast<double *>(smem_raw) + (size_t)warp * Lay::words;
+    const int slot = lane / W, k = lane - slot * W;
+    const int stride = gridDim.x * kWarpsPerBlock * S;
+    for (int base = (blockIdx.x * kWarpsPerBlock + warp) * S; base < nq; base += stride) {
+        int npp = 0;
+        bool any = false;
+        if (lane < S) {
+            // (a slot without a live item keeps a valid quartet and no primitives)
+            const int qi = base + lane;
+            const int4 e = list[qi < nq ? qi : nq - 1];
+            const PairInfo &pb = pairs[e.x];
+            const PairInfo &pk = pairs[e.y];
+            SlotData &s = sd[warp][lane];
+            s.live = qi < nq && !epi.screened(pb, pk, e.x, e.y);
+            any = s.live;
+            npp = s.live ? e.w : 0;   // (0 too where every primitive pair was dropped: zero integrals)
+            s.q = make_qctx(pb, pk, e.x, e.y);
+            s.npb = pb.nprim;
+            s.pp0 = e.z;
+            s.npp = npp;
+            s.pb_off = pb.prim_off;
+            s.pk_off = pk.prim_off;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                s.A[x] = pb.A[x];
+                s.AB[x] = pb.AB[x];
+                s.C[x] = pk.A[x];
+                s.CD[x] = pk.AB[x];
             }
         }
-        __syncthreads();
-        const int maxpp = s_maxpp;
-
-        R acc[NCD];
+        const int maxpp = (int)__reduce_max_sync(0xffffffffu, (unsigned)npp);
+        if (!__any_sync(0xffffffffu, any)) continue;   // nothing but screened items
+        __syncwarp();
+        const bool live = slot < S && sd[warp][slot < S ? slot : 0].live;
+#pragma unroll 1
+        for (int half = 0; half < Lay::HALVES; ++half) {
+            const int c = half * Lay::NCW + k / ND, d = k - k / ND * ND;
+            const int ox = cart_l(LC, c, 0) * (LD + 1) + cart_l(LD, d, 0);
+            const int oy = cart_l(LC, c, 1) * (LD + 1) + cart_l(LD, d, 1);
+            const int oz = cart_l(LC, c, 2) * (LD + 1) + cart_l(LD, d, 2);
+            double acc[NAB];
 #pragma unroll
-        for (int c = 0; c < NCD; ++c) acc[c] = (R)0;
-
-        for (int pp0 = 0; pp0 < maxpp; pp0 += PB) {
-            // this pass: primitive quartets pp0 .. pp0 + nb - 1 of every slot
-            const int nb = maxpp - pp0 < PB ? maxpp - pp0 : PB;
-            // roots and weights (with the primitive-quartet prefactor)
-            for (int t = tid; t < nb * NSQ * NR; t += kBlockThreads) {
-                const int b = t / (NSQ * NR), rem = t - b * (NSQ * NR), s = rem / NR, r = rem - s * NR;
-                const int pp = pp0 + b;
-                const SlotData &S = sd[s];
-                if (pp < S.npp) {
-                    const int g = S.pp0 + pp;
-                    const int jb = g / S.npk, jk = g - jb * S.npk;
-                    const PrimPair P = prims[S.pb_off + jb];
-                    const PrimPair Q = prims[S.pk_off + jk];
-                    const double zpe = P.zeta + Q.zeta;
-                    const double PQx = P.P[0] - Q.P[0], PQy = P.P[1] - Q.P[1], PQz = P.P[2] - Q.P[2];
-                    const double T = P.zeta * Q.zeta / zpe * (PQx * PQx + PQy * PQy + PQz * PQz);
-                    double u, w;
-                    if constexpr (NR == 1) {
-                        double uu[1], ww[1];
-                        rys_roots<1>(T, uu, ww);
-                        u = uu[0];
-                        w = ww[0];
-                    } else {
+            for (int ab = 0; ab < NAB; ++ab) acc[ab] = 0.0;
+            for (int pp0 = 0; pp0 < maxpp; pp0 += PB) {
+                const int nb = maxpp - pp0 < PB ? maxpp - pp0 : PB;
+                if (lane < nb * S * NR) {
+                    const int bs = lane / NR, r = lane - bs * NR, b = bs / S;
+                    const SlotData &s = sd[warp][bs - b * S];
+                    if (pp0 + b < s.npp) {
+                        // bra primitives fastest
+                        const int g = s.pp0 + pp0 + b, jk = g / s.npb, jb = g - jk * s.npb;
+                        const PrimJK P = load_prim_jk(prims + s.pb_off + jb), Q = load_prim_jk(prims + s.pk_off + jk);
+                        const double PQ[3] = {P.P[0] - Q.P[0], P.P[1] - Q.P[1], P.P[2] - Q.P[2]};
+                        const double rs = rsqrt_nr(P.zeta + Q.zeta), izpe = rs * rs;
+                        const double T = P.zeta * Q.zeta * izpe * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+                        double u, w;
                         rys_root(NR, r, T, u, w);
-                    }
-                    su[b][s][r] = u;
-                    sw[b][s][r] = w * P.K * Q.K * rsqrt(zpe);
-                    if (r == 0) {
-                        SlotPrim &p = sp[b][s];
-                        p.zeta = P.zeta;
-                        p.eta = Q.zeta;
-                        p.PQ[0] = PQx;
-                        p.PQ[1] = PQy;
-                        p.PQ[2] = PQz;
-                        for (int x = 0; x < 3; ++x) {
-                            p.PA[x] = P.P[x] - S.A[x];
-                            p.QC[x] = Q.P[x] - S.C[x];
+                        const RysCoef f = rys_coef(u, P.zeta, Q.zeta, P.izeta, Q.izeta, izpe);
+                        RysRoots<NR> &o = sr[warp][bs];
+                        o.w[r] = w * P.K * Q.K * rs;
+                        o.b00[r] = f.b00;
+                        o.b10[r] = f.b10;
+                        o.b01[r] = f.b01;
+                        o.ce[r] = f.ce;
+                        o.cz[r] = f.cz;
+                        if (r == 0) {
+#pragma unroll
+                            for (int x = 0; x < 3; ++x) {
+                                o.PA[x] = P.P[x] - s.A[x];
+                                o.QC[x] = Q.P[x] - s.C[x];
+                                o.PQ[x] = PQ[x];
+                            }
                         }
                     }
-                } else {
-                    su[b][s][r] = 0.0;
-                    sw[b][s][r] = 0.0;
-                    if (r == 0) {
-                        SlotPrim &p = sp[b][s];
-                        p.zeta = p.eta = 1.0;
-                        for (int x = 0; x < 3; ++x) p.PA[x] = p.QC[x] = p.PQ[x] = 0.0;
+                }
+                __syncwarp();
+                for (int t = lane; t < nb * S * NR * 3; t += 32) {
+                    const int bs = t / (NR * 3), rx = t - bs * (NR * 3), r = rx / 3, x = rx - r * 3, b = bs / S;
+                    const SlotData &s = sd[warp][bs - b * S];
+                    if (pp0 + b < s.npp) {
+                        const RysRoots<NR> &o = sr[warp][bs];
+                        const RysCoef f{o.b00[r], o.b10[r], o.b01[r], o.ce[r], o.cz[r]};
+                        rys2d_c<LA, LB, LC, LD, double>(f, o.PA[x], o.QC[x], o.PQ[x], s.AB[x], s.CD[x],
+                                                        x == 0 ? o.w[r] : 1.0, tab + bs * SW + (x * NR + r) * G2D);
                     }
                 }
-            }
-            __syncthreads();
-            // 2-D integrals, one (pass quartet, slot, root, axis) per task; weight on x
-            for (int t = tid; t < nb * NSQ * NR * 3; t += kBlockThreads) {
-                const int b = t / (NSQ * NR * 3), rb = t - b * (NSQ * NR * 3);
-                const int s = rb / (NR * 3), rem = rb - s * NR * 3, r = rem / 3, x = rem - r * 3;
-                const SlotPrim &p = sp[b][s];
-                rys2d<LA, LB, LC, LD, R>(su[b][s][r], p.zeta, p.eta, p.PA[x], p.QC[x], p.PQ[x], sd[s].AB[x],
-                                         sd[s].CD[x], x == 0 ? sw[b][s][r] : 1.0,
-                                         sg + ((size_t)((b * NSQ + s) * 3 + x) * NR + r) * G2D);
-            }
-            __syncthreads();
-            // assembly: this thread's bra pair (ia, ib) times every ket pair
-            if (active) {
-                for (int b = 0; b < nb; ++b) {
-                    const R *gx = sg + (size_t)((b * NSQ + slot) * 3 + 0) * NR * G2D + ox;
-                    const R *gy = sg + (size_t)((b * NSQ + slot) * 3 + 1) * NR * G2D + oy;
-                    const R *gz = sg + (size_t)((b * NSQ + slot) * 3 + 2) * NR * G2D + oz;
+                __syncwarp();
+                if (live) {
+                    const int left = sd[warp][slot].npp - pp0, mine = left < nb ? left : nb;
+#pragma unroll 1
+                    for (int b = 0; b < mine; ++b) {
+                        const double *gx = tab + (b * S + slot) * SW + ox, *gy = tab + (b * S + slot) * SW + NR * G2D + oy,
+                                     *gz = tab + (b * S + slot) * SW + 2 * NR * G2D + oz;
+#pragma unroll 1
+                        for (int r = 0; r < NR; ++r, gx += G2D, gy += G2D, gz += G2D) {
+                            // entries (a, b') of each axis: one address, compile-time offsets
+                            double X[(LA + 1) * (LB + 1)], Y[(LA + 1) * (LB + 1)], Z[(LA + 1) * (LB + 1)];
 #pragma unroll
-                    for (int r = 0; r < NR; ++r)
-#pragma unroll
-                        for (int ic = 0; ic < NC; ++ic)
-#pragma unroll
-                            for (int id = 0; id < ND; ++id) {
-                                const int cx = cart_lx(LC, ic) * (LD + 1) + cart_lx(LD, id);
-                                const int cy = cart_ly(LC, ic) * (LD + 1) + cart_ly(LD, id);
-                                const int cz = cart_lz(LC, ic) * (LD + 1) + cart_lz(LD, id);
-                                acc[ic * ND + id] += gx[r * G2D + cx] * gy[r * G2D + cy] * gz[r * G2D + cz];
+                            for (int m = 0; m < (LA + 1) * (LB + 1); ++m) {
+                                X[m] = gx[m * (LC + 1) * (LD + 1)];
+                                Y[m] = gy[m * (LC + 1) * (LD + 1)];
+                                Z[m] = gz[m * (LC + 1) * (LD + 1)];
                             }
+#pragma unroll
+                            for (int ab = 0; ab < NAB; ++ab) {
+                                const int ia = ab / NB, ib = ab % NB;
+                                acc[ab] = fma(X[cart_lx(LA, ia) * (LB + 1) + cart_lx(LB, ib)] *
+                                                  Y[cart_ly(LA, ia) * (LB + 1) + cart_ly(LB, ib)],
+                                              Z[cart_lz(LA, ia) * (LB + 1) + cart_lz(LB, ib)], acc[ab]);
+                            }
+                        }
+                    }
                 }
+                __syncwarp();   // the next pass, or the epilogue's buffer, overwrites the tables
             }
+            epi.template lane_quartet<LA, LB, LC, LD, Lay::NCW>(sd[warp][slot < S ? slot : 0].q, c, d, lane, live, acc,
+                                                                tab);
         }
-
-        if constexpr (Epi::kTile) {
-            constexpr int ST = NCD + 1;
-            double *V = reinterpret_cast<double *>(smem_raw) + (size_t)slot * NAB * ST;
-            __syncthreads();   // the tile overwrites the 2-D integrals
-            if (active && sd[slot].q.bra >= 0) epi.template tile_store<LA, LB, LC, LD, R>(sd[slot].q, ia, ib, acc, V);
-            __syncthreads();
-            if (active && sd[slot].q.bra >= 0) epi.template tile_reduce<LA, LB, LC, LD>(sd[slot].q, V, ab, NAB);
-        } else {
-            if (active && sd[slot].q.bra >= 0) epi.template block_ab<LA, LB, LC, LD, R>(sd[slot].q, ia, ib, acc);
-        }
-        __syncthreads();
+        __syncwarp();   // the next items overwrite the slots
     }
 }
 
@@ -1051,19 +1077,29 @@ __host__ __device__ constexpr int pc_lb(int c) { return c == 0 ? 0 : (c == 1 ? 0
 
 template <int LA, int LB, int LC, int LD, typename R, class Epi>
 inline cudaError_t launch_eri_class(const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                                    const Epi &epi, cudaStream_t st, int nsm)
+                                    const Epi &epi, cudaStream_t st, int nsm, int nlong)
 {
     if (nq <= 0) return cudaSuccess;
     constexpr int NAB = ncart(LA) * ncart(LB), NCD = ncart(LC) * ncart(LD);
-    // thread mode while the contracted components fit in registers
-    constexpr int kThreadMax = 81;
     if constexpr (NAB * NCD <= kThreadMax) {
+        if constexpr (Epi::kCoop) {
+            // the list's first nlong items, of more than kCoopItem primitive quartets
+            if (nlong > 0) {
+                int grid = (nlong * kCoopLanes + 127) / 128;
+                if (grid > nsm * 32) grid = nsm * 32;
+                eri_thread_kernel<LA, LB, LC, LD, R, Epi, kCoopLanes><<<grid, 128, 0, st>>>(list, nlong, pairs, prims,
+                                                                                            epi);
+                list += nlong;
+                nq -= nlong;
+            }
+            if (nq == 0) return cudaGetLastError();
+        }
         int grid = (nq + 127) / 128;
         if (grid > nsm * 32) grid = nsm * 32;
         eri_thread_kernel<LA, LB, LC, LD, R, Epi><<<grid, 128, 0, st>>>(list, nq, pairs, prims, epi);
-    } else {
-        using Lay = BlockLayout<LA, LB, LC, LD, R, Epi>;
-        auto kern = eri_block_kernel<LA, LB, LC, LD, R, Epi>;
+    } else if constexpr (std::is_same_v<R, double>) {
+        using Lay = WarpLayout<LA, LB, LC, LD>;
+        auto kern = eri_warp_kernel<LA, LB, LC, LD, Epi>;
         // the attribute is per device: set once per instantiation and device
         static std::atomic<unsigned long long> attr_set{0};
         int dev = 0;
@@ -1075,9 +1111,11 @@ inline cudaError_t launch_eri_class(const int4 *list, int nq, const PairInfo *pa
             if (e != cudaSuccess) return e;
             attr_set.fetch_or(bit);
         }
-        int grid = (nq + Lay::NSQ - 1) / Lay::NSQ;
-        if (grid > nsm * 8) grid = nsm * 8;
-        kern<<<grid, kBlockThreads, Lay::bytes, st>>>(list, nq, pairs, prims, epi);
+        int grid = (nq + kWarpsPerBlock * Lay::S - 1) / (kWarpsPerBlock * Lay::S);
+        if (grid > nsm * 16) grid = nsm * 16;
+        kern<<<grid, kWarpsPerBlock * 32, Lay::bytes, st>>>(list, nq, pairs, prims, epi);
+    } else {
+        return cudaErrorInvalidValue;   // the host sends these classes' FP32 lists to the FP64 kernels
     }
     return cudaGetLastError();
 }
@@ -1085,12 +1123,12 @@ inline cudaError_t launch_eri_class(const int4 *list, int nq, const PairInfo *pa
 // Run class `qc` (0..20): bra pair class cb >= ket pair class ck.
 template <typename R, class Epi>
 inline cudaError_t launch_eri(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                              const Epi &epi, cudaStream_t st, int nsm)
+                              const Epi &epi, cudaStream_t st, int nsm, int nlong = 0)
 {
 #define PQB_CASE(CB, CK)                                                                                       \
     case CB *(CB + 1) / 2 + CK:                                                                               \
         return launch_eri_class<pc_la(CB), pc_lb(CB), pc_la(CK), pc_lb(CK), R, Epi>(list, nq, pairs, prims, epi, \
-                                                                                    st, nsm);
+                                                                                    st, nsm, nlong);
     switch (qc) {
         PQB_CASE(0, 0)
         PQB_CASE(1, 0) PQB_CASE(1, 1)

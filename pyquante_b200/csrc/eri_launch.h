@@ -16,8 +16,9 @@ struct EpiPacked;
 template <int NDEN, bool WITHK> struct EpiJKn;
 struct EpiSchwarz;
 
-cudaError_t launch_packed_f64(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                              double *out, const double *fscale, cudaStream_t st, int nsm);
+// nlong: the list's leading items of more than kCoopItem primitive quartets
+cudaError_t launch_packed_f64(int qc, const int4 *list, int nq, int nlong, const PairInfo *pairs,
+                              const PrimPair *prims, double *out, const double *fscale, cudaStream_t st, int nsm);
 cudaError_t launch_jk_f64(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
                           const double *Dscaled, double *Jacc, double *Kacc, int n, cudaStream_t st, int nsm,
                           const ItemScreen &scr = ItemScreen{});
@@ -37,8 +38,8 @@ cudaError_t launch_jk2_f64(int qc, const int4 *list, int nq, const PairInfo *pai
 cudaError_t launch_jk2_f32(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
                            const double *const Dscaled[2], const float *const Dscaled_f[2], double *const Jacc[2],
                            double *const Kacc[2], cudaStream_t st, int nsm, const ItemScreen &scr = ItemScreen{});
-cudaError_t launch_schwarz_f64(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                               unsigned long long *Q2bits, const double *fscale, cudaStream_t st, int nsm);
+cudaError_t launch_schwarz_f64(int qc, const int4 *list, int nq, int nlong, const PairInfo *pairs,
+                               const PrimPair *prims, unsigned long long *Q2bits, const double *fscale, cudaStream_t st, int nsm);
 // Adds dE2 per shell (gshell[3 nshell]) from the pre-scaled density; the
 // gather adds the shells to their atoms.
 cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,

@@ -57,10 +57,10 @@ struct pqb_ctx {
     bool have_q = false;
     // unscreened lists (packed integrals): per class offset/count into d_full
     int4 *d_full = nullptr;
-    int64_t full_off[kNumQuartetClass] = {0}, full_cnt[kNumQuartetClass] = {0};
+    int64_t full_off[kNumQuartetClass] = {0}, full_cnt[kNumQuartetClass] = {0}, full_long[kNumQuartetClass] = {0};
     // Schwarz (diagonal) list
     int4 *d_diag = nullptr;
-    int64_t diag_off[kNumQuartetClass] = {0}, diag_cnt[kNumQuartetClass] = {0};
+    int64_t diag_off[kNumQuartetClass] = {0}, diag_cnt[kNumQuartetClass] = {0}, diag_long[kNumQuartetClass] = {0};
     // screened plan: [0] FP64 part, [1] FP32-eligible part
     int4 *d_plan = nullptr;
     size_t plan_cap = 0;
@@ -1124,7 +1124,9 @@ static void order_class_items(const std::vector<const std::vector<int4> *> &segs
     for (auto &e : bybra) dst[hist[maxp - e.w]++] = e;
 }
 
-static void bucket_sorted(std::vector<std::vector<int4>> &cls, std::vector<int4> &flat, int64_t *off, int64_t *cnt)
+// nlong: each class's leading items of more than kCoopItem primitive quartets.
+static void bucket_sorted(std::vector<std::vector<int4>> &cls, std::vector<int4> &flat, int64_t *off, int64_t *cnt,
+                          int64_t *nlong)
 {
     flat.clear();
     for (int c = 0; c < kNumQuartetClass; ++c) {
@@ -1132,6 +1134,7 @@ static void bucket_sorted(std::vector<std::vector<int4>> &cls, std::vector<int4>
         cnt[c] = (int64_t)cls[c].size();
         flat.resize(flat.size() + cls[c].size());
         order_class_items({&cls[c]}, flat.data() + off[c]);
+        nlong[c] = std::count_if(cls[c].begin(), cls[c].end(), [](const int4 &e) { return e.w > kCoopItem; });
     }
 }
 
@@ -1296,7 +1299,7 @@ static int shells_upload_batch_impl(pqb_ctx *ctx, int nmol, const int *mol_shell
     PQB_CK(ctx, cudaMemcpy(ctx->d_mol_off, ctx->mol_off.data(), sizeof(long long) * nmol, cudaMemcpyHostToDevice));
     PQB_CK(ctx, cudaMemcpy(ctx->d_mol_n, ctx->mol_n.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
     std::vector<int4> flat;
-    bucket_sorted(dcls, flat, ctx->diag_off, ctx->diag_cnt);
+    bucket_sorted(dcls, flat, ctx->diag_off, ctx->diag_cnt, ctx->diag_long);
     PQB_CK(ctx, cudaMalloc(&ctx->d_diag, sizeof(int4) * std::max<size_t>(flat.size(), 1)));
     PQB_CK(ctx, cudaMemcpy(ctx->d_diag, flat.data(), sizeof(int4) * flat.size(), cudaMemcpyHostToDevice));
     return PQB_OK;
@@ -1325,7 +1328,7 @@ static int schwarz_impl(pqb_ctx *ctx, double *Q_host, void *stream)
     const int np = (int)ctx->pairs.size();
     PQB_CK(ctx, cudaMemsetAsync(ctx->d_q2, 0, sizeof(unsigned long long) * np, st));
     for (int c = 0; c < kNumQuartetClass; ++c)
-        PQB_CK(ctx, launch_schwarz_f64(c, ctx->d_diag + ctx->diag_off[c], (int)ctx->diag_cnt[c], ctx->d_pairs,
+        PQB_CK(ctx, launch_schwarz_f64(c, ctx->d_diag + ctx->diag_off[c], (int)ctx->diag_cnt[c], (int)ctx->diag_long[c], ctx->d_pairs,
                                        ctx->d_prims, ctx->d_q2, ctx->d_fscale, st, ctx->nsm));
     if (!ctx->d_Qpair) PQB_CK(ctx, cudaMalloc(&ctx->d_Qpair, sizeof(double) * np));
     double *dQ = ctx->d_Qpair;
@@ -1640,7 +1643,7 @@ static int ensure_full_list(pqb_ctx *ctx)
             cls[qc].push_back(e);
         }
     std::vector<int4> flat;
-    bucket_sorted(cls, flat, ctx->full_off, ctx->full_cnt);
+    bucket_sorted(cls, flat, ctx->full_off, ctx->full_cnt, ctx->full_long);
     PQB_CK(ctx, cudaMalloc(&ctx->d_full, sizeof(int4) * std::max<size_t>(flat.size(), 1)));
     PQB_CK(ctx, cudaMemcpy(ctx->d_full, flat.data(), sizeof(int4) * flat.size(), cudaMemcpyHostToDevice));
     return PQB_OK;
@@ -1664,7 +1667,7 @@ static int eri_packed_impl(pqb_ctx *ctx, double *out, int64_t len, void *stream)
     for (int k = 0; k < pqb_ctx::kStreams; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
     for (int c = kNumQuartetClass - 1, k = 0; c >= 0; --c) {
         if (ctx->full_cnt[c] == 0) continue;
-        PQB_CK(ctx, launch_packed_f64(c, ctx->d_full + ctx->full_off[c], (int)ctx->full_cnt[c], ctx->d_pairs,
+        PQB_CK(ctx, launch_packed_f64(c, ctx->d_full + ctx->full_off[c], (int)ctx->full_cnt[c], (int)ctx->full_long[c], ctx->d_pairs,
                                       ctx->d_prims, out, ctx->d_fscale, ctx->streams[k++ % pqb_ctx::kStreams],
                                       ctx->nsm));
     }
@@ -1722,9 +1725,10 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
     // in an FP64 build both parts of a class are one list (the plan is
     // class-major): one launch per class, over more items.  A small mixed build
     // runs the same way: it is bound by launches and chains, not by arithmetic
-    const bool merged = mode != PQB_MIXED || ctx->small_plan;
+    const bool one_list = mode != PQB_MIXED || ctx->small_plan;
     for (int i = 0, k = 0; i < 2 * kNumQuartetClass; ++i) {
         const int part = order[i] / kNumQuartetClass, c = order[i] % kNumQuartetClass;
+        const bool merged = one_list || warp_class(c);   // (the warp-mode classes have FP64 kernels only)
         if (merged && part == 1) continue;
         const int nq = (int)(ctx->plan_cnt[part][c] + (merged ? ctx->plan_cnt[1][c] : 0));
         if (nq == 0) continue;
@@ -1984,7 +1988,7 @@ int pqb_jk_direct_class(pqb_ctx *ctx, const double *D, double *Jacc, double *Kac
     const int nq = (int)ctx->plan_cnt[part][qclass];
     scale_elements_kernel<<<ctx->nsm * 4, 256, 0, st>>>(D, ctx->d_escale, ctx->d_Dscaled, ctx->d_Dscaled_f,
                                                          ctx->dense_len);
-    if (mode == PQB_MIXED && part == 1)
+    if (mode == PQB_MIXED && part == 1 && !warp_class(qclass))
         PQB_CK(ctx, launch_jk_f32(qclass, list, nq, ctx->d_pairs, ctx->d_prims, ctx->d_Dscaled, ctx->d_Dscaled_f, Jacc,
                                   Kacc, ctx->nbf, st, ctx->nsm));
     else

@@ -60,6 +60,27 @@ __host__ __device__ inline int pair_class(int la, int lb)   // la >= lb
     return la * (la + 1) / 2 + lb;
 }
 
+// Lists of whole quartets (packed integrals, Schwarz factors) hold items of up
+// to 64^4 primitive quartets; in thread mode kCoopLanes lanes share one of more
+// than kCoopItem.
+constexpr int kCoopItem = 24, kCoopLanes = 8;
+
+// Components of quartet class qc; classes of more than kThreadMax run in warp
+// mode, in FP64 in both precision modes.
+constexpr int kThreadMax = 81;
+
+__host__ __device__ constexpr int pair_components(int c)   // ss ps pp ds dp dd
+{
+    return c == 0 ? 1 : (c == 1 ? 3 : (c == 2 ? 9 : (c == 3 ? 6 : (c == 4 ? 18 : 36))));
+}
+
+inline bool warp_class(int qc)
+{
+    int cb = 0;
+    while ((cb + 1) * (cb + 2) / 2 <= qc) ++cb;
+    return pair_components(cb) * pair_components(qc - cb * (cb + 1) / 2) > kThreadMax;
+}
+
 // quartet class index for bra class cb >= ket class ck
 __host__ __device__ inline int quartet_class(int cb, int ck) { return cb * (cb + 1) / 2 + ck; }
 
