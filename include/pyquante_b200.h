@@ -113,6 +113,16 @@ int pqb_shell_dmax(pqb_ctx *ctx, const double *D, double *shell_dmax, void *stre
 int pqb_purify_step(int nmat, int n, const double *P, const double *P2, const double *P3, double *P_out, int *done,
                     double tol, void *stream);
 
+/* The whole purification of nmat symmetric n x n device matrices, n at most
+ * 112, one block per matrix: from F (its symmetric part is used), the number of
+ * occupied states nocc[m] and, per matrix, pad[n] != 0 for padded dimensions
+ * (held above the real spectrum; NULL: none), the projector P on the nocc
+ * lowest states by at most maxit steps of pqb_purify_step from the linear start
+ * of the Gershgorin bounds; done[m] (may be NULL) = 1 where |tr(P - P^2)| <
+ * tol n was reached.  PQB_E_SHAPE above n = 112. */
+int pqb_purify(int nmat, int n, const double *F, const double *nocc, const unsigned char *pad, double *P, int *done,
+               int maxit, double tol, void *stream);
+
 /* Schwarz factors Q_ab = sqrt(max |(ab|ab)|) for every shell pair, computed
  * on the device; copied to Q_host (length npairs) when it is not NULL. */
 int pqb_schwarz(pqb_ctx *ctx, double *Q_host, void *stream);

@@ -82,10 +82,23 @@ def purify(Fp, nocc, pad=None, tol=1e-13, maxit=200, fixed=False, check=1):
     idempotent to rounding (|tr(P - P^2)| < tol n), tested on the host every
     ``check`` steps (converged matrices are kept meanwhile); fixed=True runs exactly
     maxit steps with no host check instead (converged matrices are kept),
-    so that the loop can be captured in a CUDA graph.  Each step is two
-    batched GEMMs and one fused trace-and-update kernel (pqb_purify_step)."""
+    so that the loop can be captured in a CUDA graph.  Matrices of up to
+    PQB_PURIFY_MAX rows take one kernel for everything (pqb_purify); for larger
+    ones each step is two batched GEMMs and one fused trace-and-update kernel
+    (pqb_purify_step)."""
     from . import _lib
     lib = _lib.load()
+    if Fp.is_cuda and Fp.dim() == 3 and Fp.shape[1] == Fp.shape[2] <= _lib.PQB_PURIFY_MAX:
+        B, n = Fp.shape[0], Fp.shape[-1]
+        Fc = Fp.to(torch.float64).contiguous()
+        no = torch.as_tensor(nocc, dtype=torch.float64, device=Fp.device).reshape(-1).expand(B).contiguous()
+        pd = None if pad is None else pad.to(torch.uint8).expand(B, n).contiguous()
+        P = torch.empty_like(Fc)
+        rc = lib.pqb_purify(B, n, _lib.ptr(Fc), _lib.ptr(no), _lib.ptr(pd), _lib.ptr(P), None, int(maxit), float(tol),
+                            _lib.stream_ptr())
+        if rc != _lib.PQB_OK:
+            raise _lib.EngineError(rc, "pqb_purify")
+        return P
     Fp = 0.5 * (Fp + Fp.transpose(1, 2))
     nb = Fp.shape[-1]
     nocc = torch.as_tensor(nocc, dtype=Fp.dtype, device=Fp.device).reshape(-1)

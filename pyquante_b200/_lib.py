@@ -37,6 +37,8 @@ SIGNATURES = {
     "pqb_set_molecule_mask": (ctypes.c_int, [_vp, _vp]),
     "pqb_set_density_screen": (ctypes.c_int, [_vp, _vp, ctypes.c_double]),
     "pqb_shell_dmax": (ctypes.c_int, [_vp, _vp, _vp, _vp]),
+    "pqb_purify": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, ctypes.c_int, ctypes.c_double,
+                                  _vp]),
     "pqb_purify_step": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, ctypes.c_double, _vp]),
     "pqb_schwarz": (ctypes.c_int, [_vp, _c_dbl_p, _vp]),
     "pqb_num_pairs": (ctypes.c_int, [_vp]),
@@ -78,6 +80,8 @@ SIGNATURES = {
     "pqb_boys_rows_eval": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, _vp, _vp]),
     "pqb_rys_eval": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp]),
 }
+
+PQB_PURIFY_MAX = 112   # largest matrix of pqb_purify
 
 
 class EngineUnavailable(RuntimeError):

@@ -71,6 +71,39 @@ def test_purification_equals_eigenprojector():
                 assert np.abs(P[b, m:, :]).max() < 1e-12 and np.abs(P[b, :, m:]).max() < 1e-12
 
 
+@pytest.mark.parametrize("n,nocc", [(2, 1), (7, 5), (15, 4), (16, 16), (17, 3), (95, 25), (111, 40), (112, 1), (113, 30)])
+def test_purification_at_the_kernels_sizes(n, nocc):
+    """The one-kernel purification at its tiles' edges and the largest it
+    takes (113: the GEMM form), against the same iteration in numpy (which
+    reaches the eigenprojector in 200 steps for all but (112, 1)); the
+    unsymmetric part of F does not count."""
+    from pyquante_b200.LA2 import purify
+    rng = np.random.default_rng(n)
+    Q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    e = np.sort(rng.uniform(-20, 3, n))
+    e[nocc:] += 0.7
+    A = rng.standard_normal((n, n))
+    F = (Q * e) @ Q.T + (A - A.T)
+    P = purify(torch.tensor(F[None], device="cuda"), nocc).cpu().numpy()[0]
+    S = 0.5 * (F + F.T)
+    d = np.diag(S)
+    r = np.abs(S).sum(1) - np.abs(d)
+    hi, lo, mu = (d + r).max() + 1.0, (d - r).min(), d.mean()
+    ref = min(nocc / (hi - mu), (n - nocc) / (mu - lo)) / n * (mu * np.eye(n) - S) + nocc / n * np.eye(n)
+    for _ in range(200):
+        R2 = ref @ ref
+        R3 = R2 @ ref
+        den = np.trace(ref - R2)
+        if abs(den) < 1e-13 * n:
+            break
+        c = min(max(np.trace(R2 - R3) / den, 0.0), 1.0)
+        ref = ((1 + c) * R2 - R3) / c if c >= 0.5 else ((1 - 2 * c) * ref + (1 + c) * R2 - R3) / (1 - c)
+    if (n, nocc) != (112, 1):
+        assert np.abs(ref - Q[:, :nocc] @ Q[:, :nocc].T).max() < 1e-10
+    assert np.abs(P - ref).max() < 1e-10
+    assert np.array_equal(P, P.T) or n > 112
+
+
 def test_molecule_mask_skips_masked_molecules():
     """pqb_set_molecule_mask: the masked molecules' J and K blocks come out
     zero and the others' equal the unmasked build (FP64 and mixed, with the
