@@ -123,6 +123,11 @@ int pqb_purify_step(int nmat, int n, const double *P, const double *P2, const do
 int pqb_purify(int nmat, int n, const double *F, const double *nocc, const unsigned char *pad, double *P, int *done,
                int maxit, double tol, void *stream);
 
+/* x[m] with A[m] x[m] = b[m] for nmat dense n x n systems back to back, n at
+ * most 17 (PQB_E_SHAPE above), by Gauss-Jordan elimination with partial
+ * pivoting (the DIIS equations of a batch). */
+int pqb_solve_small(int nmat, int n, const double *A, const double *b, double *x, void *stream);
+
 /* Schwarz factors Q_ab = sqrt(max |(ab|ab)|) for every shell pair, computed
  * on the device; copied to Q_host (length npairs) when it is not NULL. */
 int pqb_schwarz(pqb_ctx *ctx, double *Q_host, void *stream);

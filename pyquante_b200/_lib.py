@@ -39,6 +39,7 @@ SIGNATURES = {
     "pqb_shell_dmax": (ctypes.c_int, [_vp, _vp, _vp, _vp]),
     "pqb_purify": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, ctypes.c_int, ctypes.c_double,
                                   _vp]),
+    "pqb_solve_small": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp]),
     "pqb_purify_step": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, ctypes.c_double, _vp]),
     "pqb_schwarz": (ctypes.c_int, [_vp, _c_dbl_p, _vp]),
     "pqb_num_pairs": (ctypes.c_int, [_vp]),
@@ -82,6 +83,7 @@ SIGNATURES = {
 }
 
 PQB_PURIFY_MAX = 112   # largest matrix of pqb_purify
+PQB_SOLVE_MAX = 17      # largest system of pqb_solve_small
 
 
 class EngineUnavailable(RuntimeError):

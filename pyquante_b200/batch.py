@@ -185,10 +185,18 @@ class _Bucket:
 
 def _solve_small(A, b):
     """x with A x = b for a batch of small systems (A: (B, n, n), b: (B, n)) by
-    Gauss-Jordan elimination with partial pivoting, in plain tensor
-    operations (no library solver, no host synchronisation), so that it can
-    be captured in a CUDA graph.  A singular system gives non-finite x."""
+    Gauss-Jordan elimination with partial pivoting (no library solver, no
+    host synchronisation), so that it can be captured in a CUDA graph: one
+    kernel on the GPU up to PQB_SOLVE_MAX rows, else plain tensor operations.
+    A singular system gives non-finite x."""
     Bn, n = A.shape[0], A.shape[-1]
+    if A.is_cuda and A.dtype == torch.float64 and n <= _lib.PQB_SOLVE_MAX:
+        A, b = A.contiguous(), b.contiguous()
+        x = torch.empty_like(b)
+        rc = _lib.load().pqb_solve_small(Bn, n, _lib.ptr(A), _lib.ptr(b), _lib.ptr(x), _lib.stream_ptr())
+        if rc != _lib.PQB_OK:
+            raise _lib.EngineError(rc, "pqb_solve_small")
+        return x
     M = torch.cat([A, b[..., None]], dim=-1)
     ar = torch.arange(n, device=A.device)[None, :]
     for j in range(n):

@@ -104,6 +104,25 @@ def test_purification_at_the_kernels_sizes(n, nocc):
     assert np.array_equal(P, P.T) or n > 112
 
 
+@pytest.mark.parametrize("n", [1, 2, 8, 9, 10, 17, 18])
+def test_small_solver_against_lapack(n):
+    """_solve_small on the GPU (18: the tensor form): pivoting needed, and a
+    singular system of the batch leaves the others alone."""
+    from pyquante_b200.batch import _solve_small
+    rng = np.random.default_rng(n)
+    B = 7
+    A = rng.standard_normal((B, n, n))
+    A[:, 0, 0] = 0.0 if n > 1 else 1.0
+    b = rng.standard_normal((B, n))
+    x = np.linalg.solve(A, b[..., None])[..., 0]
+    A[3] = 0.0
+    got = _solve_small(torch.tensor(A, device="cuda"), torch.tensor(b, device="cuda")).cpu().numpy()
+    ok = [m for m in range(B) if m != 3]
+    cond = np.linalg.cond(A[ok]).max()
+    assert np.abs(got[ok] - x[ok]).max() < 1e-14 * cond * np.abs(x[ok]).max() * n
+    assert not np.isfinite(got[3]).any()
+
+
 def test_molecule_mask_skips_masked_molecules():
     """pqb_set_molecule_mask: the masked molecules' J and K blocks come out
     zero and the others' equal the unmasked build (FP64 and mixed, with the
