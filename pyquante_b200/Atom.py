@@ -16,7 +16,7 @@ class Atom:
         return self.r[i]
 
     def pos(self):
-        return tuple(float(v) for v in self.r)
+        return tuple(np.asarray(self.r, dtype=float).tolist())
 
     def dist2(self, other):
         return float(((self.r - other.r) ** 2).sum())

@@ -29,8 +29,8 @@ class CGBF:
         pbf.coef = float(coefficient)
         self.prims.append(pbf)
         self.pnorms.append(pbf.norm)
-        self.pexps.append(float(exponent))
-        self.pcoefs.append(float(coefficient))
+        self.pexps.append(pbf.exp)
+        self.pcoefs.append(pbf.coef)
 
     def reset_powers(self, px, py, pz):
         self.powers = (px, py, pz)

@@ -61,8 +61,9 @@ def _oneint_functions(bfs, atoms):
 
 def get1ints(bfs, atoms):
     """Overlap S and h = T + V_nuc (PyQuante/Ints.py:73-87), numpy arrays."""
-    S, T, V = _oneint_functions(_bfs_list(bfs), atoms)
-    return S, T + V
+    ctx = _lib.context()
+    S, T, V = oneint(FunctionTable(_bfs_list(bfs), ctx.device), atoms, ctx)
+    return S.cpu().numpy(), T.add_(V).cpu().numpy()
 
 
 def getS(bfs):
@@ -287,8 +288,8 @@ def get2JmK(Ints, D):
         else:
             Dh = np.ascontiguousarray(D, dtype=np.float64)
             G = np.empty((n, n))
+        # (G is pageable: complete when the call returns)
         Ints.get2jmk_host(Dh, G)
-        Ints.synchronize()
         return G
     J, K = _jk(Ints, D)
     return _back(2.0 * J - K, D)

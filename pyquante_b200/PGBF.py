@@ -26,8 +26,10 @@ def primitive_norm(alpha, powers):
 class PGBF:
     def __init__(self, exponent, origin, powers=(0, 0, 0), norm=1.0):
         self.exp = float(exponent)
-        self.origin = tuple(float(c) for c in origin)
-        self.powers = tuple(int(p) for p in powers)
+        x, y, z = origin
+        self.origin = (float(x), float(y), float(z))
+        l, m, n = powers
+        self.powers = (int(l), int(m), int(n))
         self.norm = primitive_norm(self.exp, self.powers)
         self.coef = 1.0
 

@@ -186,11 +186,11 @@ __device__ __forceinline__ double attraction(const OneWarp &w, const double *A, 
 // primitive pairs goes first, one per lane (overlap and kinetic terms there,
 // the pair's data to shared memory unless its Gaussian factor is exactly
 // zero); then the lanes share the chunk's (primitive pair, atom) tasks.
-// Bound by FP64 latency and issue: C16H34 / 6-31G* (N = 308, 50 atoms) took
-// 11.6 ms (12.6 ms a get1ints call, now 1.24 ms) with one thread per (i, j),
-// which looped over its primitives, atoms
-// and Rys roots in local-memory tables, the lanes of a warp on unlike powers.
-__global__ void __launch_bounds__(kOneWarps * 32) oneint_kernel(int n, FuncTable ft, int natoms,
+// Bound by FP64 latency and issue: C16H34 / 6-31G* (N = 308, 50 atoms) takes
+// 0.24 ms (0.27 with the registers uncapped, 12 warps an SM instead of 20); 11.6
+// ms with one thread per (i, j), which looped over its primitives, atoms and Rys
+// roots in local-memory tables, the lanes of a warp on unlike powers.
+__global__ void __launch_bounds__(kOneWarps * 32, 5) oneint_kernel(int n, FuncTable ft, int natoms,
                                                                 const double *__restrict__ atoms, double *S,
                                                                 double *Tk, double *V)
 {

@@ -103,6 +103,10 @@ struct pqb_ctx {
     double *d_Jacc2 = nullptr, *d_Kacc2 = nullptr;   // second density's graph accumulators
     // pqb_get2jmk_host: D in, G out, and J, K of its builds outside the graph
     double *d_hD = nullptr, *d_hG = nullptr, *d_hJ = nullptr, *d_hK = nullptr;
+    // ... and, for pageable host arrays, the whole call as one graph over
+    // page-locked copies of D and G ([mode])
+    double *h_D = nullptr, *h_G = nullptr;
+    cudaGraphExec_t host_graph[2] = {nullptr, nullptr};
     ItemScreen scr{};                // caller-owned molecule mask / shell density bounds of the direct builds
     double *d_Qpair = nullptr;       // Schwarz factor per pair (device)
     int4 *d_shell_info = nullptr;    // per shell: first function within its molecule, functions, molecule
@@ -956,6 +960,27 @@ static int host_threads()
     return (int)std::min(32u, std::max(1u, hw));
 }
 
+// Capture what `record` puts on the context's capture stream into exec.
+template <class F> static int capture_graph(pqb_ctx *ctx, cudaGraphExec_t &exec, F record)
+{
+    if (!ctx->cap_stream) PQB_CK(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
+    PQB_CK(ctx, cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = record(ctx->cap_stream);
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(ctx->cap_stream, &g);   // always ends the capture
+    if (rc != PQB_OK || e != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return rc != PQB_OK ? rc : fail(ctx, PQB_E_CUDA, "graph capture: %s", cudaGetErrorString(e));
+    }
+    const cudaError_t ei = cudaGraphInstantiate(&exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ei != cudaSuccess) {
+        exec = nullptr;
+        return fail(ctx, PQB_E_CUDA, "graph instantiate: %s", cudaGetErrorString(ei));
+    }
+    return PQB_OK;
+}
+
 extern "C" {
 
 int pqb_version(void) { return 1; }
@@ -1003,6 +1028,10 @@ static void drop_graphs(pqb_ctx *ctx)
         ctx->graph_exec[gi] = nullptr;
         ctx->graph_warm[gi] = false;
     }
+    for (cudaGraphExec_t &g : ctx->host_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
 }
 
 static void release_basis(pqb_ctx *ctx)
@@ -1018,6 +1047,9 @@ static void release_basis(pqb_ctx *ctx)
     free_dev(ctx->d_hJ);
     free_dev(ctx->d_hK);
     ctx->d_hD = ctx->d_hG = ctx->d_hJ = ctx->d_hK = nullptr;
+    if (ctx->h_D) cudaFreeHost(ctx->h_D);
+    if (ctx->h_G) cudaFreeHost(ctx->h_G);
+    ctx->h_D = ctx->h_G = nullptr;
     free_dev(ctx->d_Dscaled2);
     free_dev(ctx->d_Dscaled2_f);
     ctx->d_Dscaled2 = nullptr;
@@ -1708,9 +1740,6 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
     const double *Ds[2] = {ctx->d_Dscaled, ctx->d_Dscaled2};
     const float *Dsf[2] = {ctx->d_Dscaled_f, ctx->d_Dscaled2_f};
     const ItemScreen &mm = ctx->scr;
-    // fork: class launches spread over the context's streams, heaviest first
-    PQB_CK(ctx, cudaEventRecord(ctx->ev_fork, st));
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
     int order[2 * kNumQuartetClass];
     double cost[2 * kNumQuartetClass];
     for (int i = 0; i < 2 * kNumQuartetClass; ++i) {
@@ -1726,13 +1755,21 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
     // class-major): one launch per class, over more items.  A small mixed build
     // runs the same way: it is bound by launches and chains, not by arithmetic
     const bool one_list = mode != PQB_MIXED || ctx->small_plan;
-    for (int i = 0, k = 0; i < 2 * kNumQuartetClass; ++i) {
+    int count[2 * kNumQuartetClass], launches = 0;
+    for (int i = 0; i < 2 * kNumQuartetClass; ++i) {
         const int part = order[i] / kNumQuartetClass, c = order[i] % kNumQuartetClass;
         const bool merged = one_list || warp_class(c);   // (the warp-mode classes have FP64 kernels only)
-        if (merged && part == 1) continue;
-        const int nq = (int)(ctx->plan_cnt[part][c] + (merged ? ctx->plan_cnt[1][c] : 0));
+        count[i] = merged && part == 1 ? 0 : (int)(ctx->plan_cnt[part][c] + (merged ? ctx->plan_cnt[1][c] : 0));
+        launches += count[i] > 0;
+    }
+    // fork: class launches spread over the context's streams, heaviest first
+    const int nst = std::min(ctx->nstreams, launches);
+    if (nst > 0) PQB_CK(ctx, cudaEventRecord(ctx->ev_fork, st));
+    for (int k = 0; k < nst; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
+    for (int i = 0, k = 0; i < 2 * kNumQuartetClass; ++i) {
+        const int part = order[i] / kNumQuartetClass, c = order[i] % kNumQuartetClass, nq = count[i];
         if (nq == 0) continue;
-        cudaStream_t sk = ctx->streams[k++ % ctx->nstreams];
+        cudaStream_t sk = ctx->streams[k++ % nst];
         const int4 *list = ctx->d_plan + ctx->plan_off[part][c];
         const bool f32 = part == 1;
         if (jonly) {
@@ -1756,7 +1793,7 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
         }
     }
     // join
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) {
+    for (int k = 0; k < nst; ++k) {
         PQB_CK(ctx, cudaEventRecord(ctx->ev_join[k], ctx->streams[k]));
         PQB_CK(ctx, cudaStreamWaitEvent(st, ctx->ev_join[k], 0));
     }
@@ -1791,27 +1828,13 @@ static int ensure_acc_pair(pqb_ctx *ctx, double *&J, double *&K)
 static int ensure_build_graph(pqb_ctx *ctx, int nden, bool jonly, int mode, int gi)
 {
     if (ctx->graph_exec[gi]) return PQB_OK;
-    if (!ctx->cap_stream) PQB_CK(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
     int rc = ensure_acc_pair(ctx, ctx->d_Jacc, ctx->d_Kacc);
     if (rc == PQB_OK && nden == 2) rc = ensure_acc_pair(ctx, ctx->d_Jacc2, ctx->d_Kacc2);
     if (rc != PQB_OK) return rc;
     double *const Ja[2] = {ctx->d_Jacc, ctx->d_Jacc2};
     double *const Ka[2] = {jonly ? nullptr : ctx->d_Kacc, ctx->d_Kacc2};
-    PQB_CK(ctx, cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
-    rc = launch_build(ctx, nden, Ja, Ka, mode, ctx->cap_stream, false);
-    cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(ctx->cap_stream, &g);   // always ends the capture
-    if (rc != PQB_OK || e != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        return rc != PQB_OK ? rc : fail(ctx, PQB_E_CUDA, "graph capture: %s", cudaGetErrorString(e));
-    }
-    const cudaError_t ei = cudaGraphInstantiate(&ctx->graph_exec[gi], g, 0);
-    cudaGraphDestroy(g);
-    if (ei != cudaSuccess) {
-        ctx->graph_exec[gi] = nullptr;
-        return fail(ctx, PQB_E_CUDA, "graph instantiate: %s", cudaGetErrorString(ei));
-    }
-    return PQB_OK;
+    return capture_graph(ctx, ctx->graph_exec[gi],
+                         [&](cudaStream_t cs) { return launch_build(ctx, nden, Ja, Ka, mode, cs, false); });
 }
 
 // J and K of nden densities D[s] into J[s], K[s] (K[0] == nullptr with one
@@ -1892,6 +1915,50 @@ int pqb_jk_direct(pqb_ctx *ctx, const double *D, double *J, double *K, int mode,
     return jk_direct_impl(ctx, 1, Dv, Jv, Kv, mode, stream);
 }
 
+static bool pageable(const void *p)
+{
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
+}
+
+// One launch for a repeated call on pageable arrays: D in, build, G out.
+static int get2jmk_pageable(pqb_ctx *ctx, const double *D_host, double *G_host, int mode, cudaStream_t st)
+{
+    const int n = ctx->nbf;
+    const size_t bytes = sizeof(double) * (size_t)n * n;
+    if (!ctx->h_D) PQB_CK(ctx, cudaMallocHost(&ctx->h_D, bytes));
+    if (!ctx->h_G) PQB_CK(ctx, cudaMallocHost(&ctx->h_G, bytes));
+    cudaGraphExec_t &exec = ctx->host_graph[mode == PQB_MIXED ? 1 : 0];
+    if (!exec) {
+        int rc = ensure_acc_pair(ctx, ctx->d_Jacc, ctx->d_Kacc);
+        if (rc != PQB_OK) return rc;
+        rc = capture_graph(ctx, exec, [&](cudaStream_t cs) {
+            PQB_CK(ctx, cudaMemcpyAsync(ctx->d_hD, ctx->h_D, bytes, cudaMemcpyHostToDevice, cs));
+            scale_elements_kernel<<<ctx->nsm * 4, 256, 0, cs>>>(ctx->d_hD, ctx->d_escale, ctx->d_Dscaled,
+                                                                 ctx->d_Dscaled_f, ctx->dense_len);
+            double *const Ja[2] = {ctx->d_Jacc, nullptr}, *const Ka[2] = {ctx->d_Kacc, nullptr};
+            const int r = launch_build(ctx, 1, Ja, Ka, mode, cs, false);
+            if (r != PQB_OK) return r;
+            const int64_t P = (int64_t)n * (n + 1) / 2;
+            take_2jmk_kernel<<<(unsigned)((P + 255) / 256), 256, 0, cs>>>(ctx->d_Jacc, ctx->d_Kacc, ctx->d_hG, n,
+                                                                          ctx->d_escale);
+            PQB_CK(ctx, cudaGetLastError());
+            PQB_CK(ctx, cudaMemcpyAsync(ctx->h_G, ctx->d_hG, bytes, cudaMemcpyDeviceToHost, cs));
+            return (int)PQB_OK;
+        });
+        if (rc != PQB_OK) return rc;
+    }
+    memcpy(ctx->h_D, D_host, bytes);
+    PQB_CK(ctx, cudaGraphLaunch(exec, st));
+    PQB_CK(ctx, cudaStreamSynchronize(st));
+    memcpy(G_host, ctx->h_G, bytes);
+    return PQB_OK;
+}
+
 static int get2jmk_host_impl(pqb_ctx *ctx, const double *D_host, double *G_host, int mode, void *stream)
 {
     if (!ctx || !D_host || !G_host) return fail(ctx, PQB_E_ARG, "pqb_get2jmk_host: bad arguments");
@@ -1905,6 +1972,11 @@ static int get2jmk_host_impl(pqb_ctx *ctx, const double *D_host, double *G_host,
     for (double **b : bufs)
         if (!*b) PQB_CK(ctx, cudaMalloc(b, bytes));
     cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PQB_CK(ctx, cudaStreamIsCapturing(st, &cs));
+    if (ctx->use_graph && cs == cudaStreamCaptureStatusNone && ctx->graph_warm[mode == PQB_MIXED ? 1 : 0] &&
+        pageable(D_host) && pageable(G_host))
+        return get2jmk_pageable(ctx, D_host, G_host, mode, st);
     PQB_CK(ctx, cudaMemcpyAsync(ctx->d_hD, D_host, bytes, cudaMemcpyHostToDevice, st));
     const double *Dv[2] = {ctx->d_hD, nullptr};
     double *Jv[2] = {ctx->d_hJ, nullptr}, *Kv[2] = {ctx->d_hK, nullptr};

@@ -79,29 +79,47 @@ def detect_shells(bfs, max_l=2):
 
 
 class FunctionTable:
-    """Per-function device table: origin, powers, prim_off, exps, cn, norms."""
+    """Per-function device table: origin, powers, prim_off, exps, cn, norms
+    (views of one buffer, copied to the device at once)."""
 
     def __init__(self, bfs, device):
         n = len(bfs)
         off = [0]
-        exps, cn = [], []
+        exps, pcoefs, pnorms, origin, powers, norms = [], [], [], [], [], []
         for bf in bfs:
-            if len(bf.pexps) != len(bf.pcoefs) or len(bf.pexps) != len(bf.pnorms) or not bf.pexps:
+            k = len(bf.pexps)
+            if k != len(bf.pcoefs) or k != len(bf.pnorms) or not k:
                 raise ValueError("inconsistent primitive lists in %r" % (bf,))
-            exps.extend(bf.pexps)
-            cn.extend(c * m for c, m in zip(bf.pcoefs, bf.pnorms))
+            exps += bf.pexps
+            pcoefs += bf.pcoefs
+            pnorms += bf.pnorms
+            origin += bf.origin
+            powers += bf.powers
+            norms.append(bf.norm)
             off.append(len(exps))
-        dev = torch.device("cuda", device)
-        f64 = dict(dtype=torch.float64, device=dev)
-        i32 = dict(dtype=torch.int32, device=dev)
+        if len(origin) != 3 * n or len(powers) != 3 * n:
+            raise ValueError("a function's origin and powers have three components")
+        np_ = len(exps)
         self.n = n
-        self.powers_host = np.array([bf.powers for bf in bfs], dtype=np.int32).reshape(n, 3)
-        self.origin = torch.tensor([bf.origin for bf in bfs], **f64).reshape(n, 3).contiguous()
-        self.powers = torch.tensor(self.powers_host, **i32).contiguous()
-        self.prim_off = torch.tensor(off, **i32)
-        self.exps = torch.tensor(exps, **f64)
-        self.cn = torch.tensor(cn, **f64)
-        self.norms = torch.tensor([bf.norm for bf in bfs], **f64)
+        self.powers_host = np.array(powers, dtype=np.int32).reshape(n, 3)
+        # doubles: origin, exps, cn, norms; then ints: powers, prim_off
+        nd, ni = 4 * n + 2 * np_, 4 * n + 1
+        host = np.empty(nd + (ni + 1) // 2)
+        host[:3 * n] = origin
+        host[3 * n:3 * n + np_] = exps
+        host[3 * n + np_:3 * n + 2 * np_] = np.array(pcoefs, dtype=np.float64) * np.array(pnorms, dtype=np.float64)
+        host[3 * n + 2 * np_:nd] = norms
+        ints = host[nd:].view(np.int32)
+        ints[:3 * n] = powers
+        ints[3 * n:ni] = off
+        buf = torch.from_numpy(host).to(torch.device("cuda", device))
+        ibuf = buf[nd:].view(torch.int32)
+        self.origin = buf[:3 * n].view(n, 3)
+        self.exps = buf[3 * n:3 * n + np_]
+        self.cn = buf[3 * n + np_:3 * n + 2 * np_]
+        self.norms = buf[3 * n + 2 * np_:nd]
+        self.powers = ibuf[:3 * n].view(n, 3)
+        self.prim_off = ibuf[3 * n:ni]
 
     def args(self):
         return (self.n, ptr(self.origin), ptr(self.powers), ptr(self.prim_off), ptr(self.exps), ptr(self.cn),
@@ -114,9 +132,7 @@ def oneint(ft, atoms, ctx, stream=None):
     if int(ft.powers_host.sum(axis=1).max(initial=0)) > 3:
         raise _lib.EngineError(_lib.PQB_E_CLASS, "one-electron integrals support up to f functions")
     dev = ft.origin.device
-    S = torch.empty((n, n), dtype=torch.float64, device=dev)
-    T = torch.empty_like(S)
-    V = torch.empty_like(S)
+    S, T, V = torch.empty((3, n, n), dtype=torch.float64, device=dev).unbind(0)
     atoms = list(atoms or [])
     xyz = (ctypes.c_double * max(3 * len(atoms), 1))(*[c for a in atoms for c in a.pos()])
     z = (ctypes.c_double * max(len(atoms), 1))(*[float(a.atno) for a in atoms])

@@ -56,15 +56,17 @@ def rhf_gradient_from_density(mol, eng, D, W, precision="fp64", schwarz=1e-12, f
     eng.ctx.check(lib.pqb_set_shell_atoms(h, (ctypes.c_int * len(sa))(*sa)))
     eng.plan(schwarz, fp32_threshold)
     mode = _lib.PQB_MIXED if precision == "mixed" else _lib.PQB_FP64
-    eng.ctx.check(lib.pqb_grad_2e(h, _lib.ptr(D), _lib.ptr(grad), mode, _lib.stream_ptr()))
     fa = torch.tensor([bf.atid for bf in eng.bfs], dtype=torch.int32, device=dev)
     xyz = (ctypes.c_double * (3 * nat))(*[c for a in mol.atoms for c in a.pos()])
     z = (ctypes.c_double * nat)(*[float(a.atno) for a in mol.atoms])
     ft = eng.ft
+    # (pqb_grad_1e waits for its own kernel; the two-electron part then runs
+    # while the host adds up the nuclear repulsion)
     eng.ctx.check(lib.pqb_grad_1e(h, *ft.args(), _lib.ptr(fa), nat, xyz, z, _lib.ptr(D), _lib.ptr(W), _lib.ptr(grad),
                                   _lib.stream_ptr()))
-    g = grad.view(nat, 3).cpu().numpy()
-    return g + nuclear_repulsion_gradient(mol)
+    eng.ctx.check(lib.pqb_grad_2e(h, _lib.ptr(D), _lib.ptr(grad), mode, _lib.stream_ptr()))
+    nuc = nuclear_repulsion_gradient(mol)
+    return grad.view(nat, 3).cpu().numpy() + nuc
 
 
 def rhf_with_gradient(mol, basis_data=None, **opts):
