@@ -156,9 +156,11 @@ int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *c
  * PQB_PARAM_THREADS = host threads that pqb_plan enumerates and orders the
  * quartets on (0, the default: all hardware threads up to 32 once a plan
  * has 4M shell quartets or more, else 1); the plan is the same for any
- * count. */
+ * count; PQB_PARAM_HERMITE = thousands of primitive quartets with a d shell
+ * in the plan from which pqb_jk_direct builds J alone in the Hermite basis
+ * (default 1500; 0 at any size). */
 enum { PQB_PARAM_CHUNK = 0, PQB_PARAM_STREAMS = 1, PQB_PARAM_ORDER = 2, PQB_PARAM_PACKED_KERNEL = 3,
-       PQB_PARAM_GRAPH = 4, PQB_PARAM_THREADS = 5 };
+       PQB_PARAM_GRAPH = 4, PQB_PARAM_THREADS = 5, PQB_PARAM_HERMITE = 6 };
 int pqb_set_param(pqb_ctx *ctx, int param, int qclass, int value);
 
 /* Per-class statistics of the current plan, arrays of 2*21 int64 indexed

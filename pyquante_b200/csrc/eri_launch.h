@@ -40,6 +40,28 @@ cudaError_t launch_jk2_f32(int qc, const int4 *list, int nq, const PairInfo *pai
                            double *const Kacc[2], cudaStream_t st, int nsm, const ItemScreen &scr = ItemScreen{});
 cudaError_t launch_schwarz_f64(int qc, const int4 *list, int nq, int nlong, const PairInfo *pairs,
                                const PrimPair *prims, unsigned long long *Q2bits, const double *fscale, cudaStream_t st, int nsm);
+// Coulomb matrix alone in the Hermite basis (eri_jengine.cu): the primitive
+// pairs of each L = La + Lb (n[L] from off[L] of list, sorted by the shell
+// pair's Schwarz factor, descending), and their Hermite density H and potential
+// V (nherm(L) values each from hoff[L]).
+struct JPrim {
+    double zeta, P[3], Q;
+    int pair, prim;
+};
+struct JLists {
+    JPrim *list = nullptr;
+    double *H = nullptr, *V = nullptr;
+    int n[5] = {0}, off[5] = {0};
+    int64_t hoff[5] = {0}, words = 0;
+};
+cudaError_t launch_hermite_pairs(int n, const int2 *src, const PairInfo *pairs, const PrimPair *prims, const double *Q,
+                                 JPrim *out, cudaStream_t st);
+cudaError_t launch_hermite_density(int L, const JLists &l, const PairInfo *pairs, const PrimPair *prims, const double *D,
+                                   int nbf, cudaStream_t st);
+cudaError_t launch_hermite_coulomb(int LP, int LQ, const JLists &l, double thresh, cudaStream_t st, int nsm);
+// first[pair]: offset of the pair's V
+cudaError_t launch_hermite_fock(int npair, const PairInfo *pairs, const PrimPair *prims, const int64_t *first,
+                                const double *V, int nbf, const double *escale, double *J, cudaStream_t st);
 // Adds dE2 per shell (gshell[3 nshell]) from the pre-scaled density; the
 // gather adds the shells to their atoms.
 cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,

@@ -207,7 +207,7 @@ def main():
                 pairs = [(cu[k], cw[k]) for k in range(7)] + [(0.0, 0.0)]
                 lines.append("  " + ", ".join("%.9ef, %.9ef" % (a, b) for a, b in pairs) + ",")
     lines.append("};")
-    lines.append("PQB_TABQ double pqb_boys_tab[PQB_BOYS_NGRID * PQB_BOYS_NORD] = {")
+    lines.append("PQB_TABQ __align__(64) double pqb_boys_tab[PQB_BOYS_NGRID * PQB_BOYS_NORD] = {")
     for row in boys_tab:
         lines.append("  " + ", ".join("%.17e" % v for v in row) + ",")
     lines.append("};")

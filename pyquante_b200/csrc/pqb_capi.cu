@@ -88,6 +88,7 @@ struct pqb_ctx {
     static constexpr int kStreams = 16;
     cudaStream_t streams[kStreams] = {nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[kStreams] = {nullptr};
+    int made = 0;                    // streams made so far (see Fan)
     bool have_plan = false;
     // pqb_jk_direct replays a captured graph of the class launches (one per
     // mode), accumulating into ctx-owned J/K; rebuilt after any change of
@@ -107,6 +108,13 @@ struct pqb_ctx {
     // page-locked copies of D and G ([mode])
     double *h_D = nullptr, *h_G = nullptr;
     cudaGraphExec_t host_graph[2] = {nullptr, nullptr};
+    // Coulomb-only builds in the Hermite basis (see ensure_jlists): the lists,
+    // each pair's place in V, and what they depend on
+    JLists jl;
+    int64_t *d_jfirst = nullptr;
+    double plan_thresh = 0.0;        // Schwarz threshold of the current plan
+    bool sharded = false;            // the current plan holds one rank's share
+    int64_t hermite_least = 1500000; // see hermite_route
     ItemScreen scr{};                // caller-owned molecule mask / shell density bounds of the direct builds
     double *d_Qpair = nullptr;       // Schwarz factor per pair (device)
     int4 *d_shell_info = nullptr;    // per shell: first function within its molecule, functions, molecule
@@ -960,6 +968,88 @@ static int host_threads()
     return (int)std::min(32u, std::max(1u, hw));
 }
 
+// Independent launches from one point of `main`: launch k goes to branch k mod n,
+// and `main` goes on when all have ended.  While `main` captures, a branch is a set
+// of dependencies in its graph; else one of the context's streams.  Those cost 75
+// us each to make, 1.2 ms for all 16, more than a first build of (H2O)8 takes; so a
+// call makes four at most and the context gets there with its fourth call: first
+// J of C8H18 / 6-31G** in a new context 3.0 -> 2.2 ms.
+struct Fan {
+    pqb_ctx *ctx;
+    cudaStream_t main;
+    int n = 0;
+    bool capturing = false;
+    std::vector<cudaGraphNode_t> root;
+    cudaGraphNode_t tail[pqb_ctx::kStreams] = {nullptr};
+
+    Fan(pqb_ctx *c, cudaStream_t st) : ctx(c), main(st) {}
+    cudaError_t deps(const cudaGraphNode_t *&d, size_t &nd)
+    {
+        cudaStreamCaptureStatus cs;
+        return cudaStreamGetCaptureInfo(main, &cs, nullptr, nullptr, &d, &nd);
+    }
+    cudaError_t fork(int branches)
+    {
+        n = std::max(1, std::min(branches, (int)pqb_ctx::kStreams));
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(main, &cs);
+        if (e != cudaSuccess) return e;
+        capturing = cs == cudaStreamCaptureStatusActive;
+        if (capturing) {
+            const cudaGraphNode_t *d = nullptr;
+            size_t nd = 0;
+            if ((e = deps(d, nd)) == cudaSuccess) root.assign(d, d + nd);
+            return e;
+        }
+        if (!ctx->ev_fork && (e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming)) != cudaSuccess) return e;
+        for (int k = 0; k < 4 && ctx->made < n; ++k) {
+            cudaEvent_t &ev = ctx->ev_join[ctx->made];
+            if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
+            e = cudaStreamCreateWithFlags(&ctx->streams[ctx->made], cudaStreamNonBlocking);
+            if (e != cudaSuccess) return e;
+            ++ctx->made;
+        }
+        n = std::min(n, ctx->made);
+        if ((e = cudaEventRecord(ctx->ev_fork, main)) != cudaSuccess) return e;
+        for (int k = 0; k < n && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0);
+        return e;
+    }
+    // launch(stream) as the k-th
+    template <class F> cudaError_t run(int k, F launch)
+    {
+        k %= n;
+        if (!capturing) return launch(ctx->streams[k]);
+        cudaError_t e = tail[k] ? cudaStreamUpdateCaptureDependencies(main, &tail[k], 1, cudaStreamSetCaptureDependencies)
+                                : cudaStreamUpdateCaptureDependencies(main, root.data(), root.size(),
+                                                                      cudaStreamSetCaptureDependencies);
+        if (e == cudaSuccess) e = launch(main);
+        const cudaGraphNode_t *d = nullptr;
+        size_t nd = 0;
+        if (e == cudaSuccess) e = deps(d, nd);
+        // (a launch of nothing leaves the branch as it was)
+        if (e == cudaSuccess && nd == 1 && (root.size() != 1 || *d != root[0])) tail[k] = *d;
+        return e;
+    }
+    cudaError_t join()
+    {
+        cudaError_t e = cudaSuccess;
+        if (capturing) {
+            cudaGraphNode_t last[pqb_ctx::kStreams];
+            int m = 0;
+            for (int k = 0; k < n; ++k)
+                if (tail[k]) last[m++] = tail[k];
+            return m ? cudaStreamUpdateCaptureDependencies(main, last, m, cudaStreamSetCaptureDependencies)
+                     : cudaStreamUpdateCaptureDependencies(main, root.data(), root.size(),
+                                                           cudaStreamSetCaptureDependencies);
+        }
+        for (int k = 0; k < n && e == cudaSuccess; ++k) {
+            e = cudaEventRecord(ctx->ev_join[k], ctx->streams[k]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(main, ctx->ev_join[k], 0);
+        }
+        return e;
+    }
+};
+
 // Capture what `record` puts on the context's capture stream into exec.
 template <class F> static int capture_graph(pqb_ctx *ctx, cudaGraphExec_t &exec, F record)
 {
@@ -1009,18 +1099,6 @@ int pqb_create(pqb_ctx **out, int device)
     return PQB_OK;
 }
 
-static cudaError_t ensure_streams(pqb_ctx *ctx)
-{
-    if (ctx->ev_fork) return cudaSuccess;
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) {
-        cudaError_t e = cudaStreamCreateWithFlags(&ctx->streams[k], cudaStreamNonBlocking);
-        if (e != cudaSuccess) return e;
-        e = cudaEventCreateWithFlags(&ctx->ev_join[k], cudaEventDisableTiming);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
-}
-
 static void drop_graphs(pqb_ctx *ctx)
 {
     for (int gi = 0; gi < 6; ++gi) {
@@ -1034,9 +1112,20 @@ static void drop_graphs(pqb_ctx *ctx)
     }
 }
 
+static void drop_jlists(pqb_ctx *ctx)
+{
+    free_dev(ctx->jl.list);
+    free_dev(ctx->jl.H);
+    free_dev(ctx->jl.V);
+    free_dev(ctx->d_jfirst);
+    ctx->jl = JLists{};
+    ctx->d_jfirst = nullptr;
+}
+
 static void release_basis(pqb_ctx *ctx)
 {
     drop_graphs(ctx);
+    drop_jlists(ctx);
     free_dev(ctx->d_Jacc);
     free_dev(ctx->d_Kacc);
     free_dev(ctx->d_Jacc2);
@@ -1358,6 +1447,8 @@ static int schwarz_impl(pqb_ctx *ctx, double *Q_host, void *stream)
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
     const int np = (int)ctx->pairs.size();
+    drop_graphs(ctx);
+    drop_jlists(ctx);   // sorted by the factors that this call computes
     PQB_CK(ctx, cudaMemsetAsync(ctx->d_q2, 0, sizeof(unsigned long long) * np, st));
     for (int c = 0; c < kNumQuartetClass; ++c)
         PQB_CK(ctx, launch_schwarz_f64(c, ctx->d_diag + ctx->diag_off[c], (int)ctx->diag_cnt[c], (int)ctx->diag_long[c], ctx->d_pairs,
@@ -1532,6 +1623,8 @@ int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *c
     }
     if (need) PQB_CK(ctx, cudaMemcpy(ctx->d_plan, ctx->plan_h.data(), sizeof(int4) * need, cudaMemcpyHostToDevice));
     ctx->have_plan = true;
+    ctx->plan_thresh = schwarz_thresh;
+    ctx->sharded = false;
     if (counts) {
         counts[0] = total;
         counts[1] = nitems[0];
@@ -1578,6 +1671,10 @@ int pqb_set_param(pqb_ctx *ctx, int param, int qclass, int value)
         ctx->plan_threads = value;
         ctx->have_plan = false;   // takes effect at the next pqb_plan
         return PQB_OK;
+    case PQB_PARAM_HERMITE:
+        if (value < 0) return fail(ctx, PQB_E_ARG, "hermite %d out of range", value);
+        ctx->hermite_least = (int64_t)value * 1000;
+        return PQB_OK;
     }
     return fail(ctx, PQB_E_ARG, "unknown parameter %d", param);
 }
@@ -1622,6 +1719,7 @@ static int plan_shard_impl(pqb_ctx *ctx, int rank, int nranks)
     memcpy(ctx->plan_cnt, cnt, sizeof cnt);
     memcpy(ctx->plan_prims, prims, sizeof prims);
     ctx->plan_h.swap(out);
+    ctx->sharded = ctx->sharded || nranks > 1;
     return PQB_OK;
 }
 
@@ -1694,19 +1792,16 @@ static int eri_packed_impl(pqb_ctx *ctx, double *out, int64_t len, void *stream)
         const int rc = ensure_full_list(ctx);
         if (rc != PQB_OK) return rc;
     }
-    PQB_CK(ctx, ensure_streams(ctx));
-    PQB_CK(ctx, cudaEventRecord(ctx->ev_fork, st));
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
+    Fan fan(ctx, st);
+    PQB_CK(ctx, fan.fork(pqb_ctx::kStreams));
     for (int c = kNumQuartetClass - 1, k = 0; c >= 0; --c) {
         if (ctx->full_cnt[c] == 0) continue;
-        PQB_CK(ctx, launch_packed_f64(c, ctx->d_full + ctx->full_off[c], (int)ctx->full_cnt[c], (int)ctx->full_long[c], ctx->d_pairs,
-                                      ctx->d_prims, out, ctx->d_fscale, ctx->streams[k++ % pqb_ctx::kStreams],
-                                      ctx->nsm));
+        PQB_CK(ctx, fan.run(k++, [&](cudaStream_t sk) {
+            return launch_packed_f64(c, ctx->d_full + ctx->full_off[c], (int)ctx->full_cnt[c], (int)ctx->full_long[c],
+                                     ctx->d_pairs, ctx->d_prims, out, ctx->d_fscale, sk, ctx->nsm);
+        }));
     }
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) {
-        PQB_CK(ctx, cudaEventRecord(ctx->ev_join[k], ctx->streams[k]));
-        PQB_CK(ctx, cudaStreamWaitEvent(st, ctx->ev_join[k], 0));
-    }
+    PQB_CK(ctx, fan.join());
     return PQB_OK;
 }
 
@@ -1762,41 +1857,28 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
         count[i] = merged && part == 1 ? 0 : (int)(ctx->plan_cnt[part][c] + (merged ? ctx->plan_cnt[1][c] : 0));
         launches += count[i] > 0;
     }
-    // fork: class launches spread over the context's streams, heaviest first
-    const int nst = std::min(ctx->nstreams, launches);
-    if (nst > 0) PQB_CK(ctx, cudaEventRecord(ctx->ev_fork, st));
-    for (int k = 0; k < nst; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
+    // class launches spread over the branches, heaviest first
+    Fan fan(ctx, st);
+    if (launches) PQB_CK(ctx, fan.fork(std::min(ctx->nstreams, launches)));
     for (int i = 0, k = 0; i < 2 * kNumQuartetClass; ++i) {
         const int part = order[i] / kNumQuartetClass, c = order[i] % kNumQuartetClass, nq = count[i];
         if (nq == 0) continue;
-        cudaStream_t sk = ctx->streams[k++ % nst];
         const int4 *list = ctx->d_plan + ctx->plan_off[part][c];
-        const bool f32 = part == 1;
-        if (jonly) {
-            if (f32)
-                PQB_CK(ctx, launch_j_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Dsf[0], Jacc[0], sk, ctx->nsm,
-                                         mm));
-            else
-                PQB_CK(ctx, launch_j_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Jacc[0], sk, ctx->nsm, mm));
-        } else if (nden == 2) {
-            if (f32)
-                PQB_CK(ctx, launch_jk2_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds, Dsf, Jacc, Kacc, sk, ctx->nsm,
-                                           mm));
-            else
-                PQB_CK(ctx, launch_jk2_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds, Jacc, Kacc, sk, ctx->nsm, mm));
-        } else if (f32) {
-            PQB_CK(ctx, launch_jk_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Dsf[0], Jacc[0], Kacc[0], n, sk,
-                                      ctx->nsm, mm));
-        } else {
-            PQB_CK(ctx, launch_jk_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Jacc[0], Kacc[0], n, sk,
-                                      ctx->nsm, mm));
-        }
+        PQB_CK(ctx, fan.run(k++, [&](cudaStream_t sk) {
+            if (jonly && part == 1)
+                return launch_j_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Dsf[0], Jacc[0], sk, ctx->nsm, mm);
+            if (jonly) return launch_j_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Jacc[0], sk, ctx->nsm, mm);
+            if (nden == 2 && part == 1)
+                return launch_jk2_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds, Dsf, Jacc, Kacc, sk, ctx->nsm, mm);
+            if (nden == 2)
+                return launch_jk2_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds, Jacc, Kacc, sk, ctx->nsm, mm);
+            if (part == 1)
+                return launch_jk_f32(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Dsf[0], Jacc[0], Kacc[0], n, sk,
+                                     ctx->nsm, mm);
+            return launch_jk_f64(c, list, nq, ctx->d_pairs, ctx->d_prims, Ds[0], Jacc[0], Kacc[0], n, sk, ctx->nsm, mm);
+        }));
     }
-    // join
-    for (int k = 0; k < nst; ++k) {
-        PQB_CK(ctx, cudaEventRecord(ctx->ev_join[k], ctx->streams[k]));
-        PQB_CK(ctx, cudaStreamWaitEvent(st, ctx->ev_join[k], 0));
-    }
+    if (launches) PQB_CK(ctx, fan.join());
     return PQB_OK;
 }
 
@@ -1837,9 +1919,110 @@ static int ensure_build_graph(pqb_ctx *ctx, int nden, bool jonly, int mode, int 
                          [&](cudaStream_t cs) { return launch_build(ctx, nden, Ja, Ka, mode, cs, false); });
 }
 
+// Whether a Coulomb-only build goes through the Hermite basis: for one whole,
+// unscreened molecule whose plan holds at least 1.5 M surviving primitive quartets
+// with a d shell.  What the Hermite form saves grows with the momenta (its work is
+// one product per pair of Hermite functions, not per quartet of components), and
+// its 22 launches take 60 - 100 us whatever the size.  Hermite / class kernels, us, by such quartets:
+//   (H2O)5 6-31G* 0.3 M 83 / 68;  (H2O)5 6-31G** 0.4 M 94 / 85;  C4H10 6-31G*
+//   1.4 M 151 / 145;  (H2O)8 6-31G** 1.7 M 190 / 242;  C5H12 6-31G* 2.8 M 231 /
+//   254;  C8H18 6-31G* 9.9 M 617 / 885, 6-31G** 12.8 M 916 / 1561.
+// With s and p alone the class kernels stay ahead at every size (STO-3G: C8H18
+// 185 / 157, C20H42 1113 / 1097).
+static bool hermite_route(const pqb_ctx *ctx)
+{
+    if (ctx->nmol != 1 || ctx->sharded || ctx->scr.molmask || ctx->scr.dmax || !ctx->have_q) return false;
+    constexpr int kFirstD = 6;   // classes 0 .. 5 are those of ss, ps and pp pairs
+    int64_t prims = 0;
+    for (int part = 0; part < 2; ++part)
+        for (int c = kFirstD; c < kNumQuartetClass; ++c) prims += ctx->plan_prims[part][c];
+    return prims >= ctx->hermite_least;
+}
+
+// The Hermite lists of a Coulomb-only build, made on first use: the shell pairs
+// of each L = La + Lb by descending Schwarz factor, their primitive pairs in turn.
+// Without memory for them the lists stay empty (not an error: the class kernels
+// need none).
+static int ensure_jlists(pqb_ctx *ctx, cudaStream_t st)
+{
+    if (ctx->jl.list) return PQB_OK;
+    drop_graphs(ctx);   // a build captured while there was no memory is one of the class kernels
+    const auto &pairs = ctx->pairs;
+    const int np = (int)pairs.size();
+    std::vector<std::pair<double, int>> byL[5];   // (-Q, pair): ascending is descending Q, equal ones by index
+    size_t nsrc = 0;
+    for (int p = 0; p < np; ++p) {
+        byL[pairs[p].la + pairs[p].lb].emplace_back(-ctx->Q[p], p);
+        nsrc += pairs[p].nprim;
+    }
+    JLists l;
+    std::vector<int2> src;
+    src.reserve(nsrc);
+    std::vector<int64_t> first(np, 0);
+    for (int L = 0; L < 5; ++L) {
+        std::sort(byL[L].begin(), byL[L].end());
+        const int nh = (L + 1) * (L + 2) * (L + 3) / 6;
+        l.off[L] = (int)src.size();
+        l.hoff[L] = l.words;
+        for (const auto &[negq, p] : byL[L]) {
+            first[p] = l.hoff[L] + (int64_t)((int)src.size() - l.off[L]) * nh;
+            for (int k = 0; k < pairs[p].nprim; ++k) src.push_back(make_int2(p, k));
+        }
+        l.n[L] = (int)src.size() - l.off[L];
+        l.words += (int64_t)l.n[L] * nh;
+    }
+    int2 *d_src = nullptr;
+    const size_t n = std::max<size_t>(src.size(), 1), words = std::max<int64_t>(l.words, 1);
+    cudaError_t e = cudaMalloc(&d_src, sizeof(int2) * n);
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_jfirst, sizeof(int64_t) * std::max(np, 1));
+    if (e == cudaSuccess) e = cudaMalloc(&l.H, sizeof(double) * words);
+    if (e == cudaSuccess) e = cudaMalloc(&l.V, sizeof(double) * words);
+    if (e == cudaSuccess) e = cudaMalloc(&l.list, sizeof(JPrim) * n);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_src, src.data(), sizeof(int2) * src.size(), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(ctx->d_jfirst, first.data(), sizeof(int64_t) * np, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = launch_hermite_pairs((int)src.size(), d_src, ctx->d_pairs, ctx->d_prims, ctx->d_Qpair, l.list, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host vectors and d_src go
+    free_dev(d_src);
+    ctx->jl = l;
+    if (e != cudaSuccess) {
+        drop_jlists(ctx);
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            return PQB_OK;
+        }
+        return fail(ctx, PQB_E_CUDA, "Hermite lists: %s", cudaGetErrorString(e));
+    }
+    return PQB_OK;
+}
+
+// V of the scaled density in d_Dscaled: the Hermite density, then every pair of
+// lists on the context's streams, the costliest first.
+static int launch_hermite(pqb_ctx *ctx, cudaStream_t st)
+{
+    const JLists &l = ctx->jl;
+    PQB_CK(ctx, cudaMemsetAsync(l.V, 0, sizeof(double) * l.words, st));
+    Fan dens(ctx, st), coul(ctx, st);
+    PQB_CK(ctx, dens.fork(std::min(5, ctx->nstreams)));
+    for (int L = 0; L < 5; ++L)
+        PQB_CK(ctx, dens.run(L, [&](cudaStream_t sk) {
+            return launch_hermite_density(L, l, ctx->d_pairs, ctx->d_prims, ctx->d_Dscaled, ctx->nbf, sk);
+        }));
+    PQB_CK(ctx, dens.join());
+    PQB_CK(ctx, coul.fork(std::min(15, ctx->nstreams)));
+    int k = 0;
+    for (int lp = 4; lp >= 0; --lp)
+        for (int lq = lp; lq >= 0; --lq)
+            PQB_CK(ctx, coul.run(k++, [&](cudaStream_t sk) {
+                return launch_hermite_coulomb(lq, lp, l, ctx->plan_thresh, sk, ctx->nsm);
+            }));
+    PQB_CK(ctx, coul.join());
+    return PQB_OK;
+}
+
 // J and K of nden densities D[s] into J[s], K[s] (K[0] == nullptr with one
-// density: J alone).
-// J and K of nden densities.  With G (one density, J and K wanted): G = 2J - K
+// density: J alone).  With G (one density, J and K wanted): G = 2J - K
 // as well; on the graph path G alone is written (J, K untouched), else J and
 // K are written and then combined.
 static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], double *const J[2], double *const K[2],
@@ -1848,7 +2031,6 @@ static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], doub
     const bool jonly = nden == 1 && !K[0];
     const int n = ctx->nbf;
     cudaStream_t st = (cudaStream_t)stream;
-    PQB_CK(ctx, ensure_streams(ctx));
     if (nden == 2 && !ctx->d_Dscaled2) {
         const size_t len = std::max<long long>(ctx->dense_len, 1);
         PQB_CK(ctx, cudaMalloc(&ctx->d_Dscaled2, sizeof(double) * len));
@@ -1870,6 +2052,29 @@ static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], doub
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PQB_CK(ctx, cudaStreamIsCapturing(st, &cs));
     const int gi = (jonly ? 4 : (nden == 2 ? 2 : 0)) + (mode == PQB_MIXED ? 1 : 0);
+    // J alone in the Hermite basis (FP64 in both modes).  A caller's capture uses
+    // it only once the lists are there: making them allocates.
+    const bool hermite = jonly && hermite_route(ctx);
+    if (hermite && cs == cudaStreamCaptureStatusNone) {
+        const int rc = ensure_jlists(ctx, st);
+        if (rc != PQB_OK) return rc;
+    }
+    if (hermite && ctx->jl.list) {
+        int rc = PQB_OK;
+        if (ctx->use_graph && cs == cudaStreamCaptureStatusNone && ctx->graph_warm[gi]) {
+            if (!ctx->graph_exec[gi])
+                rc = capture_graph(ctx, ctx->graph_exec[gi], [&](cudaStream_t c) { return launch_hermite(ctx, c); });
+            if (rc != PQB_OK) return rc;
+            PQB_CK(ctx, cudaGraphLaunch(ctx->graph_exec[gi], st));
+        } else {
+            rc = launch_hermite(ctx, st);
+            if (rc != PQB_OK) return rc;
+            if (cs == cudaStreamCaptureStatusNone) ctx->graph_warm[gi] = true;
+        }
+        PQB_CK(ctx, launch_hermite_fock((int)ctx->pairs.size(), ctx->d_pairs, ctx->d_prims, ctx->d_jfirst, ctx->jl.V, n,
+                                        ctx->d_escale, J[0], st));
+        return PQB_OK;
+    }
     if (ctx->use_graph && ctx->nmol == 1 && cs == cudaStreamCaptureStatusNone && ctx->graph_warm[gi]) {
         const int rc = ensure_build_graph(ctx, nden, jonly, mode, gi);
         if (rc != PQB_OK) return rc;
@@ -1912,7 +2117,13 @@ int pqb_jk_direct(pqb_ctx *ctx, const double *D, double *J, double *K, int mode,
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     const double *Dv[2] = {D, nullptr};
     double *Jv[2] = {J, nullptr}, *Kv[2] = {K, nullptr};
-    return jk_direct_impl(ctx, 1, Dv, Jv, Kv, mode, stream);
+    try {
+        return jk_direct_impl(ctx, 1, Dv, Jv, Kv, mode, stream);
+    } catch (const std::bad_alloc &) {
+        return fail(ctx, PQB_E_NOMEM, "pqb_jk_direct: host allocation failed");
+    } catch (...) {
+        return fail(ctx, PQB_E_STATE, "pqb_jk_direct: unexpected host exception");
+    }
 }
 
 static bool pageable(const void *p)
@@ -2006,7 +2217,13 @@ int pqb_jk_direct2(pqb_ctx *ctx, const double *Da, const double *Db, double *Ja,
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     const double *Dv[2] = {Da, Db};
     double *Jv[2] = {Ja, Jb}, *Kv[2] = {Ka, Kb};
-    return jk_direct_impl(ctx, 2, Dv, Jv, Kv, mode, stream);
+    try {
+        return jk_direct_impl(ctx, 2, Dv, Jv, Kv, mode, stream);
+    } catch (const std::bad_alloc &) {
+        return fail(ctx, PQB_E_NOMEM, "pqb_jk_direct2: host allocation failed");
+    } catch (...) {
+        return fail(ctx, PQB_E_STATE, "pqb_jk_direct2: unexpected host exception");
+    }
 }
 
 int pqb_set_molecule_mask(pqb_ctx *ctx, const int *mask)
@@ -2257,7 +2474,6 @@ static int set_shell_atoms_impl(pqb_ctx *ctx, const int *shell_atom)
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     // what pqb_grad_2e needs, so that it allocates nothing itself
     if (!ctx->d_gshell) PQB_CK(ctx, cudaMalloc(&ctx->d_gshell, sizeof(double) * 3 * ctx->nshell));
-    PQB_CK(ctx, ensure_streams(ctx));
     if (!ctx->d_shell_atom) PQB_CK(ctx, cudaMalloc(&ctx->d_shell_atom, sizeof(int) * ctx->nshell));
     PQB_CK(ctx, cudaMemcpy(ctx->d_shell_atom, shell_atom, sizeof(int) * ctx->nshell, cudaMemcpyHostToDevice));
     return PQB_OK;
@@ -2286,18 +2502,17 @@ static int grad_2e_impl(pqb_ctx *ctx, const double *D, double *grad, int mode, v
                                                          ctx->dense_len);
     PQB_CK(ctx, cudaMemsetAsync(ctx->d_gshell, 0, sizeof(double) * 3 * ctx->nshell, st));
     // highest angular momentum first: its items run longest
-    PQB_CK(ctx, cudaEventRecord(ctx->ev_fork, st));
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) PQB_CK(ctx, cudaStreamWaitEvent(ctx->streams[k], ctx->ev_fork, 0));
+    Fan fan(ctx, st);
+    PQB_CK(ctx, fan.fork(pqb_ctx::kStreams));
     for (int c = kNumQuartetClass - 1, k = 0; c >= 0; --c) {
         const int nq = (int)(ctx->plan_cnt[0][c] + ctx->plan_cnt[1][c]);
         if (nq == 0) continue;
-        PQB_CK(ctx, launch_grad(c, ctx->d_plan + ctx->plan_off[0][c], nq, ctx->d_pairs, ctx->d_prims, ctx->d_Dscaled,
-                                ctx->d_gshell, ctx->streams[k++ % pqb_ctx::kStreams], ctx->nsm));
+        PQB_CK(ctx, fan.run(k++, [&](cudaStream_t sk) {
+            return launch_grad(c, ctx->d_plan + ctx->plan_off[0][c], nq, ctx->d_pairs, ctx->d_prims, ctx->d_Dscaled,
+                               ctx->d_gshell, sk, ctx->nsm);
+        }));
     }
-    for (int k = 0; k < pqb_ctx::kStreams; ++k) {
-        PQB_CK(ctx, cudaEventRecord(ctx->ev_join[k], ctx->streams[k]));
-        PQB_CK(ctx, cudaStreamWaitEvent(st, ctx->ev_join[k], 0));
-    }
+    PQB_CK(ctx, fan.join());
     PQB_CK(ctx, launch_grad_gather(ctx->nshell, ctx->d_shell_atom, ctx->d_gshell, grad, st));
     return PQB_OK;
 }

@@ -567,3 +567,41 @@ def test_engine_rejects_bad_shapes():
         eng.ctx.check(eng.ctx.lib.pqb_jk_direct(eng.ctx.h, _lib.ptr(bad), _lib.ptr(bad), _lib.ptr(bad), 0,
                                                 _lib.stream_ptr()))
     assert ei.value.code == _lib.PQB_E_STATE
+
+
+@pytest.mark.parametrize("schwarz", [0.0, 1e-12, 1e-6])
+@pytest.mark.parametrize("mol,basis", [(geometries.water(), "sto-3g"), (geometries.water_cluster(2, seed=5), "6-31g**"),
+                                       (geometries.alkane(3), "6-31g*")])
+def test_hermite_coulomb_equals_the_full_builds_j(mol, basis, schwarz):
+    """The Coulomb-only build in the Hermite basis against J of the J/K build
+    on the same plan (the same quartets): one list block and several, every pair
+    class, first call, graph replay and a caller's capture; a sharded plan adds up
+    over its ranks.  Sums of up to 1e6 FP64 terms: 1e-12 of the largest element."""
+    bs = BasisSet(mol, basis)
+    eng = BasisEngine(bs.bfs)
+    eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_HERMITE, 0, 0))   # at any size
+    n = eng.nbf
+    g = torch.Generator().manual_seed(n)
+    D = torch.randn(n, n, generator=g, dtype=torch.float64)
+    D = (D + D.T).cuda().contiguous()
+    J, _ = eng.jk(D, schwarz=schwarz)
+    tol = 1e-12 * float(J.abs().max())
+    for _ in range(3):
+        assert float((eng.j(D, schwarz=schwarz) - J).abs().max()) < tol
+    assert float((eng.j(D, "mixed", schwarz=schwarz) - J).abs().max()) < tol
+    out = torch.empty_like(D)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        eng.j(D, schwarz=schwarz, J=out)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float((out - J).abs().max()) < tol
+    parts = torch.zeros_like(D)
+    for rank in range(2):
+        eng._plan_key = None
+        eng.plan(schwarz)
+        eng.ctx.check(eng.ctx.lib.pqb_plan_shard(eng.ctx.h, rank, 2))
+        parts += eng.j(D, schwarz=schwarz)
+    eng._plan_key = None
+    assert float((parts - J).abs().max()) < tol
