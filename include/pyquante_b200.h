@@ -221,12 +221,15 @@ int pqb_jk_direct_class(pqb_ctx *ctx, const double *D, double *Jacc, double *Kac
                         void *stream);
 
 /* AO -> MO transformation for MP2 (replaces the Python loops of
- * PyQuante/MP.py:20-75 TransformIntsMP2 and :77-97 MP2).  The quarter
- * transformations are FP64 GEMMs the caller runs (cuBLAS); these move the
- * data between them.  All pointers are device memory; no context.
+ * PyQuante/MP.py:20-75 TransformIntsMP2 and :77-97 MP2): the quarter
+ * transformations that read a packed index (the two others are FP64 GEMMs the
+ * caller runs), and the gathers and sums around them.  All pointers are
+ * device memory; no context.
  * pqb_mo_unpack_rows: out[r][k][l] = (IJ|kl) for the packed bra rows
  *   IJ = row0 .. row0+nrows-1 of the packed array ints (len = P(P+1)/2,
  *   P = nbf(nbf+1)/2): out holds nrows * nbf * nbf doubles.
+ * pqb_mo_contract_rows: out[(b*nrows + r)*nbf + l] =
+ *   sum_k C[k*nb + b] (row0 + r|kl), straight from the packed array.
  * pqb_mo_unpack_pairs: out[(mu*nbf + nu)*ncol + c] = Y[pair(mu,nu)*ncol + c]
  *   (rows stored per packed AO pair, unpacked to both orders).
  * pqb_mo_contract_pairs: out[((a*nbf + nu)*nb + b)*nj + j] =
@@ -238,6 +241,8 @@ int pqb_jk_direct_class(pqb_ctx *ctx, const double *D, double *Jacc, double *Kac
  * pqb_mp2_pairs: Epair[a*nocc + b] = sum_rs (ar|bs)(2(ar|bs) - (as|br)) /
  *   (e_a + e_b - e_r - e_s) from V[((a*nvirt + r)*nocc + b)*nvirt + s]. */
 int pqb_mo_unpack_rows(const double *ints, int64_t len, int nbf, int64_t row0, int nrows, double *out, void *stream);
+int pqb_mo_contract_rows(const double *ints, int64_t len, int nbf, int64_t row0, int nrows, const double *C, int nb,
+                         double *out, void *stream);
 int pqb_mo_unpack_pairs(const double *Y, int nbf, int64_t ncol, double *out, void *stream);
 int pqb_mo_contract_pairs(const double *Y, int nbf, int nb, int nj, const double *C, int na, double *out, void *stream);
 int pqb_mo_pack(const double *Z, int nocc, int nmo, double *moints, int64_t len, void *stream);

@@ -6,15 +6,14 @@
 ``Ints`` is the packed AO array of ``Ints.getints`` (a PackedInts, a torch
 tensor or an array).  The reference transforms one index at a time in
 Python loops, O(N^5) calls of ``dot``; here the four quarter transformations
-are FP64 matrix products on the GPU: three cuBLAS DGEMMs through torch and the
-engine's own contraction over one index of the packed AO pair
-(pqb_mo_contract_pairs), with the gather of the 8-fold packed order into
-dense rows (pqb_mo_unpack_rows) before and the pair energies
-(pqb_mp2_pairs) after them.  Everything is FP64: no reduced-precision
+are FP64 matrix products on the GPU: the first (pqb_mo_contract_rows) reads
+the 8-fold packed order as it is, the third (pqb_mo_contract_pairs) the packed
+AO pair, the second and fourth are cuBLAS DGEMMs through torch; the pair
+energies (pqb_mp2_pairs) follow.  Everything is FP64: no reduced-precision
 tensor-core path.
 
     1. (mu nu|sigma eta) -> (mu nu|b j): per batch of packed AO pairs mu >= nu,
-       unpack the rows and contract sigma with C[:, b], then eta with C[:, j]
+       contract sigma with C[:, b], then eta with C[:, j]
        (occupied b first: 2 P N^2 nocc operations instead of 2 P N^2 nvirt);
     2. (mu nu|b j) -> (a i|b j): contract mu with C[:, a] on the packed pair
        rows, then nu with C[:, i].
@@ -28,7 +27,7 @@ import torch
 from . import _lib
 from ._lib import ptr, stream_ptr
 
-# bytes of one batch of unpacked AO rows (N^2 doubles per row)
+# bytes of one batch of half-contracted AO rows (N nocc doubles per row)
 _ROW_BATCH_BYTES = 512 << 20
 
 
@@ -49,25 +48,21 @@ def _check(rc, what):
 def _half_transform(ints, nbf, Cb, Cj, stream=None):
     """Y[nb, P, nj] = (mu nu|b j) = sum_{sigma eta} Cb[sigma, b] Cj[eta, j]
     (mu nu|sigma eta) for every packed AO pair mu >= nu.  The occupied index
-    goes first: it is the smaller one, and both steps are then plain GEMMs of
-    tall matrices."""
+    goes first, straight from the packed order: it is the smaller one, and the
+    second step is then a plain GEMM."""
     lib = _lib.load()
     P = nbf * (nbf + 1) // 2
     nb, nj = Cb.shape[1], Cj.shape[1]
     Y = torch.empty((nb, P, nj), dtype=torch.float64, device=ints.device)
-    batch = max(1, min(P, _ROW_BATCH_BYTES // (8 * nbf * nbf)))
-    X = torch.empty((batch, nbf, nbf), dtype=torch.float64, device=ints.device)
+    batch = max(1, min(P, _ROW_BATCH_BYTES // (8 * nbf * max(nb, 1))))
     T = torch.empty(nb * batch * nbf, dtype=torch.float64, device=ints.device)
-    CbT = Cb.T.contiguous()
     Cjb = Cj.expand(nb, nbf, nj)
     for r0 in range(0, P, batch):
         nr = min(batch, P - r0)
-        Xb = X[:nr]
-        _check(lib.pqb_mo_unpack_rows(ptr(ints), ints.numel(), nbf, r0, nr, ptr(Xb), stream_ptr(stream)),
-               "pqb_mo_unpack_rows")
         T1 = T[:nb * nr * nbf]
-        torch.matmul(CbT, Xb.view(nr * nbf, nbf).T, out=T1.view(nb, nr * nbf))        # sigma -> b
-        torch.bmm(T1.view(nb, nr, nbf), Cjb, out=Y[:, r0:r0 + nr])                    # eta -> j
+        _check(lib.pqb_mo_contract_rows(ptr(ints), ints.numel(), nbf, r0, nr, ptr(Cb), nb, ptr(T1),
+                                        stream_ptr(stream)), "pqb_mo_contract_rows")    # sigma -> b
+        torch.bmm(T1.view(nb, nr, nbf), Cjb, out=Y[:, r0:r0 + nr])                      # eta -> j
     return Y
 
 

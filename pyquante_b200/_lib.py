@@ -66,6 +66,8 @@ SIGNATURES = {
                                    _c_dbl_p, _vp, _vp, _vp, _vp]),
     "pqb_mo_unpack_rows": (ctypes.c_int, [_vp, ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int, _vp, _vp]),
     "pqb_mo_unpack_pairs": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int64, _vp, _vp]),
+    "pqb_mo_contract_rows": (ctypes.c_int, [_vp, ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int, _vp,
+                                            ctypes.c_int, _vp, _vp]),
     "pqb_mo_contract_pairs": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, _vp, _vp]),
     "pqb_mo_pack": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int64, _vp]),
     "pqb_mp2_pairs": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp]),

@@ -139,3 +139,24 @@ def test_contract_pairs_at_tile_edges(n, nb, nj, na):
     full[:, j, i] = Y
     want = torch.einsum("ma,bmnj->anbj", C, full)
     assert float((out - want).abs().max()) < 1e-13 * n * float(want.abs().max().clamp(min=1.0))
+
+
+@pytest.mark.parametrize("n,nb,row0,nrows", [(1, 1, 0, 1), (7, 3, 2, 26), (8, 8, 0, 36), (9, 9, 44, 1), (25, 17, 3, 300),
+                                             (41, 16, 0, 861), (64, 70, 2000, 80), (150, 30, 11000, 325),
+                                             (199, 40, 19800, 100), (255, 1, 30000, 20), (289, 18, 41898, 7)])
+def test_contract_rows_at_tile_edges(n, nb, row0, nrows):
+    """Against the dense FP64 product of the unpacked rows: sums of n terms of
+    order one (1e-13 leaves a hundred roundings)."""
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    P = n * (n + 1) // 2
+    ints = torch.randn(P * (P + 1) // 2, generator=g, dtype=torch.float64, device="cuda")
+    C = torch.randn(n, nb, generator=g, dtype=torch.float64, device="cuda")
+    out = torch.full((nb, nrows, n), float("nan"), dtype=torch.float64, device="cuda")
+    assert lib.pqb_mo_contract_rows(_lib.ptr(ints), ints.numel(), n, row0, nrows, _lib.ptr(C), nb, _lib.ptr(out),
+                                    _lib.stream_ptr()) == _lib.PQB_OK
+    X = torch.empty(nrows, n, n, dtype=torch.float64, device="cuda")
+    assert lib.pqb_mo_unpack_rows(_lib.ptr(ints), ints.numel(), n, row0, nrows, _lib.ptr(X),
+                                  _lib.stream_ptr()) == _lib.PQB_OK
+    want = torch.einsum("kb,rkl->brl", C, X)
+    assert float((out - want).abs().max()) < 1e-13 * n * float(want.abs().max().clamp(min=1.0))
