@@ -575,7 +575,7 @@ def run_dft(a):
                       "data": "synthetic", "dtype": "f64",
                       "config": dict(out, workload=WORKLOAD, grid_points=npts, nbf=nbf, energy=e, scf_s=scf_s,
                                      bfgrid_bytes=8 * npts * nbf,
-                                     path="pqb_grid_amps/pqb_grid_rowdot/pqb_xc_svwn + cuBLAS DGEMM; "
+                                     path="pqb_grid_amps/pqb_grid_density/pqb_xc_svwn/pqb_grid_fock; "
                                           "pqb_jk_direct with K = NULL")}))
 
 

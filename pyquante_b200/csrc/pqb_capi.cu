@@ -545,7 +545,7 @@ __global__ void jk_packed_kernel(const double *__restrict__ ints, const double *
 //   Jacc[k,l] += 2 v' D_ij   per-warp partials in shared memory, summed
 //                            over the CTA's rows once per segment
 //   Kacc[i,l] += v' D_jk     register row accI[m] (lane-owned columns)
-//   Kacc[i,k] += v' D_jl     per-segment partials over 8 lane groups, parked
+//   Kacc[i,k] += v' D_jl     per-segment partials over 4 lane groups, parked
 //                            in a shared ring and folded into column k of
 //                            accI once per 32-segment block
 //   Kacc[j,l] += v' D_ik     register rows accJ[q][m]
@@ -554,7 +554,7 @@ __global__ void jk_packed_kernel(const double *__restrict__ ints, const double *
 constexpr int kRgWarps = 8, kRgRPW = 2, kRgRows = kRgWarps * kRgRPW, kRgPrefetch = 3;
 // segment-sum ring: kRgNv values (row i, rows j_q) x kRgParts partials x 32
 // columns, rows padded to 33 so that the writers hit distinct banks
-constexpr int kRgParts = 8;
+constexpr int kRgParts = 4;
 constexpr int kRgNv = 1 + kRgRPW, kRgRingPitch = 33, kRgRing = kRgNv * kRgParts * kRgRingPitch;
 
 __device__ __forceinline__ double warp_sum(double x)
@@ -593,76 +593,99 @@ __device__ __forceinline__ void rg_static_for(std::integer_sequence<int, Is...>,
     (f(std::integral_constant<int, Is>{}), ...);
 }
 
-// Jacc[k, l] for l <= k from the CTA's per-warp column partials of one
-// segment (one barrier per segment; the partials are double-buffered).
+// Jacc[k + s, l] for l <= k + s, s < NS, from the CTA's per-warp column partials
+// of those segments (one barrier per call; the partials are double-buffered).
+template <int NS>
 __device__ __forceinline__ void rg_column_sums(const double *jcb, int stride, double *Jacc, int n, int k)
 {
     __syncthreads();
-    for (int l = threadIdx.x; l <= k; l += kRgWarps * 32) {
-        double s = 0.0;
+    for (int l = threadIdx.x; l < k + NS; l += kRgWarps * 32) {
+        double s[NS];
 #pragma unroll
-        for (int w = 0; w < kRgWarps; ++w) s += jcb[w * stride + l];
-        if (s != 0.0) atomicAdd(Jacc + (int64_t)k * n + l, s);
+        for (int h = 0; h < NS; ++h) {
+            s[h] = 0.0;
+#pragma unroll
+            for (int w = 0; w < kRgWarps; ++w) s[h] += jcb[(h * kRgWarps + w) * stride + l];
+        }
+#pragma unroll
+        for (int h = 0; h < NS; ++h)
+            if (l <= k + h && s[h] != 0.0) atomicAdd(Jacc + (int64_t)(k + h) * n + l, s[h]);
     }
 }
 
-// Segment k (< i) of the warp's rows, k in [32 KB, 32 KB + 31]: the chunk
-// count KB + 1 and the register slot KB of column k are compile-time, so the
-// register rows stay in registers and the segment sums are plain adds.
-template <int MAXM, int KB>
-__device__ __forceinline__ void rg_segment(RgRows<MAXM> &r, const double *__restrict__ D, const double *Di,
-                                           double *jcw, double *ring, int n, int i, int k, int lane)
+// Segments k .. k + NS - 1 (< i) of the warp's rows, in [32 KB, 32 KB + 31]: the
+// chunk count KB + 1 and the register slot KB of these columns are compile-time,
+// so the register rows stay in registers and the segment sums are plain adds.
+// Two at a time share the loads of D_jl and D_il and a barrier: N = 60 78 -> 59
+// us, 150 304 -> 280, 200 680 -> 662, 300 3719 -> 2820, 380 7646 -> 6404.  Up to
+// eight register slots two blocks share an SM at 128 registers a thread, and the
+// pairs stop where theirs would spill (N = 200: 735 us with pairs throughout, 837
+// with one block an SM).
+constexpr int rg_paired_blocks(int maxm) { return maxm <= 6 ? 5 : maxm <= 8 ? 3 : maxm; }
+
+template <int MAXM, int KB, int NS>
+__device__ __forceinline__ void rg_segments(RgRows<MAXM> &r, const double *__restrict__ D, const double *Di,
+                                            double *jcw, int stride, double *ring, int n, int i, int k, int lane)
 {
-    const int KL0 = k * (k + 1) / 2;
     const double *Dk = D + (int64_t)k * n;
-    const double Dik = __ldg(Di + k);
-    double Djk[kRgRPW], kik[kRgRPW], kjk[kRgRPW];
+    double Dik[NS], Djk[NS][kRgRPW], kik[NS], kjk[NS][kRgRPW];
+    int KL0[NS];
 #pragma unroll
-    for (int q = 0; q < kRgRPW; ++q) {
-        Djk[q] = r.wq[q] * __ldg(r.Djp[q] + k);
-        kik[q] = 0.0;
-        kjk[q] = 0.0;
+    for (int h = 0; h < NS; ++h) {
+        KL0[h] = (k + h) * (k + h + 1) / 2;
+        Dik[h] = __ldg(Di + k + h);
+        kik[h] = 0.0;
+#pragma unroll
+        for (int q = 0; q < kRgRPW; ++q) {
+            Djk[h][q] = r.wq[q] * __ldg(r.Djp[q] + k + h);
+            kjk[h][q] = 0.0;
+        }
     }
 #pragma unroll
     for (int m = 0; m <= KB; ++m) {
         const int l = 32 * m + lane;
-        const bool inseg = m < KB || l <= k;
-        const double Dkl = inseg ? __ldg(Dk + l) : 0.0;
-        const double Dil = inseg ? __ldg(Di + l) : 0.0;
-        double jcol = 0.0;
+        const bool any = m < KB || l < k + NS;
+        const double Dil = any ? __ldg(Di + l) : 0.0;
+        double wDjl[kRgRPW];
 #pragma unroll
-        for (int q = 0; q < kRgRPW; ++q) {
-            const bool ok = r.okq[q] && inseg;
-            double v = ok ? __ldg(r.rowp[q] + KL0 + l) : 0.0;
-            const double Djl = ok ? __ldg(r.Djp[q] + l) : 0.0;
-            if (m == KB && l == k) v *= 0.5;
-            r.jrow[q] = fma(v, Dkl, r.jrow[q]);
-            jcol = fma(v, r.Dij2[q], jcol);
-            kik[q] = fma(v, Djl, kik[q]);
-            r.accI[m] = fma(v, Djk[q], r.accI[m]);
-            kjk[q] = fma(v, Dil, kjk[q]);
-            r.accJ[q][m] = fma(v, Dik, r.accJ[q][m]);
+        for (int q = 0; q < kRgRPW; ++q) wDjl[q] = any ? r.wq[q] * __ldg(r.Djp[q] + l) : 0.0;
+#pragma unroll
+        for (int h = 0; h < NS; ++h) {
+            const bool inseg = m < KB || l <= k + h;
+            const double Dkl = inseg ? __ldg(Dk + h * n + l) : 0.0;
+            double jcol = 0.0;
+#pragma unroll
+            for (int q = 0; q < kRgRPW; ++q) {
+                double v = r.okq[q] && inseg ? __ldg(r.rowp[q] + KL0[h] + l) : 0.0;
+                if (m == KB && l == k + h) v *= 0.5;
+                r.jrow[q] = fma(v, Dkl, r.jrow[q]);
+                jcol = fma(v, r.Dij2[q], jcol);
+                kik[h] = fma(v, wDjl[q], kik[h]);
+                r.accI[m] = fma(v, Djk[h][q], r.accI[m]);
+                kjk[h][q] = fma(v, Dil, kjk[h][q]);
+                r.accJ[q][m] = fma(v, Dik[h], r.accJ[q][m]);
+            }
+            jcw[h * kRgWarps * stride + l] = jcol;
         }
-        jcw[l] = jcol;
     }
     // the segment sums Kacc[i,k] (value 0) and Kacc[j_q,k] (value 1 + q):
     // butterfly levels down to kRgParts leave lane p < kRgParts with the sum
     // over lanes p + kRgParts t, parked in the warp's ring until the
     // 32-segment block is folded
-    double sv[kRgNv];
-    sv[0] = 0.0;
 #pragma unroll
-    for (int q = 0; q < kRgRPW; ++q) {
-        sv[0] = fma(r.wq[q], kik[q], sv[0]);
-        sv[1 + q] = kjk[q];
-    }
+    for (int h = 0; h < NS; ++h) {
+        double sv[kRgNv];
+        sv[0] = kik[h];
 #pragma unroll
-    for (int v = 0; v < kRgNv; ++v)
+        for (int q = 0; q < kRgRPW; ++q) sv[1 + q] = kjk[h][q];
 #pragma unroll
-        for (int o = 16; o >= kRgParts; o >>= 1) sv[v] += __shfl_xor_sync(0xffffffffu, sv[v], o);
-    if (lane < kRgParts) {
+        for (int v = 0; v < kRgNv; ++v)
 #pragma unroll
-        for (int v = 0; v < kRgNv; ++v) ring[(v * kRgParts + lane) * kRgRingPitch + (k & 31)] = sv[v];
+            for (int o = 16; o >= kRgParts; o >>= 1) sv[v] += __shfl_xor_sync(0xffffffffu, sv[v], o);
+        if (lane < kRgParts) {
+#pragma unroll
+            for (int v = 0; v < kRgNv; ++v) ring[(v * kRgParts + lane) * kRgRingPitch + ((k + h) & 31)] = sv[v];
+        }
     }
 }
 
@@ -751,20 +774,20 @@ __device__ __forceinline__ void rg_last_segment(RgRows<MAXM> &r, const double *_
 }
 
 template <int MAXM>
-__global__ void __launch_bounds__(kRgWarps * 32) jk_packed_reg_kernel(const double *__restrict__ ints,
+__global__ void __launch_bounds__(kRgWarps * 32, MAXM <= 8 ? 2 : 1) jk_packed_reg_kernel(const double *__restrict__ ints,
                                                                       const double *__restrict__ D, double *Jacc,
                                                                       double *Kacc, int n,
                                                                       const int2 *__restrict__ tiles, int ntiles)
 {
-    // column partials of a segment, double-buffered: jc[2][kRgWarps][MAXM * 32];
+    // column partials of two segments, double-buffered: jc[2][2][kRgWarps][MAXM * 32];
     // per-warp rows i, summed at the end: kis[kRgWarps][MAXM * 32]
     extern __shared__ double rg_smem[];
     constexpr int kStride = MAXM * 32;
     double *jc = rg_smem;
-    double(*kis)[kStride] = reinterpret_cast<double(*)[kStride]>(rg_smem + 2 * kRgWarps * kStride);
+    double(*kis)[kStride] = reinterpret_cast<double(*)[kStride]>(rg_smem + 4 * kRgWarps * kStride);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // per-warp ring of segment-sum partials: [value][partial p][column k % 32]
-    double *ring = rg_smem + 3 * kRgWarps * kStride + warp * kRgRing;
+    double *ring = rg_smem + 5 * kRgWarps * kStride + warp * kRgRing;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int i = tiles[t].x, j0 = tiles[t].y;
         const int64_t I0 = (int64_t)i * (i + 1) / 2;
@@ -802,22 +825,33 @@ __global__ void __launch_bounds__(kRgWarps * 32) jk_packed_reg_kernel(const doub
             constexpr int KB = decltype(kbc)::value;
             if (32 * KB >= i) return;
             const int kend = min(32 * KB + 31, i - 1);
-            for (int k = 32 * KB; k <= kend; ++k) {
-                if (pf_ok && k + kRgPrefetch <= i) {
-                    const int kk = k + kRgPrefetch;
-                    prefetch_l2(pf_row + kk * (kk + 1) / 2, kk < i ? kk + 1 : pf_j + 1);
+            int k = 32 * KB;
+            auto ahead = [&](int kk) {
+                if (pf_ok && kk <= i) prefetch_l2(pf_row + kk * (kk + 1) / 2, kk < i ? kk + 1 : pf_j + 1);
+            };
+            if constexpr (KB < rg_paired_blocks(MAXM)) {
+                for (; k < kend; k += 2) {
+                    ahead(k + kRgPrefetch);
+                    ahead(k + 1 + kRgPrefetch);
+                    double *jcb = jc + buf * 2 * kRgWarps * kStride;
+                    rg_segments<MAXM, KB, 2>(r, D, Di, jcb + warp * kStride, kStride, ring, n, i, k, lane);
+                    rg_column_sums<2>(jcb, kStride, Jacc, n, k);
+                    buf ^= 1;
                 }
-                double *jcb = jc + buf * kRgWarps * kStride;
-                rg_segment<MAXM, KB>(r, D, Di, jcb + warp * kStride, ring, n, i, k, lane);
-                rg_column_sums(jcb, kStride, Jacc, n, k);
+            }
+            for (; k <= kend; ++k) {
+                ahead(k + kRgPrefetch);
+                double *jcb = jc + buf * 2 * kRgWarps * kStride;
+                rg_segments<MAXM, KB, 1>(r, D, Di, jcb + warp * kStride, kStride, ring, n, i, k, lane);
+                rg_column_sums<1>(jcb, kStride, Jacc, n, k);
                 buf ^= 1;
             }
             rg_fold_block<MAXM, KB>(r, ring, kend, lane);
         });
         {
-            double *jcb = jc + buf * kRgWarps * kStride;
+            double *jcb = jc + buf * 2 * kRgWarps * kStride;
             rg_last_segment<MAXM>(r, D, Di, jcb + warp * kStride, n, i, lane);
-            rg_column_sums(jcb, kStride, Jacc, n, i);
+            rg_column_sums<1>(jcb, kStride, Jacc, n, i);
         }
 #pragma unroll
         for (int q = 0; q < kRgRPW; ++q) {
@@ -851,7 +885,7 @@ template <int MAXM>
 static cudaError_t launch_packed_reg(const double *ints, const double *D, double *J, double *K, int nbf,
                                      const int2 *tiles, int ntiles, int grid, cudaStream_t st)
 {
-    const size_t smem = sizeof(double) * (3 * kRgWarps * MAXM * 32 + kRgWarps * kRgRing);
+    const size_t smem = sizeof(double) * (5 * kRgWarps * MAXM * 32 + kRgWarps * kRgRing);
     cudaError_t e = cudaFuncSetAttribute(jk_packed_reg_kernel<MAXM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;

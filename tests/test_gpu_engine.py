@@ -311,6 +311,27 @@ def test_stored_register_kernel_every_row_width(n):
     torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 16, 17, 32, 33, 34, 65, 95, 97, 128, 129, 161, 193, 225, 257])
+def test_stored_register_kernel_segment_pairs(n):
+    """pqb_jk_packed's register kernel takes column segments in twos, with one
+    left over per block of 32 and the last of a row by itself: sizes either side
+    of those ends, against the one-block-per-row kernel (sums of up to n^2 products
+    of order one)."""
+    from pyquante_b200.engine import jk_packed
+    P = n * (n + 1) // 2
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ints = torch.rand(P * (P + 1) // 2, dtype=torch.float64, device="cuda", generator=g) - 0.5
+    Dt = torch.as_tensor(_rand_density(n, n), device="cuda")
+    ctx = _lib.Context(torch.cuda.current_device())
+    out = []
+    for simple in (1, 0):
+        ctx.check(ctx.lib.pqb_set_param(ctx.h, _lib.PQB_PARAM_PACKED_KERNEL, 0, simple))
+        out.append(jk_packed(ints, Dt, ctx))
+    scale = float(Dt.abs().sum())
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) < 1e-12 * scale * n
+
+
 def test_direct_build_graph_replay_matches_launches():
     """pqb_jk_direct replays a captured CUDA graph of its class launches from
     the second call per mode on; replays, one-by-one launches and a re-plan
