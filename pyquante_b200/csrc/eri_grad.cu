@@ -20,18 +20,21 @@
 // The components are those of the shells' common contraction: D is the
 // pre-scaled density D'_kl = r_k r_l D_kl of the Fock-build kernels, so Gamma
 // carries the four component scales.  The gradient is summed per shell
-// (3 nshell accumulators spread the atomics that 3 natoms would serialise)
-// and gathered to the atoms at the end.
+// in kGradCopies sets of 3 nshell accumulators, one set per block in turn, and
+// gathered to the atoms at the end.  A single set has every item of a build add
+// to the same few hundred numbers, one after the other in L2: C5H12 / 6-31G* 3.15
+// -> 1.46 ms, C10H22 / STO-3G 2.77 -> 0.96, C8H18 / 6-31G** 16.0 -> 10.1 with 64.
 //
 // Two splits (eri_grad_launch picks by the number of components):
 //  * up to 27 components: one thread per work item, everything in registers;
 //  * more: one warp per work item.  Lanes first share the (primitive quartet,
 //    root, axis) 2-D tables, which go to shared memory, then the (component,
 //    root) products.
-// A whole (H2O)4 / 6-31G* gradient takes 0.73 ms (60.6 ms with one thread per
-// item for every class, its tables and Gamma in local memory, and the classes
-// one after the other): 0.46 ms on the GPU, in which the items' serial chains
-// and the few high classes leave most of the chip idle.
+// (H2O)4 / 6-31G* takes 185 us on the GPU (0.31 ms with one set of sums; 50 ms
+// with one thread per item for every class, its tables and Gamma in local memory,
+// and the classes one after the other): the items' serial chains and the few high
+// classes leave most of the chip idle.  Four or eight lanes an item for up to 27
+// components: slower at every size (Gamma is then fetched by each).
 #include "eri_engine.cuh"
 #include "eri_launch.h"
 
@@ -52,8 +55,9 @@ template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) eri_grad_thread_kernel(const int4 *__restrict__ list, int nq,
                                                               const PairInfo *__restrict__ pairs,
                                                               const PrimPair *__restrict__ prims,
-                                                              const double *__restrict__ D, double *gshell)
+                                                              const double *__restrict__ D, double *gshell, int glen)
 {
+    gshell += (int64_t)(blockIdx.x % kGradCopies) * glen;   // this block's copy of the sums
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     constexpr int NR = (LA + LB + LC + LD + 1) / 2 + 1;
     constexpr int sD = 1, sC = (LD + 1) * sD, sB = (LC + 2) * sC, sA = (LB + 1) * sB, G2 = (LA + 2) * sA;
@@ -144,14 +148,15 @@ __global__ void __launch_bounds__(128) eri_grad_thread_kernel(const int4 *__rest
                     }
             }
         }
-        // ket shells: one atomic per lane; bra shells: one per warp while the
-        // warp holds one bra pair (the item order is bra-major)
-        if (count > 0) {
+        // last shell: one atomic per lane (neighbouring items differ in it); third:
+        // one per run of lanes that share it; bra shells: one per warp while the
+        // warp holds one bra pair (the item order is bra-major), else per run
+        const WarpRuns rbc(q.bra, q.sc, lane);
 #pragma unroll
-            for (int x = 0; x < 3; ++x) {
-                atomicAdd(gshell + 3 * q.sc + x, g9[6 + x]);
-                atomicAdd(gshell + 3 * q.sd + x, -(g9[x] + g9[3 + x] + g9[6 + x]));
-            }
+        for (int x = 0; x < 3; ++x) {
+            if (count > 0) atomicAdd(gshell + 3 * q.sd + x, -(g9[x] + g9[3 + x] + g9[6 + x]));
+            const double s = rbc.sum(g9[6 + x]);
+            if (rbc.last) atomicAdd(gshell + 3 * q.sc + x, s);
         }
         const int bra0 = __shfl_sync(0xffffffffu, q.bra, 0);
         const bool one_bra = __all_sync(0xffffffffu, bra0 == q.bra);
@@ -159,11 +164,15 @@ __global__ void __launch_bounds__(128) eri_grad_thread_kernel(const int4 *__rest
             int idx;
             const double s = warp_sum_transposed<6>(g9, lane, idx);
             if (idx < 6 && (lane & 3) == 0) atomicAdd(gshell + 3 * (idx < 3 ? q.sa : q.sb) + idx % 3, s);
-        } else if (count > 0) {
+        } else {
+            const WarpRuns rb(q.bra, 0, lane);
 #pragma unroll
             for (int x = 0; x < 3; ++x) {
-                atomicAdd(gshell + 3 * q.sa + x, g9[x]);
-                atomicAdd(gshell + 3 * q.sb + x, g9[3 + x]);
+                const double sa = rb.sum(g9[x]), sb = rb.sum(g9[3 + x]);
+                if (rb.last) {
+                    atomicAdd(gshell + 3 * q.sa + x, sa);
+                    atomicAdd(gshell + 3 * q.sb + x, sb);
+                }
             }
         }
     }
@@ -192,8 +201,9 @@ template <int LA, int LB, int LC, int LD> struct GradWarpLayout {
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(GradWarpLayout<LA, LB, LC, LD>::warps * 32)
 eri_grad_warp_kernel(const int4 *__restrict__ list, int nq, const PairInfo *__restrict__ pairs,
-                     const PrimPair *__restrict__ prims, const double *__restrict__ D, double *gshell)
+                     const PrimPair *__restrict__ prims, const double *__restrict__ D, double *gshell, int glen)
 {
+    gshell += (int64_t)(blockIdx.x % kGradCopies) * glen;   // this block's copy of the sums
     using Lay = GradWarpLayout<LA, LB, LC, LD>;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
     constexpr int NR = Lay::NR, NCOMP = Lay::NCOMP, PB = Lay::PB, PITCH = Lay::pitch, W = Lay::warps;
@@ -311,7 +321,10 @@ __global__ void grad_gather_kernel(int nshell, const int *__restrict__ shell_ato
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3 * nshell) return;
-    atomicAdd(grad + 3 * shell_atom[t / 3] + t % 3, gshell[t]);
+    double s = 0.0;
+#pragma unroll 16
+    for (int c = 0; c < kGradCopies; ++c) s += gshell[(int64_t)c * 3 * nshell + t];
+    atomicAdd(grad + 3 * shell_atom[t / 3] + t % 3, s);
 }
 
 cudaError_t launch_grad_gather(int nshell, const int *shell_atom, const double *gshell, double *grad, cudaStream_t st)
@@ -325,12 +338,12 @@ cudaError_t launch_grad_gather(int nshell, const int *shell_atom, const double *
 // mode; below, a warp's lanes would share too few products.
 template <int LA, int LB, int LC, int LD>
 static cudaError_t eri_grad_launch(const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                                   const double *D, double *gshell, cudaStream_t st, int nsm)
+                                   const double *D, double *gshell, int glen, cudaStream_t st, int nsm)
 {
     if constexpr (ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) <= 27) {
         int grid = (nq + 127) / 128;
         if (grid > nsm * 32) grid = nsm * 32;
-        eri_grad_thread_kernel<LA, LB, LC, LD><<<grid, 128, 0, st>>>(list, nq, pairs, prims, D, gshell);
+        eri_grad_thread_kernel<LA, LB, LC, LD><<<grid, 128, 0, st>>>(list, nq, pairs, prims, D, gshell, glen);
     } else {
         using Lay = GradWarpLayout<LA, LB, LC, LD>;
         auto kern = eri_grad_warp_kernel<LA, LB, LC, LD>;
@@ -338,19 +351,19 @@ static cudaError_t eri_grad_launch(const int4 *list, int nq, const PairInfo *pai
         if (e != cudaSuccess) return e;
         int grid = (nq + Lay::warps - 1) / Lay::warps;
         if (grid > nsm * 16) grid = nsm * 16;
-        kern<<<grid, Lay::warps * 32, Lay::bytes, st>>>(list, nq, pairs, prims, D, gshell);
+        kern<<<grid, Lay::warps * 32, Lay::bytes, st>>>(list, nq, pairs, prims, D, gshell, glen);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                        const double *Dscaled, double *gshell, cudaStream_t st, int nsm)
+                        const double *Dscaled, double *gshell, int nshell, cudaStream_t st, int nsm)
 {
     if (nq <= 0) return cudaSuccess;
 #define PQB_GCASE(CB, CK)                                                                                      \
     case CB *(CB + 1) / 2 + CK:                                                                               \
         return eri_grad_launch<pc_la(CB), pc_lb(CB), pc_la(CK), pc_lb(CK)>(list, nq, pairs, prims, Dscaled, gshell, \
-                                                                           st, nsm);
+                                                                           3 * nshell, st, nsm);
     switch (qc) {
         PQB_GCASE(0, 0)
         PQB_GCASE(1, 0) PQB_GCASE(1, 1)

@@ -62,9 +62,10 @@ cudaError_t launch_hermite_coulomb(int LP, int LQ, const JLists &l, double thres
 // first[pair]: offset of the pair's V
 cudaError_t launch_hermite_fock(int npair, const PairInfo *pairs, const PrimPair *prims, const int64_t *first,
                                 const double *V, int nbf, const double *escale, double *J, cudaStream_t st);
-// Adds dE2 per shell (gshell[3 nshell]) from the pre-scaled density; the
-// gather adds the shells to their atoms.
+// Adds dE2 per shell (gshell[kGradCopies][3 nshell], a block its copy) from the
+// pre-scaled density; the gather adds the copies and the shells to their atoms.
+constexpr int kGradCopies = 64;
 cudaError_t launch_grad(int qc, const int4 *list, int nq, const PairInfo *pairs, const PrimPair *prims,
-                        const double *Dscaled, double *gshell, cudaStream_t st, int nsm);
+                        const double *Dscaled, double *gshell, int nshell, cudaStream_t st, int nsm);
 cudaError_t launch_grad_gather(int nshell, const int *shell_atom, const double *gshell, double *grad, cudaStream_t st);
 }  // namespace pqb

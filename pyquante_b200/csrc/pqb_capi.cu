@@ -2507,7 +2507,7 @@ static int set_shell_atoms_impl(pqb_ctx *ctx, const int *shell_atom)
     if (!ctx->d_pairs) return fail(ctx, PQB_E_STATE, "pqb_set_shell_atoms: no basis uploaded");
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     // what pqb_grad_2e needs, so that it allocates nothing itself
-    if (!ctx->d_gshell) PQB_CK(ctx, cudaMalloc(&ctx->d_gshell, sizeof(double) * 3 * ctx->nshell));
+    if (!ctx->d_gshell) PQB_CK(ctx, cudaMalloc(&ctx->d_gshell, sizeof(double) * kGradCopies * 3 * ctx->nshell));
     if (!ctx->d_shell_atom) PQB_CK(ctx, cudaMalloc(&ctx->d_shell_atom, sizeof(int) * ctx->nshell));
     PQB_CK(ctx, cudaMemcpy(ctx->d_shell_atom, shell_atom, sizeof(int) * ctx->nshell, cudaMemcpyHostToDevice));
     return PQB_OK;
@@ -2534,7 +2534,7 @@ static int grad_2e_impl(pqb_ctx *ctx, const double *D, double *grad, int mode, v
     (void)mode;   // both lists in FP64: one launch per class over the class-major plan
     scale_elements_kernel<<<ctx->nsm * 4, 256, 0, st>>>(D, ctx->d_escale, ctx->d_Dscaled, ctx->d_Dscaled_f,
                                                          ctx->dense_len);
-    PQB_CK(ctx, cudaMemsetAsync(ctx->d_gshell, 0, sizeof(double) * 3 * ctx->nshell, st));
+    PQB_CK(ctx, cudaMemsetAsync(ctx->d_gshell, 0, sizeof(double) * kGradCopies * 3 * ctx->nshell, st));
     // highest angular momentum first: its items run longest
     Fan fan(ctx, st);
     PQB_CK(ctx, fan.fork(pqb_ctx::kStreams));
@@ -2543,7 +2543,7 @@ static int grad_2e_impl(pqb_ctx *ctx, const double *D, double *grad, int mode, v
         if (nq == 0) continue;
         PQB_CK(ctx, fan.run(k++, [&](cudaStream_t sk) {
             return launch_grad(c, ctx->d_plan + ctx->plan_off[0][c], nq, ctx->d_pairs, ctx->d_prims, ctx->d_Dscaled,
-                               ctx->d_gshell, sk, ctx->nsm);
+                               ctx->d_gshell, ctx->nshell, sk, ctx->nsm);
         }));
     }
     PQB_CK(ctx, fan.join());

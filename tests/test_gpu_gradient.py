@@ -120,3 +120,38 @@ def test_adjoint_kernels_vs_restated_reference_gradient(basis):
         eng = BasisEngine(bs.bfs)
     g = rhf_gradient_from_density(mol, eng, D, W, "fp64", 0.0)
     assert np.abs(g - go).max() < 1e-9, np.abs(g - go).max()
+
+
+@pytest.mark.parametrize("mol,basis", [(geometries.water(), "sto-3g"), (geometries.alkane(3), "6-31g*"),
+                                       (geometries.alkane(6), "sto-3g")])
+def test_two_electron_gradient_adds_up_over_shards(mol, basis):
+    """pqb_grad_2e of the whole plan against the sum over three ranks' shares,
+    whose item lists break the runs of equal pairs, the last warps and the blocks'
+    sets of sums elsewhere; up to 1e6 FP64 items: 1e-12 of the largest element."""
+    import ctypes
+
+    from pyquante_b200 import _lib
+    from pyquante_b200.engine import BasisEngine
+    from pyquante_b200.Ints import BasisSet
+    bs = BasisSet(mol, basis)
+    eng = BasisEngine(bs.bfs)
+    n, nat = eng.nbf, len(mol.atoms)
+    D = torch.randn(n, n, generator=torch.Generator().manual_seed(n), dtype=torch.float64)
+    D = (D + D.T).cuda().contiguous()
+    lib, h = eng.ctx.lib, eng.ctx.h
+    atom = np.arange(len(eng.shells["nprim"]), dtype=np.int32) % nat
+
+    def grad():
+        eng.ctx.check(lib.pqb_set_shell_atoms(h, atom.ctypes.data_as(ctypes.POINTER(ctypes.c_int))))
+        g = torch.zeros(3 * nat, dtype=torch.float64, device="cuda")
+        eng.ctx.check(lib.pqb_grad_2e(h, _lib.ptr(D), _lib.ptr(g), _lib.PQB_FP64, _lib.stream_ptr()))
+        return g
+
+    eng.plan()
+    whole, parts = grad(), 0.0
+    for rank in range(3):
+        eng._plan_key = None
+        eng.plan()
+        eng.ctx.check(lib.pqb_plan_shard(h, rank, 3))
+        parts = parts + grad()
+    assert float((whole - parts).abs().max()) < 1e-12 * float(whole.abs().max())
