@@ -311,6 +311,8 @@ struct EpiJKn {
         }
         return false;
     }
+    // this block's copy of the sums
+    __device__ __forceinline__ int64_t copy() const { return (int64_t)((int)blockIdx.x & scr.cmask) * scr.cstride; }
 
     // (called by every lane of the warp; a lane past the end of the item list
     // passes its neighbour's quartet with zero integrals)
@@ -355,7 +357,7 @@ struct EpiJKn {
             Db = Df[s] + q.bo;
         else
             Db = D[s] + q.bo;
-        double *Jb = Jacc[s] + q.bo, *Kb = Kacc[s] + q.bo;
+        double *Jb = Jacc[s] + q.bo + copy(), *Kb = Kacc[s] + q.bo + copy();
         // row bases in 64 bits, offsets within the few rows of a shell in 32
         const int nm = q.nm;
         const int64_t oa = (int64_t)q.fa * nm, ob = (int64_t)q.fb * nm, oc = (int64_t)q.fc * nm;
@@ -532,7 +534,7 @@ struct EpiJKn {
         for (int s = 0; s < NDEN; ++s) {
             const double *Db = D[s] + q.bo;
             const double *Da = Db + oa, *Dbr = Db + ob;
-            double *Jb = Jacc[s] + q.bo;
+            double *Jb = Jacc[s] + q.bo + copy();
             // Jacc[c,d] in the lane, Jacc[a,b] over the slot
             {
                 const double dcd = __ldg(Db + oc + q.fd + d);
@@ -557,7 +559,7 @@ struct EpiJKn {
                 __syncwarp();
             }
             if constexpr (!WITHK) continue;   // Coulomb only
-            double *Ka = Kacc[s] + q.bo + oa, *Kbr = Kacc[s] + q.bo + ob;
+            double *Ka = Kacc[s] + q.bo + copy() + oa, *Kbr = Kacc[s] + q.bo + copy() + ob;
             {
                 double dbd[NB], dbc[NB];
 #pragma unroll

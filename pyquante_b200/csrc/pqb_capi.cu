@@ -184,11 +184,33 @@ __global__ void shell_dmax_kernel(int nshell, const int4 *__restrict__ info, con
     if (lane == 0) dmax[s] = m;
 }
 
-// The graph path's epilogue: J and K (K2 == nullptr: J alone) from their
-// accumulators, which are left zeroed for the next replay of the build graph
-// (so the graph holds no memset nodes).
+// A[ij] + A[ji] over the copies (one or four), leaving them zeroed.  All loads
+// before the first store, which the compiler would otherwise keep behind it: four
+// round trips to L2 a matrix, 25 us at N = 95.
+constexpr int kAccCopies = 4;
+
+__device__ __forceinline__ double take_copies(double *A, int64_t ij, int64_t ji, int copies, int64_t stride)
+{
+    double v[kAccCopies], w[kAccCopies];
+#pragma unroll
+    for (int c = 0; c < kAccCopies; ++c) {
+        v[c] = c < copies ? A[c * stride + ij] : 0.0;
+        w[c] = c < copies ? A[c * stride + ji] : 0.0;
+    }
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kAccCopies; ++c) {
+        s += v[c] + w[c];
+        if (c < copies) A[c * stride + ij] = A[c * stride + ji] = 0.0;
+    }
+    return s;
+}
+
+// The graph path's epilogue: J and K (K2 == nullptr: J alone) from the copies
+// of their accumulators, which are left zeroed for the next replay of the build
+// graph (so the graph holds no memset nodes).
 __global__ void symmetrize_take_kernel(double *__restrict__ A1, double *__restrict__ M1, double *__restrict__ A2,
-                                       double *__restrict__ M2, int n, const double *__restrict__ S)
+                                       double *__restrict__ M2, int n, int copies, const double *__restrict__ S)
 {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t P = (int64_t)n * (n + 1) / 2;
@@ -199,15 +221,11 @@ __global__ void symmetrize_take_kernel(double *__restrict__ A1, double *__restri
     int j = (int)(t - (int64_t)i * (i + 1) / 2);
     const int64_t ij = (int64_t)i * n + j, ji = (int64_t)j * n + i;
     const double sc = S ? S[ij] : 1.0;
-    const double s1 = (A1[ij] + A1[ji]) * sc;
-    A1[ij] = 0.0;
-    A1[ji] = 0.0;
+    const double s1 = take_copies(A1, ij, ji, copies, (int64_t)n * n) * sc;
     M1[ij] = s1;
     M1[ji] = s1;
     if (A2) {
-        const double s2 = (A2[ij] + A2[ji]) * sc;
-        A2[ij] = 0.0;
-        A2[ji] = 0.0;
+        const double s2 = take_copies(A2, ij, ji, copies, (int64_t)n * n) * sc;
         M2[ij] = s2;
         M2[ji] = s2;
     }
@@ -217,7 +235,7 @@ __global__ void symmetrize_take_kernel(double *__restrict__ A1, double *__restri
 // symmetrised like symmetrize_take_kernel, which it replaces when the caller
 // wants G alone), leaving them zeroed.
 __global__ void take_2jmk_kernel(double *__restrict__ A1, double *__restrict__ A2, double *__restrict__ G, int n,
-                                 const double *__restrict__ S)
+                                 int copies, const double *__restrict__ S)
 {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t P = (int64_t)n * (n + 1) / 2;
@@ -228,11 +246,9 @@ __global__ void take_2jmk_kernel(double *__restrict__ A1, double *__restrict__ A
     int j = (int)(t - (int64_t)i * (i + 1) / 2);
     const int64_t ij = (int64_t)i * n + j, ji = (int64_t)j * n + i;
     const double sc = S ? S[ij] : 1.0;
-    const double g = fma(2.0, A1[ij] + A1[ji], -(A2[ij] + A2[ji])) * sc;
-    A1[ij] = 0.0;
-    A1[ji] = 0.0;
-    A2[ij] = 0.0;
-    A2[ji] = 0.0;
+    const int64_t nn = (int64_t)n * n;
+    const double sj = take_copies(A1, ij, ji, copies, nn), sk = take_copies(A2, ij, ji, copies, nn);
+    const double g = fma(2.0, sj, -sk) * sc;
     G[ij] = g;
     G[ji] = g;
 }
@@ -1850,6 +1866,15 @@ int pqb_eri_packed(pqb_ctx *ctx, double *out, int64_t len, void *stream)
     }
 }
 
+// Copies of the captured builds' accumulators (see ItemScreen): the atomics of
+// blocks that run side by side meet at the same rows of J and K, which four copies
+// spread.  Device time of a build with one / four: water / 6-31G** 58 / 52 us,
+// (H2O)8 / 6-31G** 326 / 303, mixed 307 / 281, C8H18 / 6-31G** 2111 / 2002, mixed
+// 1946 / 1828, C16H34 / 6-31G* (N = 308) 5200 / 5090, mixed 4790 / 4606; sixteen
+// give 1 % more.  One above N = 512, where the rows lie further apart and the
+// copies grow.
+static int acc_copies(const pqb_ctx *ctx) { return ctx->nmol == 1 && ctx->nbf <= 512 ? kAccCopies : 1; }
+
 // The class launches of one build into the accumulators Jacc[s], Kacc[s]
 // (zeroed here) of nden = 1 or 2 densities on stream st, forked over the
 // context's streams and joined back; they read the scaled densities
@@ -1868,7 +1893,11 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
     }
     const double *Ds[2] = {ctx->d_Dscaled, ctx->d_Dscaled2};
     const float *Dsf[2] = {ctx->d_Dscaled_f, ctx->d_Dscaled2_f};
-    const ItemScreen &mm = ctx->scr;
+    ItemScreen mm = ctx->scr;
+    if (!zero) {
+        mm.cmask = acc_copies(ctx) - 1;
+        mm.cstride = (int)ctx->dense_len;
+    }
     int order[2 * kNumQuartetClass];
     double cost[2 * kNumQuartetClass];
     for (int i = 0; i < 2 * kNumQuartetClass; ++i) {
@@ -1924,7 +1953,7 @@ static int ensure_acc_pair(pqb_ctx *ctx, double *&J, double *&K)
     free_dev(J);
     free_dev(K);
     J = K = nullptr;
-    const size_t bytes = sizeof(double) * std::max<long long>(ctx->dense_len, 1);
+    const size_t bytes = sizeof(double) * acc_copies(ctx) * std::max<long long>(ctx->dense_len, 1);
     cudaError_t e = cudaMalloc(&J, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&K, bytes);
     // zeroed once here; each use leaves them zeroed (symmetrize_take_kernel)
@@ -2115,13 +2144,14 @@ static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], doub
         PQB_CK(ctx, cudaGraphLaunch(ctx->graph_exec[gi], st));
         double *Ja[2] = {ctx->d_Jacc, ctx->d_Jacc2}, *Ka[2] = {ctx->d_Kacc, ctx->d_Kacc2};
         if (G) {
-            take_2jmk_kernel<<<(unsigned)((P + 255) / 256), 256, 0, st>>>(Ja[0], Ka[0], G, n, ctx->d_escale);
+            take_2jmk_kernel<<<(unsigned)((P + 63) / 64), 64, 0, st>>>(Ja[0], Ka[0], G, n, acc_copies(ctx),
+                                                                             ctx->d_escale);
             PQB_CK(ctx, cudaGetLastError());
             return PQB_OK;
         }
         for (int s = 0; s < nden; ++s)
-            symmetrize_take_kernel<<<(unsigned)((P + 255) / 256), 256, 0, st>>>(
-                Ja[s], J[s], jonly ? nullptr : Ka[s], jonly ? nullptr : K[s], n, ctx->d_escale);
+            symmetrize_take_kernel<<<(unsigned)((P + 63) / 64), 64, 0, st>>>(
+                Ja[s], J[s], jonly ? nullptr : Ka[s], jonly ? nullptr : K[s], n, acc_copies(ctx), ctx->d_escale);
         PQB_CK(ctx, cudaGetLastError());
         return PQB_OK;
     }
@@ -2189,8 +2219,8 @@ static int get2jmk_pageable(pqb_ctx *ctx, const double *D_host, double *G_host, 
             const int r = launch_build(ctx, 1, Ja, Ka, mode, cs, false);
             if (r != PQB_OK) return r;
             const int64_t P = (int64_t)n * (n + 1) / 2;
-            take_2jmk_kernel<<<(unsigned)((P + 255) / 256), 256, 0, cs>>>(ctx->d_Jacc, ctx->d_Kacc, ctx->d_hG, n,
-                                                                          ctx->d_escale);
+            take_2jmk_kernel<<<(unsigned)((P + 63) / 64), 64, 0, cs>>>(ctx->d_Jacc, ctx->d_Kacc, ctx->d_hG, n,
+                                                                          acc_copies(ctx), ctx->d_escale);
             PQB_CK(ctx, cudaGetLastError());
             PQB_CK(ctx, cudaMemcpyAsync(ctx->h_G, ctx->d_hG, bytes, cudaMemcpyDeviceToHost, cs));
             return (int)PQB_OK;

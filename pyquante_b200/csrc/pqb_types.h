@@ -19,12 +19,17 @@ constexpr int kNumQuartetClass = 21;             // bra class >= ket class
 //            its molecule's block); an item (ab|cd) is skipped when
 //            Q_ab Q_cd max(dmax[a], dmax[b], dmax[c], dmax[d]) < tau, Q the
 //            Schwarz factors (the incremental builds of a batched SCF digest
-//            density differences, most of which are small).
+//            density differences, most of which are small);
+// and where their sums go:
+//   cmask, cstride: block b adds to the copy b & cmask of Jacc and Kacc, cstride
+//            numbers apart (0: there is one).
 struct ItemScreen {
     const int *molmask;
     const double *dmax;
     const double *Qpair;
     double tau;
+    int cmask;
+    int cstride;
 };
 
 struct PairInfo {

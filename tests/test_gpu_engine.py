@@ -311,6 +311,25 @@ def test_stored_register_kernel_every_row_width(n):
     torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("mol,basis", [(geometries.water(), "sto-3g"), (geometries.water_cluster(3, seed=2), "6-31g**"),
+                                       (geometries.alkane(27), "6-31g*")])
+def test_replayed_builds_leave_every_copy_of_the_sums_zeroed(mol, basis):
+    """Replayed builds add into four copies of J and K up to N = 512 and into one
+    above: replays in turn of J and K, and of J alone by the same class kernels,
+    equal the first, launched build."""
+    bs = BasisSet(mol, basis)
+    n = len(bs)
+    eng = BasisEngine(bs.bfs)
+    eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_HERMITE, 0, 2**31 - 1))
+    D = torch.as_tensor(_rand_density(n, 5), device="cuda")
+    J, K = eng.jk(D, schwarz=1e-8)
+    tol = 1e-12 * max(float(J.abs().max()), float(K.abs().max()))
+    for _ in range(3):
+        Jr, Kr = eng.jk(D, schwarz=1e-8)
+        assert float((Jr - J).abs().max()) < tol and float((Kr - K).abs().max()) < tol
+        assert float((eng.j(D, schwarz=1e-8) - J).abs().max()) < tol
+
+
 @pytest.mark.parametrize("n", [1, 2, 3, 16, 17, 32, 33, 34, 65, 95, 97, 128, 129, 161, 193, 225, 257])
 def test_stored_register_kernel_segment_pairs(n):
     """pqb_jk_packed's register kernel takes column segments in twos, with one
