@@ -86,11 +86,15 @@ def _oracle_table(bs):
     return O, O.Table([O.BF(bf.origin, bf.powers, list(zip(bf.pexps, bf.pcoefs))) for bf in bs.bfs])
 
 
+REF_FOCK = os.path.join(ROOT, "oracle", "_ref", "ref_fock")
+NO_REF_FOCK = "oracle/_ref/ref_fock is not built (the reference's sources were not there at build time)"
+
+
 def reference_rate(bs, seconds, seed=0, nproc=None):
     """Quartets/s of the reference's compiled Rys engine (ref_fock, forked
     workers over bra rows) on a bounded random sample of bra rows."""
     O, tab = _oracle_table(bs)
-    exe = os.path.join(ROOT, "oracle", "_ref", "ref_fock")
+    exe = REF_FOCK
     if not os.path.exists(exe):
         raise RuntimeError("oracle/_ref/ref_fock not built (make -C oracle ref)")
     nproc = nproc or os.cpu_count() or 1
@@ -165,6 +169,9 @@ def reference_full_steps(nproc):
 def run_reference(a):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    if not os.path.exists(REF_FOCK):
+        print(json.dumps({"impl": "reference", "unavailable": NO_REF_FOCK}))
         return
     from pyquante_b200.Basis.basis import BasisSet
     bs = BasisSet(molecule(), "6-31g**")
@@ -618,7 +625,7 @@ def main():
     n = len(bs)
     Q = nominal_quartets(n)
     cpu = None
-    if rank == 0 and world == 1 and not a.no_cpu_baseline:
+    if rank == 0 and world == 1 and not a.no_cpu_baseline and os.path.exists(REF_FOCK):
         # before any CUDA work in this process: the baseline forks workers
         cpu = reference_rate(bs, a.cpu_seconds)
     from pyquante_b200.parallel import allreduce_jk, shard_plan
@@ -849,7 +856,7 @@ def main():
                          "traffic_note": "DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) summed over "
                                          "the class launches of one FP64 build of this workload; the build is "
                                          "L2-resident, so the FP64 pipe, not HBM, is the roofline",
-                         "kernel": "eri_thread_kernel/eri_block_kernel<class, EpiJK>: all class instantiations "
+                         "kernel": "eri_thread_kernel/eri_warp_kernel<class, EpiJK>: all class instantiations "
                                    "of one FP64 Fock build, launched together by pqb_jk_direct",
                          "flops_per_build": tot_fl, "flop_model": "pyquante_b200.flops (per-class counts of the "
                                                                    "kernels' FP64 operations, FMA = 2)",
@@ -880,6 +887,8 @@ def main():
                                     "kind": "reference",
                                     "sample": "%d quartets (%d random bra rows, all kl >= ij) in %.1f s" % (
                                         cpu["quartets"], cpu["rows"], cpu["seconds"])}
+        elif not os.path.exists(REF_FOCK):
+            line["cpu_baseline"] = {"unavailable": NO_REF_FOCK}
         line["per_class_fp64"] = [dict(cls="%d%d|%d%d" % r["cls"], part=r["part"], ms=round(r["ms"], 4),
                                        tflops=round(r["tflops"], 3), items=r["items"], prims=r["prims"])
                                   for r in sorted(per_class, key=lambda r: -r["ms"])]

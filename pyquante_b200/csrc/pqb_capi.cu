@@ -1255,7 +1255,7 @@ int pqb_last_error(const pqb_ctx *ctx, char *buf, size_t len)
 int pqb_num_pairs(const pqb_ctx *ctx) { return ctx ? (int)ctx->pairs.size() : 0; }
 
 // Bucket work items by class.  Within a class the items go by descending
-// primitive-quartet count (block-mode kernels advance their items in lockstep
+// primitive-quartet count (warp-mode kernels advance their items in lockstep
 // over primitive quartets; thread-mode warps get similar trip counts), then by
 // bra pair, then in generation order (ket pair ascending), so neighbouring
 // lanes share the bra and often the ket's first shell and the J/K epilogue's
