@@ -473,6 +473,10 @@ def _scf(mol, bs, precision, solver="eigh"):
             Counting.builds += 1
             return super().jk(D)
 
+        def get2jmk_host(self, D, G, stream=None):
+            Counting.builds += 1
+            return super().get2jmk_host(D, G, stream)
+
     from pyquante_b200.Ints import _engine_for, get1ints
     eng = _engine_for(bs)
     S, h = get1ints(bs, mol)

@@ -43,7 +43,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 # classes whose thread-mode kernels use the generated routines: every class
-# with LA+LB+LC+LD <= 4 (the block-mode classes keep the Rys quadrature)
+# with LA+LB+LC+LD <= 4 (the warp-mode classes keep the Rys quadrature)
 OS_CLASSES = [(0, 0, 0, 0), (1, 0, 0, 0), (1, 1, 0, 0), (1, 0, 1, 0), (2, 0, 0, 0), (1, 1, 1, 0), (2, 0, 1, 0),
               (2, 1, 0, 0), (1, 1, 1, 1), (2, 0, 1, 1), (2, 0, 2, 0), (2, 1, 1, 0), (2, 2, 0, 0)]
 

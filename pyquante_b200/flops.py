@@ -19,7 +19,7 @@ Obara--Saika classes (LA+LB+LC+LD = LT <= 4, csrc/os_classes.inc):
             (PA, QC, WP, WQ components, rho/zeta, rho/eta, the 1/(2x) factors;
             gen_os.class_flops)
   per item  the emitted horizontal transfer, plus the J/K digestion
-Rys classes (the block-mode classes, 3+ roots):
+Rys classes (the warp-mode classes, 3+ roots):
   roots     NR roots x 2 series (root, weight) x Clenshaw(14 coef): 13 x (FMA+sub)
             + final (FMA+sub)                                     = 84 / root
   setup     T, prefactor: 20
