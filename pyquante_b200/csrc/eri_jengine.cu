@@ -214,8 +214,7 @@ __device__ __forceinline__ void boys_any(double T, double *F)
     } else {
         constexpr int M0 = L <= 1 ? 0 : L - 1, ROW = L <= 1 ? 8 : 12;   // lowest order of the series; row part read
         const bool big = T >= PQB_BOYS_TMAX;
-        int k = __double2int_rn(T * PQB_BOYS_STEP_INV);
-        k = k < (int)(PQB_BOYS_TMAX * PQB_BOYS_STEP_INV) ? k : (int)(PQB_BOYS_TMAX * PQB_BOYS_STEP_INV);
+        const int k = boys_row_index(T * PQB_BOYS_STEP_INV, (int)(PQB_BOYS_TMAX * PQB_BOYS_STEP_INV));
         const double d = fma(k, 1.0 / PQB_BOYS_STEP_INV, -T);
         const double *row = pqb_boys_tab + k * PQB_BOYS_NORD;
         double f[ROW + 1];

@@ -158,7 +158,7 @@ __device__ __forceinline__ void ld4(const double *p, double &a, double &b, doubl
 //     the term is below 1e-30 of F_m) is exact enough.
 // Every lane evaluates both forms (the table row index is clamped) and keeps
 // one.  T must be non-negative and below 1e36 (exponent sums times squared
-// distances of a molecule).  Against the 40-digit values: below 2e-15
+// distances of a molecule), or NaN, which gives NaN.  Against the 40-digit values: below 2e-15
 // relative.
 __device__ __forceinline__ double rsqrt_nr_unchecked(double x)
 {
@@ -182,13 +182,28 @@ __device__ __forceinline__ void ld2(const double *p, double &a, double &b)
     asm("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(__cvta_generic_to_global(p)));
 }
 
+// The table row nearest to t = T / step >= 0, at most `last`.  The minimum is one
+// of unsigned numbers: a NaN, as a NaN coordinate gives, converts to INT_MIN from
+// a double (to 0 from a float), which as a signed number would pass an upper bound
+// and read far in front of the table.
+__device__ __forceinline__ int boys_row_index(double t, int last)
+{
+    const unsigned k = (unsigned)__double2int_rn(t);
+    return (int)(k < (unsigned)last ? k : (unsigned)last);
+}
+
+__device__ __forceinline__ int boys_row_index(float t, int last)
+{
+    const unsigned k = (unsigned)__float2int_rn(t);
+    return (int)(k < (unsigned)last ? k : (unsigned)last);
+}
+
 template <int NF>
 __device__ __forceinline__ void boys_row1(double T, double *F)
 {
     static_assert(NF == 1 || NF == 2, "F_0 or F_0, F_1");
     const bool big = T >= PQB_BOYSROW_TMAX;
-    int k = __double2int_rn(T * PQB_BOYSROW_STEP_INV);
-    k = k < PQB_BOYSROW_NGRID - 1 ? k : PQB_BOYSROW_NGRID - 1;
+    const int k = boys_row_index(T * PQB_BOYSROW_STEP_INV, PQB_BOYSROW_NGRID - 1);
     const double Tk = k * (1.0 / PQB_BOYSROW_STEP_INV), d = Tk - T, t2 = 2.0 * Tk;
     double f[8], ek;
     ld2(pqb_boys_top7 + 2 * k, f[7], ek);
@@ -215,8 +230,7 @@ __device__ __forceinline__ void boys_rowm(double T, double *F)
 {
     static_assert(M == 3 || M == 4, "F_M .. F_(M+6) from F_10");
     const bool big = T >= PQB_BOYSROW_TMAX;
-    int k = __double2int_rn(T * PQB_BOYSROW_STEP_INV);
-    k = k < PQB_BOYSROW_NGRID - 1 ? k : PQB_BOYSROW_NGRID - 1;
+    const int k = boys_row_index(T * PQB_BOYSROW_STEP_INV, PQB_BOYSROW_NGRID - 1);
     const double Tk = k * (1.0 / PQB_BOYSROW_STEP_INV), d = Tk - T, tk2 = 2.0 * Tk;
     double f[11], ek;
     ld2(pqb_boys_top10 + 2 * k, f[10], ek);
@@ -301,8 +315,7 @@ __device__ __forceinline__ void boys_os_f32(float T, float *F)
 {
     static_assert(LT <= 4, "up to F_4");
     const bool big = T >= (float)PQB_BOYSROW_TMAX;
-    int k = __float2int_rn(T * PQB_BOYSROW_STEP_INV);
-    k = k < PQB_BOYSROW_NGRID - 1 ? k : PQB_BOYSROW_NGRID - 1;
+    const int k = boys_row_index(T * (float)PQB_BOYSROW_STEP_INV, PQB_BOYSROW_NGRID - 1);
     const float Tk = k * (1.0f / PQB_BOYSROW_STEP_INV), d = Tk - T, tk2 = 2.0f * Tk;
     float f[8], ek;
     ld2f(pqb_boys_top7_f32 + 2 * k, f[7], ek);

@@ -64,3 +64,35 @@ def test_the_rule_catches_both_known_shapes():
     assert not _guarded_collectives("if (__all_sync(0xffffffffu, skip || !live)) continue")
     assert not _guarded_collectives("const long long kn = __shfl_down_sync(0xffffffffu, key, 1)")
     assert not _guarded_collectives("v += __shfl_xor_sync(0xffffffffu, v, o)")
+
+
+# A double that is converted to a table index: a NaN (a NaN coordinate, say)
+# becomes INT_MIN, which `k < last ? k : last` lets through.  So the conversion
+# is either clamped as an unsigned number or made where a comparison that NaN
+# fails has let it through.
+INDEX_CONVERSION = re.compile(r"__(double|float)2int_r[nzud]\s*\(|\(int\)\s*T\b")
+
+
+def _unclamped_conversions(src):
+    out, before = [], ""
+    for stmt, line in _statements(_strip(src)):
+        if INDEX_CONVERSION.search(stmt):
+            clamped = re.search(r"\bunsigned\s+k\s*=\s*\(unsigned\)\s*__(double|float)2int", stmt)
+            if not clamped and not re.search(r"\bif\s*\(\s*T\s*<\s*[\w\[\]]+\s*\)\s*$", before):
+                out.append(line)
+        before = stmt
+    return out
+
+
+def test_a_nan_stays_inside_every_table():
+    bad = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        bad += ["%s:%d" % (os.path.basename(path), line) for line in _unclamped_conversions(open(path).read())]
+    assert not bad, "table indices that a NaN takes out of range:\n" + "\n".join(bad)
+
+
+def test_the_table_rule_tells_the_shapes_apart():
+    assert _unclamped_conversions("int k = __double2int_rn(T * 16); k = k < 640 ? k : 640;")
+    assert _unclamped_conversions("if (T > 0) { const int iv = (int)T; }")
+    assert not _unclamped_conversions("if (T < tmax[n]) { const int iv = (int)T; }")
+    assert not _unclamped_conversions("{ const unsigned k = (unsigned)__double2int_rn(t); return min(k, last); }")
