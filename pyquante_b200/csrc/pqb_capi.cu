@@ -55,6 +55,7 @@ struct pqb_ctx {
     std::vector<PairInfo> pairs;
     std::vector<double> Q;           // Schwarz factors (host)
     bool have_q = false;
+    bool q_finite = false;           // every Schwarz factor is a finite number
     // unscreened lists (packed integrals): per class offset/count into d_full
     int4 *d_full = nullptr;
     int64_t full_off[kNumQuartetClass] = {0}, full_cnt[kNumQuartetClass] = {0}, full_long[kNumQuartetClass] = {0};
@@ -1512,6 +1513,7 @@ static int schwarz_impl(pqb_ctx *ctx, double *Q_host, void *stream)
     if (ctx->scr.dmax) ctx->scr.Qpair = dQ;
     if (e != cudaSuccess) return fail(ctx, PQB_E_CUDA, "pqb_schwarz: %s", cudaGetErrorString(e));
     ctx->have_q = true;
+    ctx->q_finite = std::all_of(ctx->Q.begin(), ctx->Q.end(), [](double q) { return std::isfinite(q); });
     if (Q_host) memcpy(Q_host, ctx->Q.data(), sizeof(double) * np);
     return PQB_OK;
 }
@@ -1992,9 +1994,13 @@ static int ensure_build_graph(pqb_ctx *ctx, int nden, bool jonly, int mode, int 
 //   254;  C8H18 6-31G* 9.9 M 617 / 885, 6-31G** 12.8 M 916 / 1561.
 // With s and p alone the class kernels stay ahead at every size (STO-3G: C8H18
 // 185 / 157, C20H42 1113 / 1097).
+// The lists are sorted by the Schwarz factors and cut where a product falls below
+// the threshold, which a NaN never does: with factors that are not finite (a
+// coordinate that is not) the plan's lists serve, which keep such quartets.
 static bool hermite_route(const pqb_ctx *ctx)
 {
-    if (ctx->nmol != 1 || ctx->sharded || ctx->scr.molmask || ctx->scr.dmax || !ctx->have_q) return false;
+    if (ctx->nmol != 1 || ctx->sharded || ctx->scr.molmask || ctx->scr.dmax || !ctx->have_q || !ctx->q_finite)
+        return false;
     constexpr int kFirstD = 6;   // classes 0 .. 5 are those of ss, ps and pp pairs
     int64_t prims = 0;
     for (int part = 0; part < 2; ++part)

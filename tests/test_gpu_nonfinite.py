@@ -6,7 +6,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from pyquante_b200 import Ints, geometries  # noqa: E402
+from pyquante_b200 import Ints, _lib, geometries  # noqa: E402
 from pyquante_b200.Basis.basis import BasisSet  # noqa: E402
 from pyquante_b200.engine import BasisEngine  # noqa: E402
 from pyquante_b200.force import rhf_gradient_from_density  # noqa: E402
@@ -44,3 +44,15 @@ def test_two_electron_matrices_and_gradient(lost, mode):
     g = rhf_gradient_from_density(mol, eng, D, D, precision=mode)
     assert np.isnan(g).all()
     assert bool(eng.eri_packed().isnan().any())
+
+
+def test_coulomb_matrix_in_the_hermite_basis(lost):
+    """The Hermite lists are sorted and cut by the Schwarz factors, which are
+    NaN here: the quartets that the plan keeps must not be lost."""
+    _, bs, _ = lost
+    eng = BasisEngine(bs.bfs)
+    eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_HERMITE, 0, 0))   # at any size
+    D = torch.eye(eng.nbf, dtype=torch.float64, device=eng.device) + 0.1
+    assert np.isnan(eng.schwarz()).any()
+    for _ in range(3):
+        assert bool(eng.j(D).isnan().all())
