@@ -114,16 +114,30 @@ class MolecularGrid:
 
     set_bf_amps = add_basis
 
-    def _work(self):
-        return torch.empty(_lib.load().pqb_grid_work(self.ng, self.nbf), dtype=torch.float64, device=self.device)
+    def _work(self, n):
+        return torch.empty(_lib.load().pqb_grid_work(self.ng, n), dtype=torch.float64, device=self.device)
+
+    def _amplitudes(self, what, n):
+        """bfgrid as the kernels read it: FP64 rows of n on the grid's device."""
+        B = self.bfgrid
+        if B is None or tuple(B.shape) != (self.ng, n):
+            raise RuntimeError("%s: no basis amplitudes on this grid (add_basis first)" % what)
+        if B.dtype != torch.float64 or B.device != self.device:
+            raise RuntimeError("%s: the amplitudes are %s on %s, not float64 on %s" % (what, B.dtype, B.device, self.device))
+        return B.contiguous()
 
     def set_density(self, D, Db=None):
         """density[:, 0] = sum_ij B_gi D_ij B_gj; density[:, 1] the same for
         Db (or a copy of the first column)."""
         lib, n = _lib.load(), self.nbf
-        if self.bfgrid is None or tuple(self.bfgrid.shape) != (self.ng, n):
-            raise RuntimeError("set_density: no basis amplitudes on this grid (add_basis first)")
-        B, work = self.bfgrid.contiguous(), self._work()
+        B, work = self._amplitudes("set_density", n), self._work(n)
+        # (the kernel writes rows of two doubles; a density of another layout that a
+        # caller has put in their place is filled from them)
+        rho = self.density
+        direct = rho.dtype == torch.float64 and rho.device == self.device and tuple(rho.shape) == (self.ng, 2) \
+            and rho.is_contiguous()
+        if not direct:
+            rho = torch.empty((self.ng, 2), dtype=torch.float64, device=self.device)
         for col, M in ((0, D), (1, Db)):
             if M is None:
                 continue
@@ -131,19 +145,23 @@ class MolecularGrid:
                                  device=self.device).contiguous()
             if tuple(Mt.shape) != (n, n):
                 raise RuntimeError("set_density: the density is %s, the basis has %d functions" % (tuple(Mt.shape), n))
-            _check(lib.pqb_grid_density(self.ng, n, ptr(B), ptr(Mt), ptr(self.density[:, col:]), 2,
+            _check(lib.pqb_grid_density(self.ng, n, ptr(B), ptr(Mt), ptr(rho[:, col:]), 2,
                                         2 if col == 0 and Db is None else 1, ptr(work), stream_ptr()),
                    "pqb_grid_density")
+        if not direct:
+            self.density[:, 0] = rho[:, 0]
+            self.density[:, 1] = rho[:, 1]
 
     def fock(self, v):
         """F_ij = sum_g B_gi v_g B_gj for a vector v over the points."""
-        B, v = self.bfgrid.contiguous(), v.contiguous()
         n = self.nbf
-        if tuple(B.shape) != (self.ng, n) or tuple(v.shape) != (self.ng,):
-            raise RuntimeError("fock: amplitudes %s and values %s do not match the grid's %d points"
-                               % (tuple(B.shape), tuple(v.shape), self.ng))
+        B = self._amplitudes("fock", n)
+        if tuple(v.shape) != (self.ng,) or v.dtype != torch.float64 or v.device != self.device:
+            raise RuntimeError("fock: %s values of %s on %s do not match the grid's %d points on %s"
+                               % (tuple(v.shape), v.dtype, v.device, self.ng, self.device))
+        v = v.contiguous()
         F = torch.empty((n, n), dtype=torch.float64, device=self.device)
-        work = self._work()
+        work = self._work(n)
         _check(_lib.load().pqb_grid_fock(self.ng, n, ptr(B), ptr(v), ptr(F), ptr(work), stream_ptr()),
                "pqb_grid_fock")
         return F
