@@ -153,8 +153,9 @@ class MolecularGrid:
             self.density[:, 1] = rho[:, 1]
 
     def fock(self, v):
-        """F_ij = sum_g B_gi v_g B_gj for a vector v over the points."""
-        n = self.nbf
+        """F_ij = sum_g B_gi v_g B_gj for a vector v over the points (of the
+        amplitudes' own width: they may be a caller's, with no basis added)."""
+        n = self.nbf if self.bfgrid is None or self.bfgrid.dim() != 2 else self.bfgrid.shape[1]
         B = self._amplitudes("fock", n)
         if tuple(v.shape) != (self.ng,) or v.dtype != torch.float64 or v.device != self.device:
             raise RuntimeError("fock: %s values of %s on %s do not match the grid's %d points on %s"

@@ -38,8 +38,15 @@ class _Kernels:
             out[c::stride] = r
         return _lib.PQB_OK
 
-    def pqb_grid_fock(self, *a):
-        raise AssertionError("reached the kernel")
+    def pqb_grid_fock(self, ng, n, B, v, F, work, stream):
+        assert self.gr.bfgrid.dtype == torch.float64 and self.gr.bfgrid.shape == (ng, n)
+
+        def array(p, count):
+            return np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ctypes.c_double)), (count,))
+
+        b = array(B, ng * n).reshape(ng, n)
+        array(F, n * n)[:] = (b.T @ (array(v, ng)[:, None] * b)).ravel()
+        return _lib.PQB_OK
 
 
 @pytest.fixture
@@ -85,3 +92,11 @@ def test_amplitudes_and_values_of_another_type_are_refused(grid):
             grid.set_density(D)
         with pytest.raises(RuntimeError):
             grid.fock(v)
+
+
+def test_fock_of_amplitudes_that_a_caller_has_set(grid):
+    """getXC's matrix needs amplitudes and no basis: a caller may bring them."""
+    grid.nbf = 0
+    v = torch.linspace(-1.0, 1.0, NG, dtype=torch.float64)
+    want = grid.bfgrid.T @ (v[:, None] * grid.bfgrid)
+    assert torch.allclose(grid.fock(v), want, rtol=1e-12, atol=1e-12)
