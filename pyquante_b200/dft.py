@@ -37,9 +37,10 @@ def getXC(gr, nel, **kwargs):
         raise NotImplementedError("gradient-corrected functionals are not built")
     gr.floor_density()
     w = gr.weights()
-    # (renormalize() with its factor kept on the GPU: the host waits once, for Exc)
+    # (renormalize() with its factor kept on the GPU: the host waits once, for Exc; a
+    # zero density, an error below, is left as it is)
     total = torch.dot(w, gr.density.sum(1))
-    gr.density *= nel / total
+    gr.density *= torch.where(total == 0.0, 1.0, nel / total)
     fxc, va, vb, _, _, _ = XC(gr.density.T, None, functional=functional)
     exc = torch.dot(w, fxc)
     Fxc = gr.fock(w * va)

@@ -11,6 +11,7 @@ import torch
 
 from pyquante_b200 import MolecularGrid as M
 from pyquante_b200 import _lib
+from pyquante_b200 import dft as dft_module
 
 NG, N = 11, 3
 
@@ -100,3 +101,19 @@ def test_fock_of_amplitudes_that_a_caller_has_set(grid):
     v = torch.linspace(-1.0, 1.0, NG, dtype=torch.float64)
     want = grid.bfgrid.T @ (v[:, None] * grid.bfgrid)
     assert torch.allclose(grid.fock(v), want, rtol=1e-12, atol=1e-12)
+
+
+def _xc_stub(rho, gamma, functional):
+    return (rho.sum(0), rho[0].contiguous(), rho[1].contiguous(), None, None, None)
+
+
+def test_getxc_of_a_zero_density_raises_and_leaves_it(grid, monkeypatch):
+    monkeypatch.setattr(dft_module, "XC", _xc_stub)
+    grid.xyzw = torch.ones(NG, 4, dtype=torch.float64)
+    grid.density = torch.full((NG, 2), 1e-12, dtype=torch.float64)   # below the floor
+    with pytest.raises(ZeroDivisionError):
+        dft_module.getXC(grid, 10)
+    assert torch.equal(grid.density, torch.zeros(NG, 2, dtype=torch.float64))
+    grid.density = torch.full((NG, 2), 0.25, dtype=torch.float64)
+    exc, F = dft_module.getXC(grid, 10)
+    assert abs(float(grid.density.sum()) - 10.0) < 1e-12 and abs(exc - 10.0) < 1e-12
