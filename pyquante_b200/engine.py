@@ -90,6 +90,8 @@ class FunctionTable:
             k = len(bf.pexps)
             if k != len(bf.pcoefs) or k != len(bf.pnorms) or not k:
                 raise ValueError("inconsistent primitive lists in %r" % (bf,))
+            if len(bf.origin) != 3 or len(bf.powers) != 3:
+                raise ValueError("the origin and powers of %r have not three components each" % (bf,))
             exps += bf.pexps
             pcoefs += bf.pcoefs
             pnorms += bf.pnorms
@@ -97,8 +99,6 @@ class FunctionTable:
             powers += bf.powers
             norms.append(bf.norm)
             off.append(len(exps))
-        if len(origin) != 3 * n or len(powers) != 3 * n:
-            raise ValueError("a function's origin and powers have three components")
         np_ = len(exps)
         self.n = n
         self.powers_host = np.array(powers, dtype=np.int32).reshape(n, 3)
