@@ -16,7 +16,9 @@ class Atom:
         return self.r[i]
 
     def pos(self):
-        return tuple(np.asarray(self.r, dtype=float).tolist())
+        r = self.r
+        # (a caller's positions may be anything of three numbers, a GPU tensor too)
+        return tuple(r.tolist()) if type(r) is np.ndarray and r.dtype == np.float64 else tuple(float(v) for v in r)
 
     def dist2(self, other):
         return float(((self.r - other.r) ** 2).sum())
