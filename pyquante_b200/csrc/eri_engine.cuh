@@ -1087,8 +1087,7 @@ inline cudaError_t launch_eri_class(const int4 *list, int nq, const PairInfo *pa
         if constexpr (Epi::kCoop) {
             // the list's first nlong items, of more than kCoopItem primitive quartets
             if (nlong > 0) {
-                int grid = (nlong * kCoopLanes + 127) / 128;
-                if (grid > nsm * 32) grid = nsm * 32;
+                const int grid = grid_blocks(nlong, 128 / kCoopLanes, nsm * 32);
                 eri_thread_kernel<LA, LB, LC, LD, R, Epi, kCoopLanes><<<grid, 128, 0, st>>>(list, nlong, pairs, prims,
                                                                                             epi);
                 list += nlong;
@@ -1096,8 +1095,7 @@ inline cudaError_t launch_eri_class(const int4 *list, int nq, const PairInfo *pa
             }
             if (nq == 0) return cudaGetLastError();
         }
-        int grid = (nq + 127) / 128;
-        if (grid > nsm * 32) grid = nsm * 32;
+        const int grid = grid_blocks(nq, 128, nsm * 32);
         eri_thread_kernel<LA, LB, LC, LD, R, Epi><<<grid, 128, 0, st>>>(list, nq, pairs, prims, epi);
     } else if constexpr (std::is_same_v<R, double>) {
         using Lay = WarpLayout<LA, LB, LC, LD>;
@@ -1113,8 +1111,7 @@ inline cudaError_t launch_eri_class(const int4 *list, int nq, const PairInfo *pa
             if (e != cudaSuccess) return e;
             attr_set.fetch_or(bit);
         }
-        int grid = (nq + kWarpsPerBlock * Lay::S - 1) / (kWarpsPerBlock * Lay::S);
-        if (grid > nsm * 16) grid = nsm * 16;
+        const int grid = grid_blocks(nq, kWarpsPerBlock * Lay::S, nsm * 16);
         kern<<<grid, kWarpsPerBlock * 32, Lay::bytes, st>>>(list, nq, pairs, prims, epi);
     } else {
         return cudaErrorInvalidValue;   // the host sends these classes' FP32 lists to the FP64 kernels

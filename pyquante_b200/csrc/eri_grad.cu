@@ -341,16 +341,14 @@ static cudaError_t eri_grad_launch(const int4 *list, int nq, const PairInfo *pai
                                    const double *D, double *gshell, int glen, cudaStream_t st, int nsm)
 {
     if constexpr (ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) <= 27) {
-        int grid = (nq + 127) / 128;
-        if (grid > nsm * 32) grid = nsm * 32;
+        const int grid = grid_blocks(nq, 128, nsm * 32);
         eri_grad_thread_kernel<LA, LB, LC, LD><<<grid, 128, 0, st>>>(list, nq, pairs, prims, D, gshell, glen);
     } else {
         using Lay = GradWarpLayout<LA, LB, LC, LD>;
         auto kern = eri_grad_warp_kernel<LA, LB, LC, LD>;
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
         if (e != cudaSuccess) return e;
-        int grid = (nq + Lay::warps - 1) / Lay::warps;
-        if (grid > nsm * 16) grid = nsm * 16;
+        const int grid = grid_blocks(nq, Lay::warps, nsm * 16);
         kern<<<grid, Lay::warps * 32, Lay::bytes, st>>>(list, nq, pairs, prims, D, gshell, glen);
     }
     return cudaGetLastError();

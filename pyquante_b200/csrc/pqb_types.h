@@ -70,6 +70,14 @@ __host__ __device__ inline int pair_class(int la, int lb)   // la >= lb
 // than kCoopItem.
 constexpr int kCoopItem = 24, kCoopLanes = 8;
 
+// Blocks for a grid-stride launch over n items, per_block at a time, `most` blocks
+// at most.  In 64 bits: an int that counted the lanes of shared items would
+// overflow from 2^28 of them (the (ss|ss) quartets of 216 contracted s shells).
+__host__ __device__ constexpr int grid_blocks(int64_t n, int per_block, int most)
+{
+    return (n + per_block - 1) / per_block < most ? (int)((n + per_block - 1) / per_block) : most;
+}
+
 // Components of quartet class qc; classes of more than kThreadMax run in warp
 // mode, in FP64 in both precision modes.
 constexpr int kThreadMax = 81;
