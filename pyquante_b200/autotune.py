@@ -30,13 +30,17 @@ def load():
 
 
 def apply(eng, tuned=None):
-    """Set the tuned knobs on a BasisEngine's context (before its plan)."""
+    """Set the tuned knobs on a BasisEngine's context (before its plan).  The
+    chunks of the stored result, which were tuned on one large basis, are the
+    most that the plan of another takes; those of a given result are set as
+    they are, as the sweep below does."""
     from . import _lib
+    param = _lib.PQB_PARAM_CHUNK_MAX if tuned is None else _lib.PQB_PARAM_CHUNK
     tuned = tuned if tuned is not None else load()
     if not tuned:
         return False
     for qc, ch in enumerate(tuned.get("chunk", [])):
-        eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_CHUNK, qc, int(ch)))
+        eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, param, qc, int(ch)))
     if "streams" in tuned:
         eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_STREAMS, 0, int(tuned["streams"])))
     if "order" in tuned:

@@ -29,7 +29,8 @@ using namespace pqb;
 // Primitive-quartet chunk for the J/K work items: long contractions
 // (up to 1296 primitive quartets for a 6-primitive s shell to the fourth)
 // are cut so no thread or block slot runs a long serial chain.  Per class,
-// tunable with pqb_set_param(PQB_PARAM_CHUNK) (default 16).
+// tunable with pqb_set_param: PQB_PARAM_CHUNK_MAX is the most that plan_chunks
+// takes (default 16), PQB_PARAM_CHUNK the length itself.
 static const int kDefaultChunk = 16;
 
 struct pqb_ctx {
@@ -81,7 +82,8 @@ struct pqb_ctx {
     long long dense_len = 0;
     long long *d_mol_off = nullptr;
     int *d_mol_n = nullptr;
-    int chunk[kNumQuartetClass];     // primitive-quartet chunk per class
+    int chunk[kNumQuartetClass];     // primitive-quartet chunk per class: the largest, or (chunk_set) the one
+    bool chunk_set[kNumQuartetClass] = {false};
     int nstreams = 16;
     bool small_plan = false;         // the current plan is one of a few molecules' latency (see plan_chunks)
     int order = 1;                   // class launch order: 0 by cost, 1 high angular momentum first
@@ -1529,7 +1531,8 @@ int pqb_schwarz(pqb_ctx *ctx, double *Q_host, void *stream)
     }
 }
 
-// The chunk of each class for a plan of this basis.  The tuned chunks (32
+// The chunk of each class for a plan of this basis, where the caller has not set
+// it.  The tuned chunks (32
 // primitive quartets an item) suit builds that fill the GPU; below that an
 // item's serial chain is the build's length (a (11|11) primitive quartet takes
 // 1.5 us), so the items are cut until a class gives about 4096 of them, to a
@@ -1563,7 +1566,8 @@ static bool plan_chunks(const pqb_ctx *ctx, int *chunk)
     }
     const int lo = (int)std::min(64.0, std::max(4.0, total / 0.75e6));
     for (int c = 0; c < kNumQuartetClass; ++c)
-        chunk[c] = std::min(ctx->chunk[c], std::max(lo, (int)std::min(1024.0, u[c] / 4096.0)));
+        chunk[c] = ctx->chunk_set[c] ? ctx->chunk[c]
+                                     : std::min(ctx->chunk[c], std::max(lo, (int)std::min(1024.0, u[c] / 4096.0)));
     return total < 9e6;
 }
 
@@ -1692,13 +1696,12 @@ int pqb_set_param(pqb_ctx *ctx, int param, int qclass, int value)
     drop_graphs(ctx);
     switch (param) {
     case PQB_PARAM_CHUNK:
+    case PQB_PARAM_CHUNK_MAX:
         if (value < 1 || value > 4096) return fail(ctx, PQB_E_ARG, "chunk %d out of range 1..4096", value);
-        if (qclass < 0) {
-            for (int c = 0; c < kNumQuartetClass; ++c) ctx->chunk[c] = value;
-        } else if (qclass < kNumQuartetClass) {
-            ctx->chunk[qclass] = value;
-        } else {
-            return fail(ctx, PQB_E_ARG, "class %d", qclass);
+        if (qclass >= kNumQuartetClass) return fail(ctx, PQB_E_ARG, "class %d", qclass);
+        for (int c = qclass < 0 ? 0 : qclass; c <= (qclass < 0 ? kNumQuartetClass - 1 : qclass); ++c) {
+            ctx->chunk[c] = value;
+            ctx->chunk_set[c] = param == PQB_PARAM_CHUNK;
         }
         ctx->have_plan = false;   // takes effect at the next pqb_plan
         return PQB_OK;

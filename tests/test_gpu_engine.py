@@ -645,3 +645,26 @@ def test_hermite_coulomb_equals_the_full_builds_j(mol, basis, schwarz):
         parts += eng.j(D, schwarz=schwarz)
     eng._plan_key = None
     assert float((parts - J).abs().max()) < tol
+
+
+def test_a_chunk_that_the_caller_sets_is_the_plans_chunk():
+    """PQB_PARAM_CHUNK (the autotuner's sweep) cuts the items of any basis at
+    that many primitive quartets; under PQB_PARAM_CHUNK_MAX, which the stored
+    tuning uses, the plan of a small basis cuts them shorter."""
+    import ctypes
+    eng = BasisEngine(BasisSet(geometries.water(), "6-31g**").bfs)
+
+    def items(param, chunk):
+        eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, param, -1, chunk))
+        eng._plan_key = None
+        c = eng.plan(0.0, 1e-5)
+        return c["fp64"] + c["fp32"], c["shell_quartets"]
+
+    prims = (ctypes.c_int64 * 42)()
+    n, quartets = items(_lib.PQB_PARAM_CHUNK, 4096)
+    eng.ctx.check(eng.ctx.lib.pqb_plan_stats(eng.ctx.h, (ctypes.c_int64 * 42)(), prims))
+    assert n == quartets
+    assert items(_lib.PQB_PARAM_CHUNK, 1)[0] == sum(prims)
+    assert items(_lib.PQB_PARAM_CHUNK_MAX, 4096)[0] > quartets
+    assert items(_lib.PQB_PARAM_CHUNK_MAX, 1)[0] == sum(prims)
+    assert items(_lib.PQB_PARAM_CHUNK, 4096)[0] == quartets
