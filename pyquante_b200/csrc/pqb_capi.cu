@@ -50,7 +50,7 @@ struct pqb_ctx {
     // d_Dscaled, and J, K are scaled by the same factors when symmetrised
     double *d_escale = nullptr, *d_Dscaled = nullptr;
     float *d_Dscaled_f = nullptr;    // single-precision copy for the FP32 lists
-    double *d_Dscaled2 = nullptr;    // the second density of pqb_jk_direct2 (allocated on first use)
+    double *d_Dscaled2 = nullptr;    // the second density of pqb_jk_direct2 (see ensure_second)
     float *d_Dscaled2_f = nullptr;
     unsigned long long *d_q2 = nullptr;
     std::vector<PairInfo> pairs;
@@ -104,7 +104,8 @@ struct pqb_ctx {
     cudaGraphExec_t graph_exec[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     bool graph_warm[6] = {false, false, false, false, false, false};   // one eager build first (one-time launch setup stays out of the capture)
     double *d_Jacc = nullptr, *d_Kacc = nullptr;
-    double *d_Jacc2 = nullptr, *d_Kacc2 = nullptr;   // second density's graph accumulators
+    double *d_Jacc2 = nullptr, *d_Kacc2 = nullptr;   // the second density's
+    double *d_acc = nullptr, *d_second = nullptr;    // allocations of their own (see ensure_accumulators)
     // pqb_get2jmk_host: D in, G out, and J, K of its builds outside the graph
     double *d_hD = nullptr, *d_hG = nullptr, *d_hJ = nullptr, *d_hK = nullptr;
     // ... and, for pageable host arrays, the whole call as one graph over
@@ -1124,6 +1125,17 @@ template <class F> static int capture_graph(pqb_ctx *ctx, cudaGraphExec_t &exec,
     return PQB_OK;
 }
 
+// Copies of a single molecule's accumulators (see ItemScreen): the atomics of
+// blocks that run side by side meet at the same rows of J and K, which four copies
+// spread, and a fourth as many roundings follow one another (water / 6-31G**, whose
+// shortest items make 324 of one quartet: 1.5e-15 of J and K's norm with one copy,
+// 0.5e-15 with four).  Device time of a build with one / four: water / 6-31G** 58 / 52 us,
+// (H2O)8 / 6-31G** 326 / 303, mixed 307 / 281, C8H18 / 6-31G** 2111 / 2002, mixed
+// 1946 / 1828, C16H34 / 6-31G* (N = 308) 5200 / 5090, mixed 4790 / 4606; sixteen
+// give 1 % more.  One above N = 512, where the rows lie further apart and the
+// copies grow.
+static int acc_copies(const pqb_ctx *ctx) { return ctx->nmol == 1 && ctx->nbf <= 512 ? kAccCopies : 1; }
+
 extern "C" {
 
 int pqb_version(void) { return 1; }
@@ -1179,11 +1191,12 @@ static void release_basis(pqb_ctx *ctx)
 {
     drop_graphs(ctx);
     drop_jlists(ctx);
-    free_dev(ctx->d_Jacc);
-    free_dev(ctx->d_Kacc);
-    free_dev(ctx->d_Jacc2);
-    free_dev(ctx->d_Kacc2);
+    free_dev(ctx->d_acc);
+    free_dev(ctx->d_second);
+    ctx->d_acc = ctx->d_second = nullptr;
     ctx->d_Jacc = ctx->d_Kacc = ctx->d_Jacc2 = ctx->d_Kacc2 = nullptr;
+    ctx->d_Dscaled2 = nullptr;
+    ctx->d_Dscaled2_f = nullptr;
     free_dev(ctx->d_hD);
     free_dev(ctx->d_hG);
     free_dev(ctx->d_hJ);
@@ -1192,16 +1205,10 @@ static void release_basis(pqb_ctx *ctx)
     if (ctx->h_D) cudaFreeHost(ctx->h_D);
     if (ctx->h_G) cudaFreeHost(ctx->h_G);
     ctx->h_D = ctx->h_G = nullptr;
-    free_dev(ctx->d_Dscaled2);
-    free_dev(ctx->d_Dscaled2_f);
-    ctx->d_Dscaled2 = nullptr;
-    ctx->d_Dscaled2_f = nullptr;
     free_dev(ctx->d_pairs);
     free_dev(ctx->d_prims);
     free_dev(ctx->d_fscale);
     free_dev(ctx->d_escale);
-    free_dev(ctx->d_Dscaled);
-    free_dev(ctx->d_Dscaled_f);
     ctx->d_escale = nullptr;
     ctx->d_Dscaled = nullptr;
     ctx->d_Dscaled_f = nullptr;
@@ -1459,9 +1466,23 @@ static int shells_upload_batch_impl(pqb_ctx *ctx, int nmol, const int *mol_shell
             for (int i = 0; i < n; ++i)
                 for (int j = 0; j < n; ++j) es[(size_t)ctx->mol_off[m] + (size_t)i * n + j] = fscale[f0 + i] * fscale[f0 + j];
         }
-        PQB_CK(ctx, cudaMalloc(&ctx->d_escale, sizeof(double) * std::max<size_t>(es.size(), 1)));
-        PQB_CK(ctx, cudaMalloc(&ctx->d_Dscaled, sizeof(double) * std::max<size_t>(es.size(), 1)));
-        PQB_CK(ctx, cudaMalloc(&ctx->d_Dscaled_f, sizeof(float) * std::max<size_t>(es.size(), 1)));
+        // one allocation (0.3 ms each): the factors, the scaled density and, of up to
+        // 512 functions of one molecule (44 MB), a second one and the accumulators of
+        // both; the densities once more in single precision
+        const size_t dl = es.size(), acc = acc_copies(ctx) > 1 ? acc_copies(ctx) * dl : 0, nd = acc ? 2 : 1;
+        PQB_CK(ctx, cudaMalloc(&ctx->d_escale, sizeof(double) * ((1 + nd) * dl + 4 * acc) + sizeof(float) * nd * dl));
+        ctx->d_Dscaled = ctx->d_escale + dl;
+        ctx->d_Dscaled_f = reinterpret_cast<float *>(ctx->d_escale + (1 + nd) * dl + 4 * acc);
+        if (acc) {
+            ctx->d_Dscaled2 = ctx->d_Dscaled + dl;
+            ctx->d_Dscaled2_f = ctx->d_Dscaled_f + dl;
+            ctx->d_Jacc = ctx->d_Dscaled2 + dl;
+            ctx->d_Kacc = ctx->d_Jacc + acc;
+            ctx->d_Jacc2 = ctx->d_Kacc + acc;
+            ctx->d_Kacc2 = ctx->d_Jacc2 + acc;
+            // (complete before the copy below begins)
+            PQB_CK(ctx, cudaMemset(ctx->d_Jacc, 0, sizeof(double) * 4 * acc));
+        }
         PQB_CK(ctx, cudaMemcpy(ctx->d_escale, es.data(), sizeof(double) * es.size(), cudaMemcpyHostToDevice));
     }
     // unscreened quartet list (packed integrals) and diagonal list (Schwarz)
@@ -1871,15 +1892,6 @@ int pqb_eri_packed(pqb_ctx *ctx, double *out, int64_t len, void *stream)
     }
 }
 
-// Copies of the captured builds' accumulators (see ItemScreen): the atomics of
-// blocks that run side by side meet at the same rows of J and K, which four copies
-// spread.  Device time of a build with one / four: water / 6-31G** 58 / 52 us,
-// (H2O)8 / 6-31G** 326 / 303, mixed 307 / 281, C8H18 / 6-31G** 2111 / 2002, mixed
-// 1946 / 1828, C16H34 / 6-31G* (N = 308) 5200 / 5090, mixed 4790 / 4606; sixteen
-// give 1 % more.  One above N = 512, where the rows lie further apart and the
-// copies grow.
-static int acc_copies(const pqb_ctx *ctx) { return ctx->nmol == 1 && ctx->nbf <= 512 ? kAccCopies : 1; }
-
 // The class launches of one build into the accumulators Jacc[s], Kacc[s]
 // (zeroed here) of nden = 1 or 2 densities on stream st, forked over the
 // context's streams and joined back; they read the scaled densities
@@ -1950,36 +1962,60 @@ static int launch_build(pqb_ctx *ctx, int nden, double *const Jacc[2], double *c
     return PQB_OK;
 }
 
-// Both accumulators of a pair or neither: a failed second allocation leaves
-// no half-made pair behind.
-static int ensure_acc_pair(pqb_ctx *ctx, double *&J, double *&K)
+// Accumulators of a large basis, made on first use (those of up to 512 functions
+// of one molecule come with the basis).  Zeroed on the stream of the build that asks for them: a
+// memset on the default stream would not wait for, nor hold up, a build on a
+// non-blocking one.  Each use leaves them zeroed (symmetrize_take_kernel).
+static int ensure_accumulators(pqb_ctx *ctx, cudaStream_t st)
 {
-    if (J && K) return PQB_OK;
-    free_dev(J);
-    free_dev(K);
-    J = K = nullptr;
-    const size_t bytes = sizeof(double) * acc_copies(ctx) * std::max<long long>(ctx->dense_len, 1);
-    cudaError_t e = cudaMalloc(&J, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&K, bytes);
-    // zeroed once here; each use leaves them zeroed (symmetrize_take_kernel)
-    if (e == cudaSuccess) e = cudaMemset(J, 0, bytes);
-    if (e == cudaSuccess) e = cudaMemset(K, 0, bytes);
-    if (e != cudaSuccess) {
-        free_dev(J);
-        free_dev(K);
-        J = K = nullptr;
-        return fail(ctx, PQB_E_CUDA, "graph accumulators: %s", cudaGetErrorString(e));
-    }
+    if (ctx->d_Jacc) return PQB_OK;
+    const size_t len = (size_t)acc_copies(ctx) * std::max<long long>(ctx->dense_len, 1);
+    PQB_CK(ctx, cudaMalloc(&ctx->d_acc, sizeof(double) * 2 * len));
+    PQB_CK(ctx, cudaMemsetAsync(ctx->d_acc, 0, sizeof(double) * 2 * len, st));
+    ctx->d_Jacc = ctx->d_acc;
+    ctx->d_Kacc = ctx->d_acc + len;
     return PQB_OK;
+}
+
+// The same for a second density: a single molecule's accumulators, the scaled
+// density and its single-precision copy.
+static int ensure_second(pqb_ctx *ctx, cudaStream_t st)
+{
+    if (ctx->d_Dscaled2) return PQB_OK;
+    const size_t dl = std::max<long long>(ctx->dense_len, 1), acc = ctx->nmol == 1 ? acc_copies(ctx) * dl : 0;
+    double *p = nullptr;
+    PQB_CK(ctx, cudaMalloc(&p, sizeof(double) * (2 * acc + dl) + sizeof(float) * dl));
+    const cudaError_t e = acc ? cudaMemsetAsync(p, 0, sizeof(double) * 2 * acc, st) : cudaSuccess;
+    if (e != cudaSuccess) {
+        free_dev(p);
+        return fail(ctx, PQB_E_CUDA, "second accumulators: %s", cudaGetErrorString(e));
+    }
+    ctx->d_second = p;
+    if (acc) {
+        ctx->d_Jacc2 = p;
+        ctx->d_Kacc2 = p + acc;
+    }
+    ctx->d_Dscaled2 = p + 2 * acc;
+    ctx->d_Dscaled2_f = reinterpret_cast<float *>(p + 2 * acc + dl);
+    return PQB_OK;
+}
+
+// After a failed build: part of it may have reached the accumulators.
+static void clear_accumulators(pqb_ctx *ctx)
+{
+    const size_t bytes = sizeof(double) * 2 * acc_copies(ctx) * std::max<long long>(ctx->dense_len, 1);
+    cudaDeviceSynchronize();
+    if (ctx->d_Jacc) cudaMemset(ctx->d_Jacc, 0, bytes);
+    if (ctx->d_Jacc2) cudaMemset(ctx->d_Jacc2, 0, bytes);
+    cudaDeviceSynchronize();
 }
 
 // Capture launch_build into the ctx-owned accumulators as a graph for
 // (nden, mode) (index gi), once; later builds replay it with one launch.
-static int ensure_build_graph(pqb_ctx *ctx, int nden, bool jonly, int mode, int gi)
+static int ensure_build_graph(pqb_ctx *ctx, int nden, bool jonly, int mode, int gi, cudaStream_t st)
 {
     if (ctx->graph_exec[gi]) return PQB_OK;
-    int rc = ensure_acc_pair(ctx, ctx->d_Jacc, ctx->d_Kacc);
-    if (rc == PQB_OK && nden == 2) rc = ensure_acc_pair(ctx, ctx->d_Jacc2, ctx->d_Kacc2);
+    const int rc = ensure_accumulators(ctx, st);
     if (rc != PQB_OK) return rc;
     double *const Ja[2] = {ctx->d_Jacc, ctx->d_Jacc2};
     double *const Ka[2] = {jonly ? nullptr : ctx->d_Kacc, ctx->d_Kacc2};
@@ -2094,25 +2130,17 @@ static int launch_hermite(pqb_ctx *ctx, cudaStream_t st)
 }
 
 // J and K of nden densities D[s] into J[s], K[s] (K[0] == nullptr with one
-// density: J alone).  With G (one density, J and K wanted): G = 2J - K
-// as well; on the graph path G alone is written (J, K untouched), else J and
-// K are written and then combined.
-static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], double *const J[2], double *const K[2],
+// density: J alone).  With G (one density): G = 2J - K alone, out of the
+// accumulators or, without them, out of the context's own J and K.
+static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], double *const *J, double *const *K,
                           int mode, void *stream, double *G = nullptr)
 {
-    const bool jonly = nden == 1 && !K[0];
+    const bool jonly = nden == 1 && !K[0] && !G;
     const int n = ctx->nbf;
     cudaStream_t st = (cudaStream_t)stream;
-    if (nden == 2 && !ctx->d_Dscaled2) {
-        const size_t len = std::max<long long>(ctx->dense_len, 1);
-        PQB_CK(ctx, cudaMalloc(&ctx->d_Dscaled2, sizeof(double) * len));
-        const cudaError_t e = cudaMalloc(&ctx->d_Dscaled2_f, sizeof(float) * len);
-        if (e != cudaSuccess) {
-            free_dev(ctx->d_Dscaled2);
-            ctx->d_Dscaled2 = nullptr;
-            ctx->d_Dscaled2_f = nullptr;
-            return fail(ctx, PQB_E_CUDA, "second scaled density: %s", cudaGetErrorString(e));
-        }
+    if (nden == 2) {
+        const int rc = ensure_second(ctx, st);
+        if (rc != PQB_OK) return rc;
     }
     double *Dsc[2] = {ctx->d_Dscaled, ctx->d_Dscaled2};
     float *Dsf[2] = {ctx->d_Dscaled_f, ctx->d_Dscaled2_f};
@@ -2147,10 +2175,26 @@ static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], doub
                                         ctx->d_escale, J[0], st));
         return PQB_OK;
     }
+    // A single molecule's build goes into the context's accumulators and is taken from
+    // there: replayed, or, the first one, launched.
+    bool taken = false;
     if (ctx->use_graph && ctx->nmol == 1 && cs == cudaStreamCaptureStatusNone && ctx->graph_warm[gi]) {
-        const int rc = ensure_build_graph(ctx, nden, jonly, mode, gi);
+        const int rc = ensure_build_graph(ctx, nden, jonly, mode, gi, st);
         if (rc != PQB_OK) return rc;
         PQB_CK(ctx, cudaGraphLaunch(ctx->graph_exec[gi], st));
+        taken = true;
+    } else if (cs == cudaStreamCaptureStatusNone && acc_copies(ctx) > 1) {
+        double *const Ja[2] = {ctx->d_Jacc, ctx->d_Jacc2};
+        double *const Ka[2] = {jonly ? nullptr : ctx->d_Kacc, ctx->d_Kacc2};
+        const int rc = launch_build(ctx, nden, Ja, Ka, mode, st, false);
+        if (rc != PQB_OK) {
+            clear_accumulators(ctx);
+            return rc;
+        }
+        ctx->graph_warm[gi] = true;
+        taken = true;
+    }
+    if (taken) {
         double *Ja[2] = {ctx->d_Jacc, ctx->d_Jacc2}, *Ka[2] = {ctx->d_Kacc, ctx->d_Kacc2};
         if (G) {
             take_2jmk_kernel<<<(unsigned)((P + 63) / 64), 64, 0, st>>>(Ja[0], Ka[0], G, n, acc_copies(ctx),
@@ -2163,6 +2207,15 @@ static int jk_direct_impl(pqb_ctx *ctx, int nden, const double *const D[2], doub
                 Ja[s], J[s], jonly ? nullptr : Ka[s], jonly ? nullptr : K[s], n, acc_copies(ctx), ctx->d_escale);
         PQB_CK(ctx, cudaGetLastError());
         return PQB_OK;
+    }
+    double *gJ[2] = {nullptr, nullptr}, *gK[2] = {nullptr, nullptr};
+    if (G) {
+        for (double **b : {&ctx->d_hJ, &ctx->d_hK})
+            if (!*b) PQB_CK(ctx, cudaMalloc(b, sizeof(double) * n * n));
+        gJ[0] = ctx->d_hJ;
+        gK[0] = ctx->d_hK;
+        J = gJ;
+        K = gK;
     }
     const int rc = launch_build(ctx, nden, J, K, mode, st);
     if (rc != PQB_OK) return rc;
@@ -2218,7 +2271,7 @@ static int get2jmk_pageable(pqb_ctx *ctx, const double *D_host, double *G_host, 
     if (!ctx->h_G) PQB_CK(ctx, cudaMallocHost(&ctx->h_G, bytes));
     cudaGraphExec_t &exec = ctx->host_graph[mode == PQB_MIXED ? 1 : 0];
     if (!exec) {
-        int rc = ensure_acc_pair(ctx, ctx->d_Jacc, ctx->d_Kacc);
+        int rc = ensure_accumulators(ctx, st);
         if (rc != PQB_OK) return rc;
         rc = capture_graph(ctx, exec, [&](cudaStream_t cs) {
             PQB_CK(ctx, cudaMemcpyAsync(ctx->d_hD, ctx->h_D, bytes, cudaMemcpyHostToDevice, cs));
@@ -2252,8 +2305,7 @@ static int get2jmk_host_impl(pqb_ctx *ctx, const double *D_host, double *G_host,
     PQB_CK(ctx, cudaSetDevice(ctx->device));
     const int n = ctx->nbf;
     const size_t bytes = sizeof(double) * (size_t)n * n;
-    double **bufs[4] = {&ctx->d_hD, &ctx->d_hG, &ctx->d_hJ, &ctx->d_hK};
-    for (double **b : bufs)
+    for (double **b : {&ctx->d_hD, &ctx->d_hG})
         if (!*b) PQB_CK(ctx, cudaMalloc(b, bytes));
     cudaStream_t st = (cudaStream_t)stream;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -2263,8 +2315,8 @@ static int get2jmk_host_impl(pqb_ctx *ctx, const double *D_host, double *G_host,
         return get2jmk_pageable(ctx, D_host, G_host, mode, st);
     PQB_CK(ctx, cudaMemcpyAsync(ctx->d_hD, D_host, bytes, cudaMemcpyHostToDevice, st));
     const double *Dv[2] = {ctx->d_hD, nullptr};
-    double *Jv[2] = {ctx->d_hJ, nullptr}, *Kv[2] = {ctx->d_hK, nullptr};
-    const int rc = jk_direct_impl(ctx, 1, Dv, Jv, Kv, mode, stream, ctx->d_hG);
+    double *const none[2] = {nullptr, nullptr};
+    const int rc = jk_direct_impl(ctx, 1, Dv, none, none, mode, stream, ctx->d_hG);
     if (rc != PQB_OK) return rc;
     PQB_CK(ctx, cudaMemcpyAsync(G_host, ctx->d_hG, bytes, cudaMemcpyDeviceToHost, st));
     return PQB_OK;

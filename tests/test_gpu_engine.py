@@ -668,3 +668,42 @@ def test_a_chunk_that_the_caller_sets_is_the_plans_chunk():
     assert items(_lib.PQB_PARAM_CHUNK_MAX, 4096)[0] > quartets
     assert items(_lib.PQB_PARAM_CHUNK_MAX, 1)[0] == sum(prims)
     assert items(_lib.PQB_PARAM_CHUNK, 4096)[0] == quartets
+
+
+def test_launched_builds_round_no_more_than_replayed_ones():
+    """Water / 6-31G** has the shortest items of all plans: the quartets of
+    contracted shells reach one element of J or K in up to 324 pieces.  A chain
+    of m additions rounds by about 0.3 sqrt(m) 2^-52 of the sum: 0.6e-15 over
+    four copies of the sums, 1.2e-15 over one, so that 0.9e-15 tells them
+    apart (mean of ten builds, Frobenius norm, against sums in extended
+    precision over the packed integrals)."""
+    from pyquante_b200.LA2 import geigh, mkdens
+    mol = geometries.water()
+    bs = BasisSet(mol, "6-31g**")
+    S, h = Ints.get1ints(bs, mol)
+    _, C = geigh(torch.as_tensor(h, device="cuda"), torch.as_tensor(S, device="cuda"))
+    D = mkdens(C, 0, 5).contiguous()
+    eng = BasisEngine(bs.bfs)
+    n = eng.nbf
+    i, j = np.tril_indices(n)
+    pair = np.zeros((n, n), dtype=np.int64)
+    pair[i, j] = pair[j, i] = np.arange(len(i))
+    IJ, KL = pair[:, :, None, None], pair[None, None]
+    hi, lo = np.maximum(IJ, KL), np.minimum(IJ, KL)
+    eri = eng.eri_packed().cpu().numpy().astype(np.longdouble)[hi * (hi + 1) // 2 + lo]
+    Dl = D.cpu().numpy().astype(np.longdouble)
+    want = 2 * (eri * Dl).sum(axis=(2, 3)) - (eri * Dl[None, :, None, :]).sum(axis=(1, 3))
+
+    def error(graph):
+        eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_GRAPH, 0, graph))
+        eng.jk(D, schwarz=0.0)
+        errs = []
+        for _ in range(10):
+            J, K = eng.jk(D, schwarz=0.0)
+            d = (2.0 * J - K).cpu().numpy().astype(np.longdouble) - want
+            errs.append(float(np.sqrt((d * d).sum() / (want * want).sum())))
+        return np.mean(errs)
+
+    launched, replayed = error(0), error(1)
+    print("launched %.2e replayed %.2e" % (launched, replayed))
+    assert launched < 0.9e-15 and replayed < 0.9e-15
