@@ -111,6 +111,7 @@ struct pqb_ctx {
     // ... and, for pageable host arrays, the whole call as one graph over
     // page-locked copies of D and G ([mode])
     double *h_D = nullptr, *h_G = nullptr;
+    bool no_page_locked = false;     // there was no memory for them: the plain pageable copies serve
     cudaGraphExec_t host_graph[2] = {nullptr, nullptr};
     // Coulomb-only builds in the Hermite basis (see ensure_jlists): the lists,
     // each pair's place in V, and what they depend on
@@ -1202,9 +1203,9 @@ static void release_basis(pqb_ctx *ctx)
     free_dev(ctx->d_hJ);
     free_dev(ctx->d_hK);
     ctx->d_hD = ctx->d_hG = ctx->d_hJ = ctx->d_hK = nullptr;
-    if (ctx->h_D) cudaFreeHost(ctx->h_D);
-    if (ctx->h_G) cudaFreeHost(ctx->h_G);
+    if (ctx->h_D) cudaFreeHost(ctx->h_D);   // (with h_G behind it)
     ctx->h_D = ctx->h_G = nullptr;
+    ctx->no_page_locked = false;
     free_dev(ctx->d_pairs);
     free_dev(ctx->d_prims);
     free_dev(ctx->d_fscale);
@@ -2262,13 +2263,28 @@ static bool pageable(const void *p)
     return at.type == cudaMemoryTypeUnregistered;
 }
 
+// The page-locked copies, made on first use; false where the system has no such
+// memory to give (asked for once a basis).
+static bool page_locked_copies(pqb_ctx *ctx)
+{
+    if (ctx->h_D || ctx->no_page_locked) return ctx->h_D != nullptr;
+    const size_t len = (size_t)ctx->nbf * ctx->nbf;
+    double *p = nullptr;
+    if (cudaMallocHost(&p, sizeof(double) * 2 * len) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->no_page_locked = true;
+        return false;
+    }
+    ctx->h_D = p;
+    ctx->h_G = p + len;
+    return true;
+}
+
 // One launch for a repeated call on pageable arrays: D in, build, G out.
 static int get2jmk_pageable(pqb_ctx *ctx, const double *D_host, double *G_host, int mode, cudaStream_t st)
 {
     const int n = ctx->nbf;
     const size_t bytes = sizeof(double) * (size_t)n * n;
-    if (!ctx->h_D) PQB_CK(ctx, cudaMallocHost(&ctx->h_D, bytes));
-    if (!ctx->h_G) PQB_CK(ctx, cudaMallocHost(&ctx->h_G, bytes));
     cudaGraphExec_t &exec = ctx->host_graph[mode == PQB_MIXED ? 1 : 0];
     if (!exec) {
         int rc = ensure_accumulators(ctx, st);
@@ -2311,7 +2327,7 @@ static int get2jmk_host_impl(pqb_ctx *ctx, const double *D_host, double *G_host,
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     PQB_CK(ctx, cudaStreamIsCapturing(st, &cs));
     if (ctx->use_graph && cs == cudaStreamCaptureStatusNone && ctx->graph_warm[mode == PQB_MIXED ? 1 : 0] &&
-        pageable(D_host) && pageable(G_host))
+        pageable(D_host) && pageable(G_host) && page_locked_copies(ctx))
         return get2jmk_pageable(ctx, D_host, G_host, mode, st);
     PQB_CK(ctx, cudaMemcpyAsync(ctx->d_hD, D_host, bytes, cudaMemcpyHostToDevice, st));
     const double *Dv[2] = {ctx->d_hD, nullptr};
