@@ -116,6 +116,7 @@ struct pqb_ctx {
     // Coulomb-only builds in the Hermite basis (see ensure_jlists): the lists,
     // each pair's place in V, and what they depend on
     JLists jl;
+    bool no_jlists = false;          // there was no memory for them: the class kernels serve until the next plan
     int64_t *d_jfirst = nullptr;
     double plan_thresh = 0.0;        // Schwarz threshold of the current plan
     bool sharded = false;            // the current plan holds one rank's share
@@ -1186,6 +1187,7 @@ static void drop_jlists(pqb_ctx *ctx)
     free_dev(ctx->d_jfirst);
     ctx->jl = JLists{};
     ctx->d_jfirst = nullptr;
+    ctx->no_jlists = false;
 }
 
 static void release_basis(pqb_ctx *ctx)
@@ -1703,6 +1705,7 @@ int pqb_plan(pqb_ctx *ctx, double schwarz_thresh, double fp32_thresh, int64_t *c
     ctx->have_plan = true;
     ctx->plan_thresh = schwarz_thresh;
     ctx->sharded = false;
+    ctx->no_jlists = false;
     if (counts) {
         counts[0] = total;
         counts[1] = nitems[0];
@@ -2051,11 +2054,11 @@ static bool hermite_route(const pqb_ctx *ctx)
 // The Hermite lists of a Coulomb-only build, made on first use: the shell pairs
 // of each L = La + Lb by descending Schwarz factor, their primitive pairs in turn.
 // Without memory for them the lists stay empty (not an error: the class kernels
-// need none).
+// need none) and are not tried for again before the next plan or Schwarz factors,
+// which drop the graphs too: a Coulomb graph is of one kind as long as it lives.
 static int ensure_jlists(pqb_ctx *ctx, cudaStream_t st)
 {
-    if (ctx->jl.list) return PQB_OK;
-    drop_graphs(ctx);   // a build captured while there was no memory is one of the class kernels
+    if (ctx->jl.list || ctx->no_jlists) return PQB_OK;
     const auto &pairs = ctx->pairs;
     const int np = (int)pairs.size();
     std::vector<std::pair<double, int>> byL[5];   // (-Q, pair): ascending is descending Q, equal ones by index
@@ -2099,6 +2102,7 @@ static int ensure_jlists(pqb_ctx *ctx, cudaStream_t st)
         drop_jlists(ctx);
         if (e == cudaErrorMemoryAllocation) {
             (void)cudaGetLastError();
+            ctx->no_jlists = true;
             return PQB_OK;
         }
         return fail(ctx, PQB_E_CUDA, "Hermite lists: %s", cudaGetErrorString(e));

@@ -87,3 +87,54 @@ out["diff"] = max(float(abs(Ints.get2JmK(ints, D) - want).max()) for _ in range(
 out["asked"] = f.host - before
 """)
     assert out["diff"] < 1e-12 and out["asked"] == 1
+
+
+HERMITE = r"""
+eng = BasisEngine(BasisSet(geometries.water_cluster(2, seed=5), "6-31g**").bfs)
+eng.ctx.check(eng.ctx.lib.pqb_set_param(eng.ctx.h, _lib.PQB_PARAM_HERMITE, 0, 0))   # at any size
+D = torch.eye(eng.nbf, dtype=torch.float64, device="cuda") + 0.1
+for _ in range(3):
+    J, K = eng.jk(D)
+J0 = torch.empty_like(J)
+def j():
+    J0.fill_(-1.0)
+    eng.j(D, J=J0)
+    return float((J0 - J).abs().max())
+"""
+
+
+def test_first_coulomb_build_leaves_the_other_graphs(tmp_path):
+    """Making the Hermite lists must not throw away the J/K build's graph."""
+    out = _child(tmp_path, HERMITE + r"""
+out["diff"] = j()
+graphs, launches = f.graphs, f.launches
+eng.jk(D, J=J, K=K)
+out["graphs"], out["launches"] = f.graphs - graphs, f.launches - launches
+""")
+    assert out["diff"] < 1e-11 and out["graphs"] == 0 and out["launches"] == 1
+
+
+def test_coulomb_builds_without_memory_for_the_lists(tmp_path):
+    """Without memory for the Hermite lists the class kernels build J, replay
+    their graph, leave the J/K graph alone and do not try for the lists at
+    every call; the next plan does."""
+    out = _child(tmp_path, HERMITE + r"""
+f.fail_device = 1
+tried = f.device
+diffs = [j()]
+out["first"] = f.device - tried
+tried, launches = f.device, f.launches
+diffs += [j() for _ in range(3)]
+out["again"], out["replayed"] = f.device - tried, f.launches - launches
+graphs = f.graphs
+eng.jk(D, J=J, K=K)
+out["graphs"] = f.graphs - graphs
+f.fail_device = 0
+tried = f.device
+eng._plan_key = None
+diffs += [j() for _ in range(3)]
+out["after"] = f.device - tried
+out["diff"] = max(diffs)
+""")
+    assert out["diff"] < 1e-11
+    assert out["first"] > 0 and out["again"] == 0 and out["replayed"] == 3 and out["graphs"] == 0 and out["after"] > 0
