@@ -124,3 +124,13 @@ def test_density_and_fock_tiles_at_their_edges(npts, n, skew):
     want = B.T @ (v[:, None] * B)
     assert float((F - want).abs().max()) <= 1e-13 * float((B.abs().T @ (v.abs()[:, None] * B.abs())).max())
     assert torch.equal(F, F.T)
+
+
+@pytest.mark.parametrize("npts,n", [(1, 1), (130, 7), (1000, 33)])
+def test_rowdot(npts, n):
+    """pqb_grid_rowdot: sums of n products, n 2^-53 of the sum of magnitudes each way."""
+    g = torch.Generator().manual_seed(n)
+    A, B = (torch.randn(npts, n, generator=g, dtype=torch.float64).cuda() for _ in range(2))
+    out = torch.full((npts,), float("nan"), dtype=torch.float64, device="cuda")
+    assert _lib.load().pqb_grid_rowdot(npts, n, _lib.ptr(A), _lib.ptr(B), _lib.ptr(out), _lib.stream_ptr()) == _lib.PQB_OK
+    assert bool(((out - (A * B).sum(1)).abs() <= 2 * n * 2.0 ** -53 * (A * B).abs().sum(1)).all())

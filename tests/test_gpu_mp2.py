@@ -160,3 +160,46 @@ def test_contract_rows_at_tile_edges(n, nb, row0, nrows):
                                   _lib.stream_ptr()) == _lib.PQB_OK
     want = torch.einsum("kb,rkl->brl", C, X)
     assert float((out - want).abs().max()) < 1e-13 * n * float(want.abs().max().clamp(min=1.0))
+
+
+def _dense_rows(ints, n, row0, nrows):
+    """(IJ|kl) of some packed rows as (nrows, n, n), by plain indexing."""
+    k, l = torch.meshgrid(torch.arange(n, device="cuda"), torch.arange(n, device="cuda"), indexing="ij")
+    KL = torch.maximum(k, l) * (torch.maximum(k, l) + 1) // 2 + torch.minimum(k, l)
+    IJ = row0 + torch.arange(nrows, device="cuda")[:, None, None]
+    hi, lo = torch.maximum(KL[None], IJ), torch.minimum(KL[None], IJ)
+    return ints[hi * (hi + 1) // 2 + lo]
+
+
+@pytest.mark.parametrize("n,nb", [
+    # one of every (strips a warp, warps along l) that a basis of up to 300 functions can get
+    (3, 30), (9, 30), (19, 3), (11, 33), (21, 30), (35, 3), (19, 33), (37, 30), (67, 3), (27, 40), (51, 65), (97, 40),
+    (35, 33), (67, 65), (129, 40), (43, 40), (85, 30), (161, 40), (51, 40), (99, 65), (193, 40), (59, 40), (117, 30),
+    (225, 40), (67, 40), (131, 65), (287, 7), (75, 40), (149, 30)])
+def test_contract_rows_in_every_layout(n, nb):
+    """Against the dense FP64 product of rows by plain indexing: each of the two
+    sums of n terms is off by at most n 2^-53 of the sum of magnitudes."""
+    P = n * (n + 1) // 2
+    nrows = min(9, P)
+    row0 = max(0, P // 2 - 4)   # numbers of the row itself, and of later rows
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ints = torch.randn(P * (P + 1) // 2, generator=g, dtype=torch.float64, device="cuda")
+    C = torch.randn(n, nb, generator=g, dtype=torch.float64, device="cuda")
+    out = torch.full((nb, nrows, n), float("nan"), dtype=torch.float64, device="cuda")
+    assert _lib.load().pqb_mo_contract_rows(_lib.ptr(ints), ints.numel(), n, row0, nrows, _lib.ptr(C), nb, _lib.ptr(out),
+                                            _lib.stream_ptr()) == _lib.PQB_OK
+    X = _dense_rows(ints, n, row0, nrows)
+    want = torch.einsum("kb,rkl->brl", C, X)
+    size = torch.einsum("kb,rkl->brl", C.abs(), X.abs())
+    assert bool(((out - want).abs() <= 2 * n * 2.0 ** -53 * size).all())
+
+
+@pytest.mark.parametrize("n,ncol", [(1, 1), (5, 3), (33, 7)])
+def test_unpack_pairs(n, ncol):
+    """Copies: rows stored per packed pair, to both orders."""
+    P = n * (n + 1) // 2
+    Y = torch.arange(P * ncol, dtype=torch.float64, device="cuda").view(P, ncol)
+    out = torch.full((n, n, ncol), -1.0, dtype=torch.float64, device="cuda")
+    assert _lib.load().pqb_mo_unpack_pairs(_lib.ptr(Y), n, ncol, _lib.ptr(out), _lib.stream_ptr()) == _lib.PQB_OK
+    i, j = torch.tril_indices(n, n, device="cuda")
+    assert torch.equal(out[i, j], Y) and torch.equal(out[j, i], Y)
