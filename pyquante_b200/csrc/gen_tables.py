@@ -195,18 +195,6 @@ def main():
                 cu, cw = funcs[2 * r], funcs[2 * r + 1]
                 lines.append("  " + ", ".join("%.17e, %.17e" % (a, b) for a, b in zip(cu, cw)) + ",")
     lines.append("};")
-    # FP32 copy for the mixed-precision kernels: per (n, interval, root) the
-    # first 7 coefficient pairs (the rest sum to < 1.1e-8 relative) and a zero
-    # pair, 64 bytes: two 256-bit loads
-    lines.append("#define PQB_RYS_NCOEF_F32 7")
-    lines.append("PQB_TABQ __align__(64) float pqb_rys_coef_f32[PQB_RYS_TABLE_SIZE / 14 * 16 / 2] = {")
-    for n in range(1, RYS_NMAX + 1):
-        for iv, funcs in enumerate(rys[n]):
-            for r in range(n):
-                cu, cw = funcs[2 * r], funcs[2 * r + 1]
-                pairs = [(cu[k], cw[k]) for k in range(7)] + [(0.0, 0.0)]
-                lines.append("  " + ", ".join("%.9ef, %.9ef" % (a, b) for a, b in pairs) + ",")
-    lines.append("};")
     lines.append("PQB_TABQ __align__(64) double pqb_boys_tab[PQB_BOYS_NGRID * PQB_BOYS_NORD] = {")
     for row in boys_tab:
         lines.append("  " + ", ".join("%.17e" % v for v in row) + ",")
