@@ -84,7 +84,7 @@ def tune(eng, D, mode="mixed", schwarz=1e-12, fp32_threshold=1e-5, verbose=True)
         eng.plan(schwarz, fp32_threshold)
         return _build_ms(eng, D, J, K, mode, schwarz, fp32_threshold, flush)
 
-    streams = 8
+    streams = 16   # (the most, as an untuned context has)
     best_t, best_ch = None, None
     for ch in CHUNKS:                                   # one chunk for every class
         t = evaluate([ch] * 21, streams)

@@ -55,8 +55,7 @@ __device__ __forceinline__ void hermite_e(int i, int j, double pa, double pb, do
     }
 }
 
-// One thread per primitive pair of the class-sorted lists: its record, and H
-// from the pre-scaled density (both orders of an off-diagonal pair).
+// One thread per primitive pair of the sorted lists: its record.
 __global__ void hermite_pairs_kernel(int n, const int2 *__restrict__ src, const PairInfo *__restrict__ pairs,
                                      const PrimPair *__restrict__ prims, const double *__restrict__ Q, JPrim *out)
 {
@@ -67,6 +66,8 @@ __global__ void hermite_pairs_kernel(int n, const int2 *__restrict__ src, const 
     out[i] = JPrim{p.zeta, p.P[0], p.P[1], p.P[2], Q[s.x], s.x, s.y};
 }
 
+// One thread per primitive pair: H from the pre-scaled density (both orders of an
+// off-diagonal pair).
 template <int L>
 __global__ void __launch_bounds__(128) hermite_density_kernel(int n, const JPrim *__restrict__ list,
                                                               const PairInfo *__restrict__ pairs,
@@ -293,8 +294,10 @@ constexpr int kJThreads = 128, kJTile = 64;
 // chunk) of LP <= LQ: the low momenta are the long lists, which fill the lanes.
 // same: one list with itself; then only pairs of q's shell
 // pair before p's count for both sides, p's own shell pair for V^p alone.
-// Bound by FP64 issue: C8H18 / 6-31G** (N = 210) 0.92 ms for the whole matrix,
-// 1.53 ms by the Fock-build kernels without exchange.
+// Bound by FP64 issue (42-55 % of the FP64 pipe in the eight largest list pairs of
+// C8H18 / 6-31G**, N = 210; with s pairs also by the shared-memory wavefronts of
+// the tile, 65-79 % of the L1 data pipe): 0.92 ms for the whole matrix, 1.53 ms by
+// the Fock-build kernels without exchange.
 template <int LP, int LQ>
 __global__ void __launch_bounds__(kJThreads) hermite_coulomb_kernel(int np, const JPrim *__restrict__ plist,
                                                                     const double *__restrict__ Hp, double *Vp, int nq,

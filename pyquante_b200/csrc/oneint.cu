@@ -9,10 +9,11 @@
 // because (x-B)^lj (x-A)^li = sum_p C(lj,p) AB^(lj-p) (x-A)^(li+p); a
 // primitive pair whose centre P lies nearer to B takes the moments about B
 // instead (the sum would cancel about A).  The binomial coefficients depend on
-// the function pair alone: a warp writes both sets to shared memory once.  A nuclear-attraction task multiplies the three axes'
-// polynomials in u and pairs the product's coefficients with F_m(T), since
-// int_0^1 t^(2m) exp(-T t^2) dt = F_m(T): no roots are needed, and the work of
-// a task follows the pair's own powers, which are uniform over the warp.
+// the function pair alone: a warp writes both sets to shared memory once.  A
+// nuclear-attraction task multiplies the three axes' polynomials in u and pairs
+// the product's coefficients with F_m(T), since int_0^1 t^(2m) exp(-T t^2) dt =
+// F_m(T): no roots are needed, and the work of a task follows the pair's own
+// powers, which are uniform over the warp.
 #include <cmath>
 #include <cstdint>
 

@@ -1556,17 +1556,21 @@ int pqb_schwarz(pqb_ctx *ctx, double *Q_host, void *stream)
 }
 
 // The chunk of each class for a plan of this basis, where the caller has not set
-// it.  The tuned chunks (32
-// primitive quartets an item) suit builds that fill the GPU; below that an
-// item's serial chain is the build's length (a (11|11) primitive quartet takes
-// 1.5 us), so the items are cut until a class gives about 4096 of them, to a
-// least length that grows with the basis's primitive quartets (each cut item
-// digests again).  Measured, FP64 build, 32 -> this rule: water / 6-31G** (0.06 M
-// primitive quartets) 84 -> 52 us, (H2O)3 / STO-3G (0.6 M) 71 -> 38, C2H6 / 6-31G*
-// (1.2 M) 92 -> 78, (H2O)3 / 6-31G** (4.3 M) 117 -> 104; C4H10 / 6-31G* (13 M) 212
-// -> 224 if it were cut to 4, so it is not.  Returns whether the mixed mode's
-// FP32-eligible lists are better merged into the FP64 launches too (below 9 M:
-// water dimer / 6-31G* 77 -> 58 us; (H2O)5 / 6-31G*, 23 M, 184 apart, 198 merged).
+// it.  The tuned chunks (32 primitive quartets an item) suit builds that fill the
+// GPU; below that an item's serial chain is the build's length (a (11|11) primitive
+// quartet takes 1.5 us), so the items are cut until a class gives about 4096 of
+// them, to a least length that grows with the basis's primitive quartets (each cut
+// item digests again).  Measured, FP64 build, us, items of 32 / this rule / 4, by
+// the primitive quartets that survive the screening:
+//   water 6-31G** 0.06 M 78 / 52 / 52;  (H2O)3 STO-3G 0.14 M 65 / 29 / 29;
+//   (H2O)2 6-31G* 0.20 M 84 / 52 / 53;  (H2O)3 6-31G** 0.77 M 87 / 66 / 61;
+//   C2H6 6-31G* 0.95 M 87 / 62 / 66;  (H2O)5 6-31G* 2.5 M 103 / 90 / 96;
+//   C4H10 6-31G* 8.1 M 168 / 170 / 262.
+// Returns whether the mixed mode's FP32-eligible lists are better merged into the
+// FP64 launches too, by the primitive quartets before the screening: below 9 M
+// (apart / merged: (H2O)2 6-31G* 0.2 M 69 / 53, (H2O)4 6-31G* 1.9 M 77 / 72, (H2O)5
+// 6-31G** 5.4 M 117 / 118, C4H10 6-31G* 8.4 M 166 / 169; two densities 94 / 74, 106 /
+// 92, 166 / 163, 219 / 228; above, C10H22 STO-3G 34 M 218 apart, 267 in FP64).
 static bool plan_chunks(const pqb_ctx *ctx, int *chunk)
 {
     double u[kNumQuartetClass] = {0.0}, total = 0.0;
@@ -2125,10 +2129,10 @@ static int launch_hermite(pqb_ctx *ctx, cudaStream_t st)
     PQB_CK(ctx, dens.join());
     PQB_CK(ctx, coul.fork(std::min(15, ctx->nstreams)));
     int k = 0;
-    for (int lp = 4; lp >= 0; --lp)
-        for (int lq = lp; lq >= 0; --lq)
+    for (int lq = 4; lq >= 0; --lq)
+        for (int lp = lq; lp >= 0; --lp)
             PQB_CK(ctx, coul.run(k++, [&](cudaStream_t sk) {
-                return launch_hermite_coulomb(lq, lp, l, ctx->plan_thresh, sk, ctx->nsm);
+                return launch_hermite_coulomb(lp, lq, l, ctx->plan_thresh, sk, ctx->nsm);
             }));
     PQB_CK(ctx, coul.join());
     return PQB_OK;
