@@ -90,13 +90,13 @@ class FunctionTable:
             k = len(bf.pexps)
             if k != len(bf.pcoefs) or k != len(bf.pnorms) or not k:
                 raise ValueError("inconsistent primitive lists in %r" % (bf,))
-            if len(bf.origin) != 3 or len(bf.powers) != 3:
-                raise ValueError("the origin and powers of %r have not three components each" % (bf,))
             exps += bf.pexps
             pcoefs += bf.pcoefs
             pnorms += bf.pnorms
-            origin += bf.origin
-            powers += bf.powers
+            x, y, z = r = bf.origin     # three of each, or a ValueError
+            origin += r
+            x, y, z = r = bf.powers
+            powers += r
             norms.append(bf.norm)
             off.append(len(exps))
         np_ = len(exps)
@@ -110,7 +110,7 @@ class FunctionTable:
         host[3 * n + np_:3 * n + 2 * np_] = np.array(pcoefs, dtype=np.float64) * np.array(pnorms, dtype=np.float64)
         host[3 * n + 2 * np_:nd] = norms
         ints = host[nd:].view(np.int32)
-        ints[:3 * n] = powers
+        ints[:3 * n] = self.powers_host.ravel()
         ints[3 * n:ni] = off
         buf = torch.from_numpy(host).to(torch.device("cuda", device))
         ibuf = buf[nd:].view(torch.int32)
