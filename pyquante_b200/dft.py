@@ -37,16 +37,20 @@ def getXC(gr, nel, **kwargs):
         raise NotImplementedError("gradient-corrected functionals are not built")
     gr.floor_density()
     w = gr.weights()
-    # (renormalize() with its factor kept on the GPU: the host waits once, for Exc; a
-    # zero density, an error below, is left as it is)
+    # renormalize() with its factor kept on the GPU, so that the host waits once, for
+    # Exc: the functional gets the scaled columns, and the grid's density is scaled
+    # when the factor is known not to be that of a zero density
     total = torch.dot(w, gr.density.sum(1))
-    gr.density *= torch.where(total == 0.0, 1.0, nel / total)
-    fxc, va, vb, _, _, _ = XC(gr.density.T, None, functional=functional)
+    factor = nel / total
+    rho = torch.empty((2, len(w)), dtype=torch.float64, device=w.device)
+    torch.mul(gr.density.T, factor, out=rho)
+    fxc, va, vb, _, _, _ = XC(rho, None, functional=functional)
     exc = torch.dot(w, fxc)
     Fxc = gr.fock(w * va)
     exc, total = torch.stack([exc, total]).tolist()
     if total == 0.0:
         raise ZeroDivisionError("the density on the grid is zero")
+    gr.density *= factor
     return exc, Fxc
 
 
