@@ -201,7 +201,8 @@ int pqb_jk_direct(pqb_ctx *ctx, const double *D, double *J, double *K, int mode,
  * G_host, such as a numpy array, when the call returns: CUDA finishes a
  * device-to-pageable copy before its cudaMemcpyAsync returns, and repeated
  * calls with both arrays pageable go through page-locked copies that the
- * context owns, the whole call being one graph launch that is waited for).
+ * context owns, where the system has such memory, the whole call being one
+ * graph launch that is waited for).
  * Single-molecule contexts; the context owns the device copies of D and G. */
 int pqb_get2jmk_host(pqb_ctx *ctx, const double *D_host, double *G_host, int mode, void *stream);
 
