@@ -92,6 +92,8 @@ def purify(Fp, nocc, pad=None, tol=1e-13, maxit=200, fixed=False, check=1):
         B, n = Fp.shape[0], Fp.shape[-1]
         Fc = Fp.to(torch.float64).contiguous()
         no = torch.as_tensor(nocc, dtype=torch.float64, device=Fp.device).reshape(-1).expand(B).contiguous()
+        if pad is not None and pad.device != Fp.device:
+            raise RuntimeError("purify: the padding is on %s, the matrices on %s" % (pad.device, Fp.device))
         pd = None if pad is None else pad.to(torch.uint8).expand(B, n).contiguous()
         P = torch.empty_like(Fc)
         rc = lib.pqb_purify(B, n, _lib.ptr(Fc), _lib.ptr(no), _lib.ptr(pd), _lib.ptr(P), None, int(maxit), float(tol),

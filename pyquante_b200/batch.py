@@ -190,7 +190,8 @@ def _solve_small(A, b):
     kernel on the GPU up to PQB_SOLVE_MAX rows, else plain tensor operations.
     A singular system gives non-finite x."""
     Bn, n = A.shape[0], A.shape[-1]
-    if A.is_cuda and A.dtype == torch.float64 and n <= _lib.PQB_SOLVE_MAX:
+    if A.is_cuda and A.dtype == b.dtype == torch.float64 and b.device == A.device and A.shape == (Bn, n, n) \
+            and b.shape == (Bn, n) and n <= _lib.PQB_SOLVE_MAX:
         A, b = A.contiguous(), b.contiguous()
         x = torch.empty_like(b)
         rc = _lib.load().pqb_solve_small(Bn, n, _lib.ptr(A), _lib.ptr(b), _lib.ptr(x), _lib.stream_ptr())

@@ -237,3 +237,25 @@ def test_batched_rhf_64_mixed_size_systems():
     print("64 systems: max |E_batched - E_single| %.3e, batched SCF %.2f s, p50 per molecule %.3f s" %
           (worst, res["scf_seconds"], float(np.percentile(res["scf_times"], 50))))
     assert worst < 1e-8
+
+
+def test_host_padding_and_mismatched_systems_are_refused():
+    """What the tensor operations refused before kernels read these by address:
+    a padding mask on the host, a right-hand side of another device or shape."""
+    from pyquante_b200.LA2 import purify
+    from pyquante_b200.batch import _solve_small
+    F = torch.diag(torch.arange(5.0, dtype=torch.float64, device="cuda"))[None].repeat(2, 1, 1)
+    pad = torch.zeros(2, 5, dtype=torch.bool)
+    with pytest.raises(RuntimeError):
+        purify(F, [2, 3], pad=pad)
+    P = purify(F, [2, 3], pad=pad.cuda())
+    want = torch.stack([torch.diag((torch.arange(5) < k).double()) for k in (2, 3)]).cuda()
+    assert float((P - want).abs().max()) < 1e-10
+    A = F + 1.0
+    for b in (torch.ones(2, 5, dtype=torch.float64), torch.ones(2, 4, dtype=torch.float64, device="cuda"),
+              torch.ones(1, 5, dtype=torch.float64, device="cuda")):
+        with pytest.raises(RuntimeError):
+            _solve_small(A, b)
+    b = torch.ones(2, 5, dtype=torch.float32, device="cuda")   # promoted, as before
+    A = A + torch.eye(5, dtype=torch.float64, device="cuda")
+    assert float((A @ _solve_small(A, b)[..., None] - 1.0).abs().max()) < 1e-10
